@@ -403,9 +403,16 @@ bool stencil_prepare(const LevelView<float>& V, long u_elems, long cell_elems, S
   // slot per plane, the plain kernel does better
   if (!TY || (TY < std::min(16, Y) && (long)TY * (X - 1) < kStThreads)) return false;
   a.TY = TY;
-  a.KZ = 32;
   a.ntj = (Y + TY - 1) / TY;
-  a.ntk = (Z + a.KZ - 1) / a.KZ;
+  // planes of a tile: 32 where that gives every SM a CTA (two halo planes in
+  // 34), fewer while it does not -- a tile marches its planes one after the
+  // other (3 to 4 us a plane), so a small batch left most SMs idle behind 32
+  // of them: one RHS at 64^3 148 us on 15 tiles of 32 planes, about 20 us on
+  // 165 tiles of 2; at 16^3 51 and 15 us
+  for (a.KZ = 32;; a.KZ /= 2) {
+    a.ntk = (Z + a.KZ - 1) / a.KZ;
+    if (a.KZ == 2 || (long)a.ntj * a.ntk * V.nrhs >= 152) break;
+  }
   a.ncarr = ncarr;
   a.uwin = (unsigned)a.Ru * 256;
   a.cwin = (unsigned)a.Rc * 256;
