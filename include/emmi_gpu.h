@@ -174,7 +174,8 @@ int emmi_solver_line_factor_format(const emmi_solver *s);
 /* The CUDA stream (cudaStream_t) every launch of this solver goes to. */
 void *emmi_solver_stream(const emmi_solver *s);
 /* the level-0 sweep shapes in use per direction d: shapes[d] = {lines per
- * block and ring depth of the fp16 substitution, threads per block of the
+ * block and ring depth (groups of five rows an end) of the complex64
+ * substitution where it works in tiles of 32 lines, threads per block of the
  * right-hand-side kernel}; *tuned = 1 when this solver's set-up timed them
  * (0: defaults or the process cache).  No counterpart in the reference. */
 int emmi_solver_sweep_shapes(const emmi_solver *s, int shapes[3][3], int *tuned);

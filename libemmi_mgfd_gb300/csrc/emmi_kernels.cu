@@ -15,54 +15,13 @@
 // Blocks of one colour neither overlap nor read each other's unknowns: a line
 // along d through (ta,tb) reads transverse neighbours at ta+-1 / tb+-1 only
 // (checked by tests/test_coloring.py), so a colour is one parallel launch.
-#include "emmi_kernels.cuh"
-
-#include <cuda_fp16.h>
+#include "emmi_line.cuh"
 
 #include <cstdio>
 #include <mutex>
 #include <type_traits>
 
 namespace emmi {
-
-// ------------------------------------------------------------ line tables
-// Position of an edge on the line along d through transverse nodes (ta,tb)
-// (a<b the other directions), in the reference's row order
-// (src/gmg.c:413-603): node s=1..n_d-1 holds E_d(s-1), E_a(ta-1), E_a(ta),
-// E_b(tb-1), E_b(tb); the last row is E_d(n_d-1).  -1 when not on the line.
-__host__ __device__ constexpr int line_pos(int d, int a, int b, int ta, int tb, int nd, int comp,
-                                          int p0, int p1, int p2) {
-  const int P[3] = {p0, p1, p2};
-  if (comp == d) return (P[a] == ta && P[b] == tb && P[d] >= 0 && P[d] < nd) ? 5 * P[d] : -1;
-  if (P[d] < 1 || P[d] >= nd) return -1;
-  if (comp == a)
-    return (P[b] == tb && (P[a] == ta - 1 || P[a] == ta)) ? 5 * (P[d] - 1) + 1 + (P[a] - ta + 1)
-                                                           : -1;
-  return (P[a] == ta && (P[b] == tb - 1 || P[b] == tb)) ? 5 * (P[d] - 1) + 3 + (P[b] - tb + 1)
-                                                         : -1;
-}
-
-// band offset of neighbour k of the row of type t on a line along d (127 if
-// the neighbour is not on the line); evaluated on an interior row.
-__host__ __device__ constexpr int line_off(int d, int t, int k) {
-  const int a = (d == 0) ? 1 : 0, b = (d == 2) ? 1 : 2;
-  const int s = 8, ta = 8, tb = 8, nd = 64;
-  const int comp = (t == 0) ? d : (t <= 2 ? a : b);
-  int P[3] = {0, 0, 0};
-  P[d] = (t == 0) ? s - 1 : s;
-  P[a] = ta - (t == 1 ? 1 : 0);
-  P[b] = tb - (t == 3 ? 1 : 0);
-  const int row = 5 * (s - 1) + t;
-  const NbrOff o = nbr_off(comp, k);
-  const int p = (comp + 1) % 3, q = (comp + 2) % 3;
-  int Q[3] = {P[0], P[1], P[2]};
-  Q[comp] += o.dc;
-  Q[p] += o.dp;
-  Q[q] += o.dq;
-  const int pos = line_pos(d, a, b, ta, tb, nd, o.comp, Q[0], Q[1], Q[2]);
-  return pos < 0 ? 127 : pos - row;
-}
-
 
 long line_count(const int n[3], int d, int color) {
   const int a = (d == 0) ? 1 : 0, b = (d == 2) ? 1 : 2;
@@ -347,110 +306,6 @@ void launch_norm(const C_t<T>* v, long n3s, int nrhs, const int* active, double*
 // holds record values [q*L, q*L+L) with L = 16/sizeof(T) (3 planes for float,
 // 6 for double), so one warp-wide 16-byte access of consecutive lines reads
 // or writes 512 contiguous bytes.
-#define WI(i, j) ((i) * ((i) + 1) / 2 + (j))
-constexpr int kRec = 12;
-
-__device__ __forceinline__ float4 pack16(const float* v) { return make_float4(v[0], v[1], v[2], v[3]); }
-__device__ __forceinline__ double2 pack16(const double* v) { return make_double2(v[0], v[1]); }
-__device__ __forceinline__ void unpack16(const float4& w, float* v) {
-  v[0] = w.x; v[1] = w.y; v[2] = w.z; v[3] = w.w;
-}
-__device__ __forceinline__ void unpack16(const double2& w, double* v) { v[0] = w.x; v[1] = w.y; }
-
-template <typename T> struct Vec16 { using V = float4; };
-template <> struct Vec16<double> { using V = double2; };
-template <typename T> constexpr int kLanes = 16 / (int)sizeof(T);
-template <typename T> constexpr int kPlanes = kRec / kLanes<T>;
-
-// p: plane 0 of one (row, line); ps: distance between planes (= lines)
-template <typename T>
-__device__ __forceinline__ void rec_put(typename Vec16<T>::V* p, long ps, const T (&v)[kRec]) {
-#pragma unroll
-  for (int q = 0; q < kPlanes<T>; q++) p[q * ps] = pack16(v + q * kLanes<T>);
-}
-template <typename T>
-__device__ __forceinline__ void rec_get(const typename Vec16<T>::V* p, long ps, T (&v)[kRec]) {
-#pragma unroll
-  for (int q = 0; q < kPlanes<T>; q++) unpack16(p[q * ps], v + q * kLanes<T>);
-}
-// values [10,11] (z or x) live in the last plane for both types
-template <typename T>
-__device__ __forceinline__ C_t<T> rec_get_x(const typename Vec16<T>::V* p, long ps) {
-  T v[kLanes<T>];
-  unpack16(p[(kPlanes<T> - 1) * ps], v);
-  return mk<T>(v[kLanes<T> - 2], v[kLanes<T> - 1]);
-}
-
-struct LineGeom {
-  int la, lb, fa, fb;  // lines per transverse direction and first index
-  long nl;             // lines of the colour
-  int nd, m;           // nodes along the line, rows
-};
-
-template <int D>
-__host__ __device__ __forceinline__ LineGeom line_geom(const int n[3], int pa, int pb) {
-  constexpr int A = (D == 0) ? 1 : 0, B = (D == 2) ? 1 : 2;
-  LineGeom g;
-  g.fa = pa ? 1 : 2;
-  g.fb = pb ? 1 : 2;
-  g.la = (n[A] - 1 >= g.fa) ? (n[A] - 1 - g.fa) / 2 + 1 : 0;
-  g.lb = (n[B] - 1 >= g.fb) ? (n[B] - 1 - g.fb) / 2 + 1 : 0;
-  g.nl = (long)g.la * g.lb;
-  g.nd = n[D];
-  g.m = 5 * n[D] - 4;
-  return g;
-}
-
-// work item -> (line, node s); threads along memory-contiguous direction
-template <int D>
-__device__ __forceinline__ bool line_item(const LineGeom& g, long id, long& l, int& s) {
-  if (id >= g.nl * g.nd) return false;
-  if (D == 0) {  // rows of an x-line are contiguous in memory
-    const unsigned u = (unsigned)id, nd = (unsigned)g.nd;
-    l = u / nd;
-    s = 1 + (int)(u - (unsigned)l * nd);
-  } else {  // neighbouring lines (consecutive i) are contiguous
-    const unsigned u = (unsigned)id, nl = (unsigned)g.nl;
-    const unsigned q = u / nl;
-    l = u - q * nl;
-    s = 1 + (int)q;
-  }
-  return true;
-}
-
-// the divisors of a colour's thread decode (one launch): rows x items
-// (x-line residual), the item-per-line divisor of line_item and the lines
-// per transverse direction
-struct LineDiv {
-  unsigned items;
-  FastDiv rows, item, la;
-};
-template <int D>
-LineDiv line_div(const int n[3], int pa, int pb) {
-  const LineGeom g = line_geom<D>(n, pa, pb);
-  LineDiv v;
-  v.items = (unsigned)(g.nl * g.nd);
-  v.rows = make_fastdiv(v.items > 0 ? v.items : 1);
-  v.item = make_fastdiv((unsigned)(D == 0 ? g.nd : (g.nl > 0 ? g.nl : 1)));
-  v.la = make_fastdiv((unsigned)(g.la > 0 ? g.la : 1));
-  return v;
-}
-// line_item with the launch's divisor
-template <int D>
-__device__ __forceinline__ bool line_item_fd(const LineGeom& g, const LineDiv& v, unsigned id,
-                                             long& l, int& s) {
-  if (id >= v.items) return false;
-  const unsigned q = fdiv(id, v.item);
-  if (D == 0) {  // rows of an x-line are contiguous in memory
-    l = q;
-    s = 1 + (int)(id - q * (unsigned)g.nd);
-  } else {  // neighbouring lines (consecutive i) are contiguous
-    l = id - q * (unsigned)g.nl;
-    s = 1 + (int)q;
-  }
-  return true;
-}
-
 // the record of row type TT of node s: band entries, diagonal, residual
 template <typename T, int D, int TT, int C>
 __device__ __forceinline__ void assemble_row(const LevelView<T>& L, const C_t<T>* u,
@@ -489,18 +344,6 @@ __device__ __forceinline__ void assemble_row(const LevelView<T>& L, const C_t<T>
   rec_put<T>(rp, ps, rec);
 }
 
-template <int D, int TT>
-__device__ __forceinline__ long line_slot(const int n[3], long S, int ta, int tb, int s) {
-  constexpr int A = (D == 0) ? 1 : 0, B = (D == 2) ? 1 : 2;
-  constexpr int C = (TT == 0) ? D : (TT <= 2 ? A : B);
-  int P[3];
-  P[D] = (TT == 0) ? s - 1 : s;
-  P[A] = ta - (TT == 1 ? 1 : 0);
-  P[B] = tb - (TT == 3 ? 1 : 0);
-  return (long)C * S + slot_id(n, P[0], P[1], P[2]);
-}
-
-// one thread per (line, node) and its five rows: y and z lines, whose
 // neighbouring lines are neighbouring slots
 template <typename T, int D>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_line_assemble(LevelView<T> L,
@@ -582,21 +425,6 @@ __global__ void __launch_bounds__(256) k_line_assemble_rows(LevelView<T> L, int 
 // accesses), filled by cp.async kRing-1 rows ahead of the elimination: the
 // row-to-row dependency of the factorization no longer waits on a memory
 // round trip.
-constexpr int kRing = 6;
-constexpr int kSolveThreads = 64;
-
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() {
-  asm volatile("cp.async.commit_group;\n" ::: "memory");
-}
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
 template <typename T>
 __global__ void __launch_bounds__(kSolveThreads) k_line_solve(const int* __restrict__ active,
                                                               long nl, int m,
@@ -741,627 +569,6 @@ __global__ void __launch_bounds__(256) k_line_apply(LevelView<T> L, int pa, int 
   }
 }
 
-// ---------------------------------------------------------------- stored line factors
-// A line's band matrix depends on the operator only, never on the iterate.
-// The complex64 solver can therefore keep the LDL^T factors of every line
-// (one record per row: L(p+i, p) for i = 1..5 and 1/d_p, the 12 values
-// k_line_solve writes in place, as planes [row][plane][line]) and sweep with
-// a residual per row and a substitution: the same arithmetic in the same
-// order as k_line_solve, so the same result, with 8 instead of 48 bytes per
-// row written by the assembly and no complex reciprocal per row.
-
-template <typename T, int D, int TT, int C, int W>
-__device__ __forceinline__ C_t<T> row_residual(const LevelView<T>& L, const C_t<T>* u,
-                                               const C_t<T>* f, const T* cells,
-                                               const Geo<T>& G, T wmu, int ta, int tb, int s,
-                                               const long ss[3]) {
-  constexpr int A = (D == 0) ? 1 : 0, B = (D == 2) ? 1 : 2;
-  int P[3];
-  P[D] = (TT == 0) ? s - 1 : s;
-  P[A] = ta - (TT == 1 ? 1 : 0);
-  P[B] = tb - (TT == 3 ? 1 : 0);
-  const int sl = P[0] + (L.n[0] + 1) * (P[1] + (L.n[1] + 1) * P[2]);  // 32-bit slot
-  EdgeCoef<T> e;
-  const C_t<T> au = apply_row<T, C, W>(L, u, cells, G, wmu, P, sl, ss, e);
-  return csub<T>(f[C * (int)L.S + sl], au);
-}
-
-// rb[rhs][row][line] = residual of every row of one colour; y and z lines:
-// a thread per (line, node) and its five rows; x lines: a thread per
-// (row type, line, node), row type slowest
-template <typename T, int D, int W>
-__global__ void __launch_bounds__(256) k_line_rhs(LevelView<T> L, int pa, int pb, LineDiv dv,
-                                                  C_t<T>* __restrict__ rb) {
-  constexpr int A = (D == 0) ? 1 : 0, B = (D == 2) ? 1 : 2;
-  const int rhs = blockIdx.y;
-  if (L.active && !L.active[rhs]) return;
-  const LineGeom g = line_geom<D>(L.n, pa, pb);
-  unsigned id = blockIdx.x * blockDim.x + threadIdx.x;
-  int rt = 0;
-  if (D == 0) {
-    rt = (int)fdiv(id, dv.rows);
-    if (rt >= 5) return;
-    id -= (unsigned)rt * dv.items;
-  }
-  long l;
-  int s;
-  if (!line_item_fd<D>(g, dv, id, l, s)) return;
-  if (D == 0 && rt > 0 && s == g.nd) return;
-  const unsigned lq = fdiv((unsigned)l, dv.la);
-  const int ta = g.fa + 2 * (int)((unsigned)l - lq * (unsigned)g.la), tb = g.fb + 2 * (int)lq;
-  const int n0 = L.n[0] + 1, n1 = L.n[1] + 1;
-  const long ss[3] = {1, (long)n0, (long)n0 * n1};
-  const C_t<T>* u = L.u + (long)rhs * 3 * L.S;
-  const C_t<T>* f = L.f + (long)rhs * 3 * L.S;
-  const T* cells = L.cells + (long)op_of(L, rhs) * 4 * L.ncell;
-  const Geo<T> G{L.geo + (long)op_of(L, rhs) * L.gstride, L.gmax1};
-  const T wmu = L.wmu[rhs];
-  C_t<T>* out = rb + (long)rhs * g.m * g.nl + l;
-  const int r0 = 5 * (s - 1);
-  auto put = [&](int row, C_t<T> v) { out[(long)row * g.nl] = v; };
-  if (D == 0) {
-    switch (rt) {
-      case 0: put(r0, row_residual<T, D, 0, D, W>(L, u, f, cells, G, wmu, ta, tb, s, ss)); break;
-      case 1: put(r0 + 1, row_residual<T, D, 1, A, W>(L, u, f, cells, G, wmu, ta, tb, s, ss)); break;
-      case 2: put(r0 + 2, row_residual<T, D, 2, A, W>(L, u, f, cells, G, wmu, ta, tb, s, ss)); break;
-      case 3: put(r0 + 3, row_residual<T, D, 3, B, W>(L, u, f, cells, G, wmu, ta, tb, s, ss)); break;
-      default: put(r0 + 4, row_residual<T, D, 4, B, W>(L, u, f, cells, G, wmu, ta, tb, s, ss)); break;
-    }
-  } else {
-    put(r0, row_residual<T, D, 0, D, W>(L, u, f, cells, G, wmu, ta, tb, s, ss));
-    if (s < g.nd) {
-      put(r0 + 1, row_residual<T, D, 1, A, W>(L, u, f, cells, G, wmu, ta, tb, s, ss));
-      put(r0 + 2, row_residual<T, D, 2, A, W>(L, u, f, cells, G, wmu, ta, tb, s, ss));
-      put(r0 + 3, row_residual<T, D, 3, B, W>(L, u, f, cells, G, wmu, ta, tb, s, ss));
-      put(r0 + 4, row_residual<T, D, 4, B, W>(L, u, f, cells, G, wmu, ta, tb, s, ss));
-    }
-  }
-}
-
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
-template <typename T>
-__device__ __forceinline__ void cp_async_c(C_t<T>* smem, const C_t<T>* gmem) {
-  if constexpr (sizeof(C_t<T>) == 8) cp_async8(smem, gmem);
-  else cp_async16(smem, gmem);
-}
-
-// Stored-factor formats: kFacF32 keeps the 12 fp32 values per row of
-// k_line_solve; kFacF16 keeps the five L values per row as fp16 complex
-// (20 bytes) and 1/d as fp32 complex (8 bytes), 28 instead of 48 bytes per
-// row for the substitution to stream.  A group's kFacF16 block of m rows x
-// nl lines: LA [m][nl] uint4 (L1..L4), LB [m][nl] half2 (L5), ID [m][nl]
-// float2, each part starting on 16 bytes.
-__host__ __device__ inline long round4(long v) { return (v + 3) / 4 * 4; }
-__host__ __device__ inline long half_fac_elems(int m, long nl) {
-  return round4(4 * m * nl) + round4(m * nl) + round4(2 * m * nl);
-}
-struct HalfFac {
-  uint4* la;
-  __half2* lb;
-  float2* id;
-};
-__host__ __device__ inline HalfFac half_fac(const float* g, int m, long nl) {
-  float* b = const_cast<float*>(g);
-  HalfFac h;
-  h.la = reinterpret_cast<uint4*>(b);
-  h.lb = reinterpret_cast<__half2*>(b + round4(4 * m * nl));
-  h.id = reinterpret_cast<float2*>(b + round4(4 * m * nl) + round4(m * nl));
-  return h;
-}
-__device__ __forceinline__ uint32_t h2u(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
-__device__ __forceinline__ float2 u2f2(uint32_t u) {
-  return __half22float2(*reinterpret_cast<__half2*>(&u));
-}
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
-
-// band entries (lower, real) and diagonal of row type TT of node s: the
-// band part of assemble_row's record
-template <typename T, int D, int TT, int C>
-__device__ __forceinline__ void band_row(const LevelView<T>& L, const T* cells, const Geo<T>& G,
-                                         T wmu, int ta, int tb, int s, int row, T (&band)[5],
-                                         C_t<T>& diag) {
-  constexpr int A = (D == 0) ? 1 : 0, B = (D == 2) ? 1 : 2;
-  int P[3];
-  P[D] = (TT == 0) ? s - 1 : s;
-  P[A] = ta - (TT == 1 ? 1 : 0);
-  P[B] = tb - (TT == 3 ? 1 : 0);
-  EdgeCoef<T> e;
-  edge_coef<T, C>(L.n, P, cells + (long)C * L.ncell, cells + 3 * L.ncell, G, wmu, e, L.imu_vol);
-#pragma unroll
-  for (int j = 0; j < 5; j++) band[j] = 0;
-#define LINE_ENTRY(K)                                                         \
-  {                                                                           \
-    constexpr int off = line_off(D, TT, K);                                   \
-    if constexpr (off < 0) {                                                  \
-      if (row + off >= 0) band[5 + off] = e.c[K];                             \
-    }                                                                         \
-  }
-  LINE_ENTRY(0) LINE_ENTRY(1) LINE_ENTRY(2) LINE_ENTRY(3) LINE_ENTRY(4) LINE_ENTRY(5)
-  LINE_ENTRY(6) LINE_ENTRY(7) LINE_ENTRY(8) LINE_ENTRY(9) LINE_ENTRY(10) LINE_ENTRY(11)
-#undef LINE_ENTRY
-  diag = mk<T>(e.dre, e.dim);
-}
-
-// Factors of every line of one colour, for group blockIdx.y of the chunk,
-// straight from the operator: a thread assembles a node's band rows in
-// registers (band_row) and runs the forward elimination of k_line_solve on
-// them -- no band records through memory -- writing factors to
-// fac + grp * gstride:
-//   FMT 0 (kFacF32): the record layout, 12 values per row, L(p+i, p) for
-//   i = 1..5 and 1/d_p;
-//   FMT 1 (kFacF16, T = float): L(p+i, p) rounded to fp16 in planes LA
-//   (i = 1..4) and LB (i = 5), 1/d_p in fp32 (ID); an L value outside the
-//   fp16 range (or not finite) sets *ovf.
-// y and z lines: neighbouring lines are neighbouring slots, so a warp's cell
-// loads coalesce; x lines read theirs along each thread's line (uncoalesced,
-// still faster than assembling records: 15.4 against 23.2 ms for the 128^3
-// batch's set-up).
-template <typename T, int D, int FMT>
-__global__ void __launch_bounds__(kSolveThreads) k_line_factor_direct(LevelView<T> L, int pa,
-                                                                      int pb, long gstride,
-                                                                      T* __restrict__ fac,
-                                                                      int* __restrict__ ovf) {
-  constexpr int A = (D == 0) ? 1 : 0, B = (D == 2) ? 1 : 2;
-  using V = typename Vec16<T>::V;
-  constexpr int NP = kPlanes<T>;
-  const int grp = blockIdx.y;
-  const LineGeom g = line_geom<D>(L.n, pa, pb);
-  const long l = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (l >= g.nl) return;
-  const unsigned lq = (unsigned)l / (unsigned)g.la;
-  const int ta = g.fa + 2 * (int)((unsigned)l - lq * (unsigned)g.la), tb = g.fb + 2 * (int)lq;
-  const T* cells = L.cells + (long)op_of(L, grp) * 4 * L.ncell;
-  const Geo<T> G{L.geo + (long)op_of(L, grp) * L.gstride, L.gmax1};
-  const T wmu = L.wmu[grp];
-  const int m = g.m, nd = g.nd;
-  const long nl = g.nl;
-  V* fout = reinterpret_cast<V*>(fac + (long)grp * gstride) + l;
-  const long rs = NP * nl;
-  HalfFac hf{};
-  if constexpr (FMT == kFacF16) hf = half_fac(fac + (long)grp * gstride, m, nl);
-  bool over = false;
-  C_t<T> W[21];
-#pragma unroll
-  for (int i = 0; i < 21; i++) W[i] = mk<T>(0, 0);
-#pragma unroll
-  for (int i = 0; i < 5; i++) W[WI(i, i)] = mk<T>(1, 0);
-  // the arriving row sits in W[WI(5, .)]: eliminate pivot row - 5 and
-  // store its factors
-  auto step = [&](int row) {
-    const C_t<T> id = crcp<T>(W[0]);
-    C_t<T> lqv[6];
-#pragma unroll
-    for (int i = 1; i < 6; i++) lqv[i] = cmul<T>(W[WI(i, 0)], id);
-#pragma unroll
-    for (int i = 1; i < 6; i++) {
-#pragma unroll
-      for (int j = 1; j <= i; j++) W[WI(i, j)] = cfms<T>(W[WI(i, j)], lqv[i], W[WI(j, 0)]);
-    }
-    const int piv = row - 5;
-    if (piv >= 0) {
-      if constexpr (FMT == kFacF32) {
-        T o[kRec];
-#pragma unroll
-        for (int i = 1; i < 6; i++) {
-          o[2 * (i - 1)] = lqv[i].x;
-          o[2 * (i - 1) + 1] = lqv[i].y;
-        }
-        o[10] = id.x;
-        o[11] = id.y;
-        rec_put<T>(fout + (long)piv * rs, nl, o);
-      } else {
-        __half2 h[5];
-#pragma unroll
-        for (int i = 1; i < 6; i++) {
-          over |= !(fabsf(lqv[i].x) <= 65504.f && fabsf(lqv[i].y) <= 65504.f);
-          h[i - 1] = __floats2half2_rn(lqv[i].x, lqv[i].y);
-        }
-        const long o = (long)piv * nl + l;
-        hf.la[o] = make_uint4(h2u(h[0]), h2u(h[1]), h2u(h[2]), h2u(h[3]));
-        hf.lb[o] = h[4];
-        hf.id[o] = make_float2(id.x, id.y);
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 5; i++) {
-#pragma unroll
-      for (int j = 0; j <= i; j++) W[WI(i, j)] = W[WI(i + 1, j + 1)];
-    }
-  };
-  T bd[5][5];
-  C_t<T> dg[5];
-  auto assemble = [&](auto tt, int s) {
-    constexpr int TT = decltype(tt)::value;
-    constexpr int C = (TT == 0) ? D : (TT <= 2 ? A : B);
-    band_row<T, D, TT, C>(L, cells, G, wmu, ta, tb, s, 5 * (s - 1) + TT, bd[TT], dg[TT]);
-  };
-  auto arrive = [&](auto tt, int s) {
-    constexpr int TT = decltype(tt)::value;
-#pragma unroll
-    for (int j = 0; j < 5; j++) W[WI(5, j)] = mk<T>(bd[TT][j], 0);
-    W[WI(5, 5)] = dg[TT];
-    step(5 * (s - 1) + TT);
-  };
-  // rows in record order: node s brings row 5(s-1) and, below the last
-  // node, its four transverse rows; a node's loads are issued together
-  for (int s = 1; s <= nd; s++) {
-    assemble(std::integral_constant<int, 0>(), s);
-    if (s < nd) {
-      assemble(std::integral_constant<int, 1>(), s);
-      assemble(std::integral_constant<int, 2>(), s);
-      assemble(std::integral_constant<int, 3>(), s);
-      assemble(std::integral_constant<int, 4>(), s);
-    }
-    arrive(std::integral_constant<int, 0>(), s);
-    if (s < nd) {
-      arrive(std::integral_constant<int, 1>(), s);
-      arrive(std::integral_constant<int, 2>(), s);
-      arrive(std::integral_constant<int, 3>(), s);
-      arrive(std::integral_constant<int, 4>(), s);
-    }
-  }
-  // five unit rows flush the last pivots (rows m..m+4)
-  for (int row = m; row < m + 5; row++) {
-#pragma unroll
-    for (int j = 0; j < 5; j++) W[WI(5, j)] = mk<T>(0, 0);
-    W[WI(5, 5)] = mk<T>(1, 0);
-    step(row);
-  }
-  if (over) atomicOr(ovf, 1);
-}
-
-// Substitution with stored factors (group grp[rhs]): rb holds the rows'
-// residuals in, z between the passes, the correction x out.
-template <typename T>
-__global__ void __launch_bounds__(kSolveThreads) k_line_subst(const int* __restrict__ active,
-                                                              const int* __restrict__ grp,
-                                                              long nl, int m,
-                                                              const T* __restrict__ fac,
-                                                              C_t<T>* __restrict__ rb) {
-  using V = typename Vec16<T>::V;
-  constexpr int NP = kPlanes<T>;
-  __shared__ V ring[kRing][NP][kSolveThreads];
-  __shared__ C_t<T> rring[kRing][kSolveThreads];
-  const int rhs = blockIdx.y;
-  if (active && !active[rhs]) return;
-  const int tid = threadIdx.x;
-  const long l = blockIdx.x * (long)blockDim.x + tid;
-  if (l >= nl) return;
-  const long rs = NP * nl;
-  const V* fb = reinterpret_cast<const V*>(fac) + (long)grp[rhs] * m * rs + l;
-  C_t<T>* rr = rb + (long)rhs * m * nl + l;
-  auto issue_f = [&](int row) {
-    const V* src = fb + (long)row * rs;
-    const int slot = row % kRing;
-#pragma unroll
-    for (int q = 0; q < NP; q++) cp_async16(&ring[slot][q][tid], src + q * nl);
-  };
-  auto take_f = [&](int row, T (&v)[kRec]) {
-    const int slot = row % kRing;
-#pragma unroll
-    for (int q = 0; q < NP; q++) unpack16(ring[slot][q][tid], v + q * kLanes<T>);
-  };
-  // forward: at step `row` the residual of row `row` arrives and pivot
-  // row-5 is eliminated with its stored factors (k_line_solve's order)
-  C_t<T> y[6];
-#pragma unroll
-  for (int i = 0; i < 6; i++) y[i] = mk<T>(0, 0);
-  for (int p = 0; p < kRing - 1; p++) {
-    if (p < m) cp_async_c<T>(&rring[p % kRing][tid], rr + (long)p * nl);
-    if (p - 5 >= 0 && p - 5 < m) issue_f(p - 5);
-    cp_async_commit();
-  }
-  for (int row = 0; row < m + 5; row++) {
-    {
-      const int q = row + kRing - 1;
-      if (q < m) cp_async_c<T>(&rring[q % kRing][tid], rr + (long)q * nl);
-      if (q - 5 >= 0 && q - 5 < m) issue_f(q - 5);
-      cp_async_commit();
-    }
-    cp_async_wait<kRing - 1>();
-    y[5] = row < m ? rring[row % kRing][tid] : mk<T>(0, 0);
-    const int piv = row - 5;
-    if (piv >= 0) {
-      T v[kRec];
-      take_f(piv, v);
-#pragma unroll
-      for (int i = 1; i < 6; i++) y[i] = cfms<T>(y[i], mk<T>(v[2 * (i - 1)], v[2 * (i - 1) + 1]), y[0]);
-      rr[(long)piv * nl] = cmul<T>(y[0], mk<T>(v[10], v[11]));  // z
-    }
-#pragma unroll
-    for (int i = 0; i < 5; i++) y[i] = y[i + 1];
-  }
-  cp_async_wait<0>();
-  __threadfence_block();  // z just stored is read back below
-  // backward: x_k = z_k - sum_i L(k+i, k) x_{k+i}
-  C_t<T> xw[5];
-#pragma unroll
-  for (int i = 0; i < 5; i++) xw[i] = mk<T>(0, 0);
-  for (int p = 0; p < kRing - 1; p++) {
-    const int q = m - 1 - p;
-    if (q >= 0) {
-      issue_f(q);
-      cp_async_c<T>(&rring[q % kRing][tid], rr + (long)q * nl);
-    }
-    cp_async_commit();
-  }
-  for (int row = m - 1; row >= 0; row--) {
-    {
-      const int q = row - (kRing - 1);
-      if (q >= 0) {
-        issue_f(q);
-        cp_async_c<T>(&rring[q % kRing][tid], rr + (long)q * nl);
-      }
-      cp_async_commit();
-    }
-    cp_async_wait<kRing - 1>();
-    T v[kRec];
-    take_f(row, v);
-    C_t<T> x = rring[row % kRing][tid];
-#pragma unroll
-    for (int i = 0; i < 5; i++) x = cfms<T>(x, mk<T>(v[2 * i], v[2 * i + 1]), xw[i]);
-#pragma unroll
-    for (int i = 4; i > 0; i--) xw[i] = xw[i - 1];
-    xw[0] = x;
-    rr[(long)row * nl] = x;
-  }
-  cp_async_wait<0>();
-}
-
-// The same substitution with kFacF16 factors of group grp[rhs] (gstride
-// values per group): the forward pass streams LA, LB and ID, the backward
-// pass LA and LB; the fp16 values are widened to fp32 and the arithmetic is
-// k_line_subst's.  NT lines per block, a cp.async ring of RING rows per
-// line: every thread's arithmetic is the same for every (NT, RING).
-//
-// D = 1 or 2 (y or z lines, whose neighbouring lines are neighbouring slots):
-// the backward pass also adds x to u at each row's slot (k_line_apply_rb's
-// work; the old u values ride the cp.async ring with the factors), so the
-// colour takes two launches and x never goes through the record buffer.
-// D = -1: x goes to rb for k_line_apply_rb.
-template <int D>
-__device__ __forceinline__ int subst_row_slot(const int n[3], long S, int ta, int tb, int row) {
-  const int s = row / 5 + 1, t = row - 5 * (s - 1);
-  switch (t) {
-    case 0: return (int)line_slot<D, 0>(n, S, ta, tb, s);
-    case 1: return (int)line_slot<D, 1>(n, S, ta, tb, s);
-    case 2: return (int)line_slot<D, 2>(n, S, ta, tb, s);
-    case 3: return (int)line_slot<D, 3>(n, S, ta, tb, s);
-    default: return (int)line_slot<D, 4>(n, S, ta, tb, s);
-  }
-}
-
-template <int NT, int RING, int D>
-__global__ void __launch_bounds__(NT) k_line_subst_h(const int* __restrict__ active,
-                                                     const int* __restrict__ grp, long nl, int m,
-                                                     long gstride, const float* __restrict__ fac,
-                                                     float2* __restrict__ rb, LevelView<float> L,
-                                                     int pa, int pb, LineDiv dv) {
-  constexpr int kRing = RING;
-  __shared__ uint4 ra[kRing][NT];
-  __shared__ uint32_t rl5[kRing][NT];
-  __shared__ float2 rd[kRing][NT];
-  __shared__ float2 rring[kRing][NT];
-  __shared__ float2 uring[D >= 1 ? kRing : 1][D >= 1 ? NT : 1];
-  const int rhs = blockIdx.y;
-  if (active && !active[rhs]) return;
-  const int tid = threadIdx.x;
-  const long l = blockIdx.x * (long)blockDim.x + tid;
-  if (l >= nl) return;
-  const HalfFac hf = half_fac(fac + (long)grp[rhs] * gstride, m, nl);
-  float2* rr = rb + (long)rhs * m * nl + l;
-  float2* u = nullptr;
-  int ta = 0, tb = 0;
-  if constexpr (D >= 1) {
-    const LineGeom g = line_geom<D>(L.n, pa, pb);
-    const unsigned lq = fdiv((unsigned)l, dv.la);
-    ta = g.fa + 2 * (int)((unsigned)l - lq * (unsigned)g.la);
-    tb = g.fb + 2 * (int)lq;
-    u = L.u + (long)rhs * 3 * L.S;
-  }
-  auto issue_l = [&](int row) {
-    const int slot = row % kRing;
-    cp_async16(&ra[slot][tid], hf.la + (long)row * nl + l);
-    cp_async4(&rl5[slot][tid], hf.lb + (long)row * nl + l);
-  };
-  auto take_l = [&](int row, float2 (&v)[5]) {
-    const int slot = row % kRing;
-    const uint4 a = ra[slot][tid];
-    v[0] = u2f2(a.x);
-    v[1] = u2f2(a.y);
-    v[2] = u2f2(a.z);
-    v[3] = u2f2(a.w);
-    v[4] = u2f2(rl5[slot][tid]);
-  };
-  // forward: at step `row` the residual of row `row` arrives and pivot
-  // row-5 is eliminated with its stored factors
-  float2 y[6];
-#pragma unroll
-  for (int i = 0; i < 6; i++) y[i] = make_float2(0.f, 0.f);
-  auto issue_fwd = [&](int q) {
-    if (q < m) cp_async8(&rring[q % kRing][tid], rr + (long)q * nl);
-    const int p = q - 5;
-    if (p >= 0 && p < m) {
-      issue_l(p);
-      cp_async8(&rd[p % kRing][tid], hf.id + (long)p * nl + l);
-    }
-    cp_async_commit();
-  };
-  for (int p = 0; p < kRing - 1; p++) issue_fwd(p);
-  for (int row = 0; row < m + 5; row++) {
-    issue_fwd(row + kRing - 1);
-    cp_async_wait<kRing - 1>();
-    y[5] = row < m ? rring[row % kRing][tid] : make_float2(0.f, 0.f);
-    const int piv = row - 5;
-    if (piv >= 0) {
-      float2 v[5];
-      take_l(piv, v);
-#pragma unroll
-      for (int i = 1; i < 6; i++) y[i] = cfms<float>(y[i], v[i - 1], y[0]);
-      rr[(long)piv * nl] = cmul<float>(y[0], rd[piv % kRing][tid]);  // z
-    }
-#pragma unroll
-    for (int i = 0; i < 5; i++) y[i] = y[i + 1];
-  }
-  cp_async_wait<0>();
-  __threadfence_block();  // z just stored is read back below
-  // backward: x_k = z_k - sum_i L(k+i, k) x_{k+i}
-  float2 xw[5];
-#pragma unroll
-  for (int i = 0; i < 5; i++) xw[i] = make_float2(0.f, 0.f);
-  auto issue_bwd = [&](int q) {
-    if (q >= 0) {
-      issue_l(q);
-      cp_async8(&rring[q % kRing][tid], rr + (long)q * nl);
-      if constexpr (D >= 1)
-        cp_async8(&uring[q % kRing][tid], u + subst_row_slot<D>(L.n, L.S, ta, tb, q));
-    }
-    cp_async_commit();
-  };
-  for (int p = 0; p < kRing - 1; p++) issue_bwd(m - 1 - p);
-  for (int row = m - 1; row >= 0; row--) {
-    issue_bwd(row - (kRing - 1));
-    cp_async_wait<kRing - 1>();
-    float2 v[5];
-    take_l(row, v);
-    float2 x = rring[row % kRing][tid];
-#pragma unroll
-    for (int i = 0; i < 5; i++) x = cfms<float>(x, v[i], xw[i]);
-#pragma unroll
-    for (int i = 4; i > 0; i--) xw[i] = xw[i - 1];
-    xw[0] = x;
-    if constexpr (D >= 1)
-      u[subst_row_slot<D>(L.n, L.S, ta, tb, row)] = cadd<float>(uring[row % kRing][tid], x);
-    else
-      rr[(long)row * nl] = x;
-  }
-  cp_async_wait<0>();
-}
-
-// u += x from rb[rhs][row][line]
-template <typename T, int D>
-__global__ void __launch_bounds__(256) k_line_apply_rb(LevelView<T> L, int pa, int pb, LineDiv dv,
-                                                       const C_t<T>* __restrict__ rb) {
-  const int rhs = blockIdx.y;
-  if (L.active && !L.active[rhs]) return;
-  const LineGeom g = line_geom<D>(L.n, pa, pb);
-  long l;
-  int s;
-  if (!line_item_fd<D>(g, dv, blockIdx.x * blockDim.x + threadIdx.x, l, s)) return;
-  const unsigned lq = fdiv((unsigned)l, dv.la);
-  const int ta = g.fa + 2 * (int)((unsigned)l - lq * (unsigned)g.la), tb = g.fb + 2 * (int)lq;
-  C_t<T>* u = L.u + (long)rhs * 3 * L.S;
-  const C_t<T>* x = rb + (long)rhs * g.m * g.nl + l;
-  const int r0 = 5 * (s - 1);
-  auto add = [&](long sl, int row) { u[sl] = cadd<T>(u[sl], x[(long)row * g.nl]); };
-  add(line_slot<D, 0>(L.n, L.S, ta, tb, s), r0);
-  if (s < g.nd) {
-    add(line_slot<D, 1>(L.n, L.S, ta, tb, s), r0 + 1);
-    add(line_slot<D, 2>(L.n, L.S, ta, tb, s), r0 + 2);
-    add(line_slot<D, 3>(L.n, L.S, ta, tb, s), r0 + 3);
-    add(line_slot<D, 4>(L.n, L.S, ta, tb, s), r0 + 4);
-  }
-}
-
-template <typename T, int D>
-static void line_factor_d(const LevelView<T>& L, int color, T* fac, int fmt, int* ovf,
-                          cudaStream_t st) {
-  const int pa = color & 1, pb = (color >> 1) & 1;
-  const long nl = line_count(L.n, D, color);
-  if (nl == 0) return;
-  const long gstride = line_factor_elems(L.n, D, color, fmt);
-  dim3 g((unsigned)((nl + kSolveThreads - 1) / kSolveThreads), L.nrhs);
-  if constexpr (std::is_same<T, float>::value) {
-    if (fmt == kFacF16) {
-      k_line_factor_direct<T, D, kFacF16><<<g, kSolveThreads, 0, st>>>(L, pa, pb, gstride, fac,
-                                                                       ovf);
-      return;
-    }
-  }
-  k_line_factor_direct<T, D, kFacF32><<<g, kSolveThreads, 0, st>>>(L, pa, pb, gstride, fac, ovf);
-}
-
-// the fp16-factor substitution's block shapes (threads per block, ring
-// depth); variant 0 is the default
-constexpr int kSubstShape[kSubstVariants][2] = {{64, 6}, {32, 6}, {128, 6}, {64, 4}, {64, 8}};
-
-int subst_variant_threads(int v) { return kSubstShape[v][0]; }
-int subst_variant_ring(int v) { return kSubstShape[v][1]; }
-
-struct SubstArgs {
-  long nl;
-  int nrhs;
-  const int* active;
-  const int* grp;
-  int m;
-  long gstride;
-  const float* fac;
-  float2* rb;
-  LevelView<float> L;
-  int pa, pb;
-  LineDiv dv;
-};
-
-template <int NT, int RING, int D>
-static void subst_h_launch(const SubstArgs& a, cudaStream_t st) {
-  dim3 g((unsigned)((a.nl + NT - 1) / NT), a.nrhs);
-  k_line_subst_h<NT, RING, D><<<g, NT, 0, st>>>(a.active, a.grp, a.nl, a.m, a.gstride, a.fac,
-                                                a.rb, a.L, a.pa, a.pb, a.dv);
-}
-
-template <int D>
-static void subst_h_variant(int v, const SubstArgs& a, cudaStream_t st) {
-  switch (v) {
-    case 1: subst_h_launch<32, 6, D>(a, st); break;
-    case 2: subst_h_launch<128, 6, D>(a, st); break;
-    case 3: subst_h_launch<64, 4, D>(a, st); break;
-    case 4: subst_h_launch<64, 8, D>(a, st); break;
-    default: subst_h_launch<64, 6, D>(a, st); break;
-  }
-}
-
-template <typename T, int D>
-static void line_sweep_fac_d(const LevelView<T>& L, int color, const T* fac, const int* grp,
-                             C_t<T>* rb, int fmt, SweepShape sh, cudaStream_t st) {
-  const int pa = color & 1, pb = (color >> 1) & 1;
-  const long nl = line_count(L.n, D, color);
-  if (nl == 0) return;
-  const long items = nl * L.n[D];
-  const int m = 5 * L.n[D] - 4;
-  dim3 g1((unsigned)((items + 255) / 256), L.nrhs);
-  const int rt = sh.rhs_threads == 128 ? 128 : 256;
-  dim3 gr((unsigned)(((D == 0 ? 5 : 1) * items + rt - 1) / rt), L.nrhs);
-  const LineDiv dv = line_div<D>(L.n, pa, pb);
-  if (L.imu_vol)
-    k_line_rhs<T, D, 1><<<gr, rt, 0, st>>>(L, pa, pb, dv, rb);
-  else
-    k_line_rhs<T, D, 0><<<gr, rt, 0, st>>>(L, pa, pb, dv, rb);
-  dim3 g2((unsigned)((nl + kSolveThreads - 1) / kSolveThreads), L.nrhs);
-  if constexpr (std::is_same<T, float>::value) {
-    if (fmt == kFacF16) {
-      const int v = sh.subst >= 0 && sh.subst < kSubstVariants ? sh.subst : 0;
-      const SubstArgs a{nl, L.nrhs, L.active, grp, m, line_factor_elems(L.n, D, color, fmt),
-                        fac, rb, L, pa, pb, dv};
-      if constexpr (D == 0) {
-        subst_h_variant<-1>(v, a, st);
-      } else {
-        subst_h_variant<D>(v, a, st);  // the update rides the backward pass
-        return;
-      }
-      k_line_apply_rb<T, D><<<g1, 256, 0, st>>>(L, pa, pb, dv, rb);
-      return;
-    }
-  }
-  k_line_subst<T><<<g2, kSolveThreads, 0, st>>>(L.active, grp, nl, m, fac, rb);
-  k_line_apply_rb<T, D><<<g1, 256, 0, st>>>(L, pa, pb, dv, rb);
-}
-
 template <typename T, int D>
 static void line_sweep_d(const LevelView<T>& L, int color, T* buf, cudaStream_t st) {
   const int pa = color & 1, pb = (color >> 1) & 1;
@@ -1380,7 +587,6 @@ static void line_sweep_d(const LevelView<T>& L, int color, T* buf, cudaStream_t 
   k_line_solve<T><<<g2, kSolveThreads, 0, st>>>(L.active, nl, m, buf);
   k_line_apply<T, D><<<g1, 256, 0, st>>>(L, pa, pb, buf);
 }
-
 // the line solve keeps a cp.async ring in shared memory: ask for the
 // largest shared-memory carveout so 12 blocks fit on an SM
 void init_line_kernels() {
@@ -1390,31 +596,10 @@ void init_line_kernels() {
                          cudaSharedmemCarveoutMaxShared);
     cudaFuncSetAttribute(k_line_solve<double>, cudaFuncAttributePreferredSharedMemoryCarveout,
                          cudaSharedmemCarveoutMaxShared);
-    cudaFuncSetAttribute(k_line_subst<float>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                         cudaSharedmemCarveoutMaxShared);
-    auto carve = [](const void* k) {
-      cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout,
-                           cudaSharedmemCarveoutMaxShared);
-    };
-    carve((const void*)k_line_subst_h<64, 6, -1>);
-    carve((const void*)k_line_subst_h<32, 6, -1>);
-    carve((const void*)k_line_subst_h<128, 6, -1>);
-    carve((const void*)k_line_subst_h<64, 4, -1>);
-    carve((const void*)k_line_subst_h<64, 8, -1>);
-    carve((const void*)k_line_subst_h<64, 6, 1>);
-    carve((const void*)k_line_subst_h<32, 6, 1>);
-    carve((const void*)k_line_subst_h<128, 6, 1>);
-    carve((const void*)k_line_subst_h<64, 4, 1>);
-    carve((const void*)k_line_subst_h<64, 8, 1>);
-    carve((const void*)k_line_subst_h<64, 6, 2>);
-    carve((const void*)k_line_subst_h<32, 6, 2>);
-    carve((const void*)k_line_subst_h<128, 6, 2>);
-    carve((const void*)k_line_subst_h<64, 4, 2>);
-    carve((const void*)k_line_subst_h<64, 8, 2>);
-    cudaFuncSetAttribute(k_line_subst<double>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                         cudaSharedmemCarveoutMaxShared);
+    init_stored_line_kernels();
   });
 }
+
 
 // scratch: m * lines * kRec values of T (see line_scratch_elems)
 template <typename T>
@@ -1424,376 +609,6 @@ void launch_line_sweep(const LevelView<T>& L, int d, int color, C_t<T>* scratch,
   else if (d == 1) line_sweep_d<T, 1>(L, color, buf, st);
   else line_sweep_d<T, 2>(L, color, buf, st);
 }
-
-long line_factor_elems(const int n[3], int d, int color, int fmt) {
-  const int m = 5 * n[d] - 4;
-  const long nl = line_count(n, d, color);
-  return fmt == kFacF16 ? half_fac_elems(m, nl) : (long)m * nl * kRec;
-}
-
-template <typename T>
-void launch_line_factor(const LevelView<T>& L, int d, int color, T* fac, int fmt, int* ovf,
-                        cudaStream_t st) {
-  if (d == 0) line_factor_d<T, 0>(L, color, fac, fmt, ovf, st);
-  else if (d == 1) line_factor_d<T, 1>(L, color, fac, fmt, ovf, st);
-  else line_factor_d<T, 2>(L, color, fac, fmt, ovf, st);
-}
-
-template <typename T>
-void launch_line_sweep_fac(const LevelView<T>& L, int d, int color, const T* fac, const int* grp,
-                           C_t<T>* rb, int fmt, cudaStream_t st, SweepShape sh) {
-  if (d == 0) line_sweep_fac_d<T, 0>(L, color, fac, grp, rb, fmt, sh, st);
-  else if (d == 1) line_sweep_fac_d<T, 1>(L, color, fac, grp, rb, fmt, sh, st);
-  else line_sweep_fac_d<T, 2>(L, color, fac, grp, rb, fmt, sh, st);
-}
-
-// ---------------------------------------------------------------- fused line relaxation
-// One launch per colour and direction.  A thread owns one line and walks it
-// twice:
-//   forward   node by node it assembles each row -- band entries and the
-//             residual of the current iterate, the row arithmetic of
-//             assemble_row -- and feeds it to the streaming LDL^T of
-//             k_line_solve: the arriving row eliminates pivot row-5, whose
-//             z = D^-1 L^-1 r and L(p+i, p), i = 1..5, are set aside;
-//   backward  x_p = z_p - sum_i L(p+i, p) x_{p+i}, u += x at the row's slot.
-// z_p waits in the level's residual buffer at row p's own slot: no other line
-// of the colour reads or writes it, and that buffer is dead while the level
-// smooths (the cycle recomputes the residual after smoothing).  L waits in
-// the line scratch, [row][line] planes per RHS:
-//   kLExact  the T-precision values (k_line_solve's arithmetic, bit for bit
-//            the same operations in the same order);
-//   kLHalf   (T = float) rounded to fp16 and used rounded by both
-//            substitutions while the elimination keeps the unrounded value:
-//            each line solve is then exact for a matrix within fp16 rounding
-//            of the line's -- the arithmetic of the stored-factor format
-//            kFacF16.  An L value outside the fp16 range sets *ovf.
-// Against the three-kernel sweep this writes no band records and reads no
-// stored factors: per row the neighbourhood of the residual, L (20 or 40
-// bytes) and z (8 bytes) out and back, and u read-modify-write.
-template <typename T, int LF> struct LineL;
-template <> struct LineL<float, kLExact> {
-  static constexpr long kBytes = 40;  // per row
-  float4* p0;
-  float4* p1;
-  float2* p2;
-  __device__ __forceinline__ LineL(void* base, int m, long nl) {
-    p0 = reinterpret_cast<float4*>(base);
-    p1 = p0 + (long)m * nl;
-    p2 = reinterpret_cast<float2*>(p1 + (long)m * nl);
-  }
-  __device__ __forceinline__ bool put(long o, const float2 (&l)[6]) {
-    p0[o] = make_float4(l[1].x, l[1].y, l[2].x, l[2].y);
-    p1[o] = make_float4(l[3].x, l[3].y, l[4].x, l[4].y);
-    p2[o] = l[5];
-    return false;
-  }
-  __device__ __forceinline__ void round(float2 (&) [6]) const {}
-  __device__ __forceinline__ void get(long o, float2 (&l)[5]) const {
-    const float4 a = p0[o], b = p1[o];
-    l[0] = make_float2(a.x, a.y);
-    l[1] = make_float2(a.z, a.w);
-    l[2] = make_float2(b.x, b.y);
-    l[3] = make_float2(b.z, b.w);
-    l[4] = p2[o];
-  }
-};
-template <> struct LineL<double, kLExact> {
-  static constexpr long kBytes = 80;
-  double2* p;
-  long ps;
-  __device__ __forceinline__ LineL(void* base, int m, long nl) {
-    p = reinterpret_cast<double2*>(base);
-    ps = (long)m * nl;
-  }
-  __device__ __forceinline__ bool put(long o, const double2 (&l)[6]) {
-#pragma unroll
-    for (int i = 0; i < 5; i++) p[i * ps + o] = l[i + 1];
-    return false;
-  }
-  __device__ __forceinline__ void round(double2 (&) [6]) const {}
-  __device__ __forceinline__ void get(long o, double2 (&l)[5]) const {
-#pragma unroll
-    for (int i = 0; i < 5; i++) l[i] = p[i * ps + o];
-  }
-};
-template <> struct LineL<float, kLHalf> {
-  static constexpr long kBytes = 20;
-  uint4* la;
-  uint32_t* lb;
-  __device__ __forceinline__ LineL(void* base, int m, long nl) {
-    la = reinterpret_cast<uint4*>(base);
-    lb = reinterpret_cast<uint32_t*>(la + (long)m * nl);
-  }
-  // l[1..5] rounded to fp16 in place (the values both substitutions use);
-  // true when one left the fp16 range
-  __device__ __forceinline__ void round(float2 (&l)[6]) const {
-#pragma unroll
-    for (int i = 1; i < 6; i++) l[i] = __half22float2(__floats2half2_rn(l[i].x, l[i].y));
-  }
-  __device__ __forceinline__ bool put(long o, const float2 (&l)[6]) {
-    __half2 h[5];
-    bool over = false;
-#pragma unroll
-    for (int i = 0; i < 5; i++) {
-      h[i] = __floats2half2_rn(l[i + 1].x, l[i + 1].y);
-      over |= !(fabsf(l[i + 1].x) <= 65504.f && fabsf(l[i + 1].y) <= 65504.f);
-    }
-    la[o] = make_uint4(h2u(h[0]), h2u(h[1]), h2u(h[2]), h2u(h[3]));
-    lb[o] = h2u(h[4]);
-    return over;
-  }
-  __device__ __forceinline__ void get(long o, float2 (&l)[5]) const {
-    const uint4 a = la[o];
-    l[0] = u2f2(a.x);
-    l[1] = u2f2(a.y);
-    l[2] = u2f2(a.z);
-    l[3] = u2f2(a.w);
-    l[4] = u2f2(lb[o]);
-  }
-};
-
-long line_l_bytes(const int n[3], int d, int color, int lf, int tsize) {
-  const long m = 5 * n[d] - 4, nl = line_count(n, d, color);
-  const long b = lf == kLHalf ? 20 : (tsize == 8 ? 80 : 40);
-  return (m * nl * b + 255) / 256 * 256;
-}
-
-// band entries (lower, real), diagonal and residual of row type TT of node s
-template <typename T, int D, int TT, int C>
-__device__ __forceinline__ void fused_row(const LevelView<T>& L, const C_t<T>* u, const C_t<T>* f,
-                                          const T* cells, const Geo<T>& G, T wmu, int ta, int tb,
-                                          int s, int row, const long ss[3], C_t<T> (&wrow)[6],
-                                          C_t<T>& r) {
-  constexpr int A = (D == 0) ? 1 : 0, B = (D == 2) ? 1 : 2;
-  int P[3];
-  P[D] = (TT == 0) ? s - 1 : s;
-  P[A] = ta - (TT == 1 ? 1 : 0);
-  P[B] = tb - (TT == 3 ? 1 : 0);
-  const int sl = P[0] + (L.n[0] + 1) * (P[1] + (L.n[1] + 1) * P[2]);  // 32-bit slot
-  EdgeCoef<T> e;
-  const C_t<T> au = apply_row<T, C>(L, u, cells, G, wmu, P, sl, ss, e);
-  r = csub<T>(f[C * (int)L.S + sl], au);
-  T band[5] = {0, 0, 0, 0, 0};
-#define LINE_ENTRY(K)                                                         \
-  {                                                                           \
-    constexpr int off = line_off(D, TT, K);                                   \
-    if constexpr (off < 0) {                                                  \
-      if (row + off >= 0) band[5 + off] = e.c[K];                             \
-    }                                                                         \
-  }
-  LINE_ENTRY(0) LINE_ENTRY(1) LINE_ENTRY(2) LINE_ENTRY(3) LINE_ENTRY(4) LINE_ENTRY(5)
-  LINE_ENTRY(6) LINE_ENTRY(7) LINE_ENTRY(8) LINE_ENTRY(9) LINE_ENTRY(10) LINE_ENTRY(11)
-#undef LINE_ENTRY
-#pragma unroll
-  for (int j = 0; j < 5; j++) wrow[j] = mk<T>(band[j], 0);
-  wrow[5] = mk<T>(e.dre, e.dim);
-}
-
-// one elimination step of the streaming LDL^T (k_line_solve's order): the
-// new row sits in W[WI(5, .)], y[5]; pivot W[0] is eliminated.  Returns
-// z = y_0 / d_0 and the multipliers l[1..5] (rounded by LS::round for kLHalf,
-// the unrounded ones updating the window)
-template <typename T, typename LS>
-__device__ __forceinline__ C_t<T> fused_eliminate(C_t<T> (&W)[21], C_t<T> (&y)[6],
-                                                  C_t<T> (&lr)[6], const LS& ls) {
-  const C_t<T> id = crcp<T>(W[0]);
-  C_t<T> lq[6];
-#pragma unroll
-  for (int i = 1; i < 6; i++) lq[i] = cmul<T>(W[WI(i, 0)], id);
-#pragma unroll
-  for (int i = 1; i < 6; i++) lr[i] = lq[i];
-  ls.round(lr);
-#pragma unroll
-  for (int i = 1; i < 6; i++) {
-#pragma unroll
-    for (int j = 1; j <= i; j++) W[WI(i, j)] = cfms<T>(W[WI(i, j)], lq[i], W[WI(j, 0)]);
-    y[i] = cfms<T>(y[i], lr[i], y[0]);
-  }
-  const C_t<T> z = cmul<T>(y[0], id);
-#pragma unroll
-  for (int i = 0; i < 5; i++) {
-#pragma unroll
-    for (int j = 0; j <= i; j++) W[WI(i, j)] = W[WI(i + 1, j + 1)];
-    y[i] = y[i + 1];
-  }
-  return z;
-}
-
-template <typename T, int D, int LF, int NT>
-__global__ void __launch_bounds__(NT) k_line_fused(LevelView<T> L, int pa, int pb, LineDiv dv,
-                                                   void* __restrict__ lbuf, long lstride,
-                                                   int* __restrict__ ovf) {
-  constexpr int A = (D == 0) ? 1 : 0, B = (D == 2) ? 1 : 2;
-  using LS = LineL<T, LF>;
-  const int rhs = blockIdx.y;
-  if (L.active && !L.active[rhs]) return;
-  const LineGeom g = line_geom<D>(L.n, pa, pb);
-  const long l = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (l >= g.nl) return;
-  const unsigned lq = fdiv((unsigned)l, dv.la);
-  const int ta = g.fa + 2 * (int)((unsigned)l - lq * (unsigned)g.la), tb = g.fb + 2 * (int)lq;
-  const int n0 = L.n[0] + 1, n1 = L.n[1] + 1;
-  const long ss[3] = {1, (long)n0, (long)n0 * n1};
-  C_t<T>* __restrict__ u = L.u + (long)rhs * 3 * L.S;
-  const C_t<T>* __restrict__ f = L.f + (long)rhs * 3 * L.S;
-  C_t<T>* __restrict__ zr = L.r + (long)rhs * 3 * L.S;
-  const T* __restrict__ cells = L.cells + (long)op_of(L, rhs) * 4 * L.ncell;
-  const Geo<T> G{L.geo + (long)op_of(L, rhs) * L.gstride, L.gmax1};
-  const T wmu = L.wmu[rhs];
-  LS ls(static_cast<char*>(lbuf) + (long)rhs * lstride, g.m, g.nl);
-  const int nd = g.nd;
-  bool over = false;
-
-  C_t<T> W[21], y[6], lr[6];
-#pragma unroll
-  for (int i = 0; i < 21; i++) W[i] = mk<T>(0, 0);
-#pragma unroll
-  for (int i = 0; i < 5; i++) {
-    W[WI(i, i)] = mk<T>(1, 0);  // dummy leading rows
-    y[i] = mk<T>(0, 0);
-  }
-  // Rows are assembled a node at a time -- the five rows' loads issued
-  // together, ahead of the node's five elimination steps -- so a node waits
-  // on memory once rather than once per row.  The arriving row (s, TT)
-  // eliminates pivot (s-1, TT): same row type, one node back; with s = 1 the
-  // pivots are the dummy leading rows.
-  C_t<T> rw[5][6], rr[5];
-  auto assemble = [&](auto tt, int s) {
-    constexpr int TT = decltype(tt)::value;
-    constexpr int C = (TT == 0) ? D : (TT <= 2 ? A : B);
-    fused_row<T, D, TT, C>(L, u, f, cells, G, wmu, ta, tb, s, 5 * (s - 1) + TT, ss, rw[TT],
-                           rr[TT]);
-  };
-  auto arrive = [&](auto tt, int s) {
-    constexpr int TT = decltype(tt)::value;
-#pragma unroll
-    for (int j = 0; j < 6; j++) W[WI(5, j)] = rw[TT][j];
-    y[5] = rr[TT];
-    const C_t<T> z = fused_eliminate<T>(W, y, lr, ls);
-    if (s >= 2) {
-      const int p = 5 * (s - 2) + TT;
-      zr[line_slot<D, TT>(L.n, L.S, ta, tb, s - 1)] = z;
-      over |= ls.put((long)p * g.nl + l, lr);
-    }
-  };
-  // trailing steps: identity rows flush pivots (s, TT) of the last rows
-  auto flush = [&](auto tt, int s) {
-    constexpr int TT = decltype(tt)::value;
-#pragma unroll
-    for (int j = 0; j < 5; j++) W[WI(5, j)] = mk<T>(0, 0);
-    W[WI(5, 5)] = mk<T>(1, 0);
-    y[5] = mk<T>(0, 0);
-    const C_t<T> z = fused_eliminate<T>(W, y, lr, ls);
-    const int p = 5 * (s - 1) + TT;
-    zr[line_slot<D, TT>(L.n, L.S, ta, tb, s)] = z;
-    over |= ls.put((long)p * g.nl + l, lr);
-  };
-  using I0 = std::integral_constant<int, 0>;
-  using I1 = std::integral_constant<int, 1>;
-  using I2 = std::integral_constant<int, 2>;
-  using I3 = std::integral_constant<int, 3>;
-  using I4 = std::integral_constant<int, 4>;
-  for (int s = 1; s < nd; s++) {
-    assemble(I0{}, s);
-    assemble(I1{}, s);
-    assemble(I2{}, s);
-    assemble(I3{}, s);
-    assemble(I4{}, s);
-    arrive(I0{}, s);
-    arrive(I1{}, s);
-    arrive(I2{}, s);
-    arrive(I3{}, s);
-    arrive(I4{}, s);
-  }
-  assemble(I0{}, nd);
-  arrive(I0{}, nd);
-  flush(I1{}, nd - 1);
-  flush(I2{}, nd - 1);
-  flush(I3{}, nd - 1);
-  flush(I4{}, nd - 1);
-  flush(I0{}, nd);
-  if (over && ovf) atomicOr(ovf, 1);
-
-  // backward: rows m-1 .. 0, i.e. (nd, 0), then (s, 4..0) for s = nd-1 .. 1
-  C_t<T> xw[5];
-#pragma unroll
-  for (int i = 0; i < 5; i++) xw[i] = mk<T>(0, 0);
-  // backward a node at a time as well: its rows' multipliers, z and u are
-  // loaded together before the five substitution steps
-  C_t<T> bl[5][5], bz[5], bu[5];
-  long bs[5];
-  auto load = [&](auto tt, int s) {
-    constexpr int TT = decltype(tt)::value;
-    bs[TT] = line_slot<D, TT>(L.n, L.S, ta, tb, s);
-    ls.get((long)(5 * (s - 1) + TT) * g.nl + l, bl[TT]);
-    bz[TT] = zr[bs[TT]];
-    bu[TT] = u[bs[TT]];
-  };
-  auto back = [&](auto tt) {
-    constexpr int TT = decltype(tt)::value;
-    C_t<T> x = bz[TT];
-#pragma unroll
-    for (int i = 0; i < 5; i++) x = cfms<T>(x, bl[TT][i], xw[i]);
-#pragma unroll
-    for (int i = 4; i > 0; i--) xw[i] = xw[i - 1];
-    xw[0] = x;
-    u[bs[TT]] = cadd<T>(bu[TT], x);
-  };
-  load(I0{}, nd);
-  back(I0{});
-  for (int s = nd - 1; s >= 1; s--) {
-    load(I4{}, s);
-    load(I3{}, s);
-    load(I2{}, s);
-    load(I1{}, s);
-    load(I0{}, s);
-    back(I4{});
-    back(I3{});
-    back(I2{});
-    back(I1{});
-    back(I0{});
-  }
-}
-
-template <typename T, int D, int LF, int NT>
-static void fused_launch(const LevelView<T>& L, int pa, int pb, long nl, void* lbuf, long lstride,
-                         int* ovf, cudaStream_t st) {
-  const LineDiv dv = line_div<D>(L.n, pa, pb);
-  dim3 g((unsigned)((nl + NT - 1) / NT), L.nrhs);
-  k_line_fused<T, D, LF, NT><<<g, NT, 0, st>>>(L, pa, pb, dv, lbuf, lstride, ovf);
-}
-
-template <typename T, int D>
-static void line_fused_d(const LevelView<T>& L, int color, void* lbuf, int lf, int nt, int* ovf,
-                         cudaStream_t st) {
-  const int pa = color & 1, pb = (color >> 1) & 1;
-  const long nl = line_count(L.n, D, color);
-  if (nl == 0) return;
-  const long lstride = line_l_bytes(L.n, D, color, lf, (int)sizeof(T));
-  if constexpr (std::is_same<T, float>::value) {
-    if (lf == kLHalf) {
-      if (nt == 32) fused_launch<T, D, kLHalf, 32>(L, pa, pb, nl, lbuf, lstride, ovf, st);
-      else if (nt == 128) fused_launch<T, D, kLHalf, 128>(L, pa, pb, nl, lbuf, lstride, ovf, st);
-      else fused_launch<T, D, kLHalf, 64>(L, pa, pb, nl, lbuf, lstride, ovf, st);
-      return;
-    }
-  }
-  if (nt == 32) fused_launch<T, D, kLExact, 32>(L, pa, pb, nl, lbuf, lstride, ovf, st);
-  else if (nt == 128) fused_launch<T, D, kLExact, 128>(L, pa, pb, nl, lbuf, lstride, ovf, st);
-  else fused_launch<T, D, kLExact, 64>(L, pa, pb, nl, lbuf, lstride, ovf, st);
-}
-
-template <typename T>
-void launch_line_fused(const LevelView<T>& L, int d, int color, void* lbuf, int lf, int nt,
-                       int* ovf, cudaStream_t st) {
-  if (d == 0) line_fused_d<T, 0>(L, color, lbuf, lf, nt, ovf, st);
-  else if (d == 1) line_fused_d<T, 1>(L, color, lbuf, lf, nt, ovf, st);
-  else line_fused_d<T, 2>(L, color, lbuf, lf, nt, ovf, st);
-}
-template void launch_line_fused<float>(const LevelView<float>&, int, int, void*, int, int, int*,
-                                       cudaStream_t);
-template void launch_line_fused<double>(const LevelView<double>&, int, int, void*, int, int, int*,
-                                        cudaStream_t);
 
 // ------------------------------------------------------------ point sweep
 // row (C, side): side 0 = E_C(N - e_C), side 1 = E_C(N); patch index 2C+side.
@@ -2141,15 +956,6 @@ void launch_zero(C_t<T>* p, long n, cudaStream_t st) {
   template void launch_zero<T>(C_t<T>*, long, cudaStream_t);
 EMMI_INST(float)
 EMMI_INST(double)
-template void launch_line_factor<float>(const LevelView<float>&, int, int, float*, int, int*,
-                                        cudaStream_t);
-template void launch_line_sweep_fac<float>(const LevelView<float>&, int, int, const float*,
-                                           const int*, C_t<float>*, int, cudaStream_t, SweepShape);
-template void launch_line_factor<double>(const LevelView<double>&, int, int, double*, int, int*,
-                                         cudaStream_t);
-template void launch_line_sweep_fac<double>(const LevelView<double>&, int, int, const double*,
-                                            const int*, C_t<double>*, int, cudaStream_t,
-                                            SweepShape);
 template void launch_residual<float, float>(const LevelView<float>&, C_t<float>*, double*, cudaStream_t);
 template void launch_residual<double, double>(const LevelView<double>&, C_t<double>*, double*, cudaStream_t);
 template void launch_residual<double, float>(const LevelView<double>&, C_t<float>*, double*, cudaStream_t);

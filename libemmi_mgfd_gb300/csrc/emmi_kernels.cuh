@@ -34,23 +34,28 @@ void launch_line_sweep(const LevelView<T>& L, int d, int color, C_t<T>* scratch,
 long line_count(const int n[3], int d, int color);
 long line_scratch_elems(const int n[3], int d, int nrhs);
 
-// stored LDL^T factors of the lines of one colour along d: T values per
-// operator group in format fmt (0: fp32 records, 12 values per row; 1: fp16
-// L and fp32 1/d, 7 values per row); launch_line_factor fills them for the
-// L.nrhs groups of L (L.op / L.wmu per group, u and f unused), the band rows
-// assembled in registers, into fac + g * line_factor_elems and sets *ovf
-// when an L value does not fit fp16 (format 1); launch_line_sweep_fac then sweeps RHS
-// r with the factors of group grp[r], rb holding (5 n_d - 4) * lines complex
-// values per RHS
+// stored LDL^T factors of the lines of one colour along d, per operator
+// group: complex128 as 12-value records ([row][plane][line], tile = 0),
+// complex64 eliminated from both ends in tiles of line_tile_width lines
+// (emmi_lines.cu), fmt kFacF32 with 48 or kFacF16 (fp16 L, fp32 1/d) with 28
+// bytes a row; line_factor_elems values of T per group.  launch_line_factor
+// fills them for the L.nrhs groups of L (L.op / L.wmu per group, u and f
+// unused), the band rows assembled in registers, into fac + g *
+// line_factor_elems and sets *ovf when an L value does not fit fp16 (kFacF16);
+// launch_line_sweep_fac then sweeps RHS r with the factors of group grp[r], rb
+// holding line_rb_elems complex values per RHS in line_fac_launches launches
 constexpr int kFacF32 = 0, kFacF16 = 1;
-long line_factor_elems(const int n[3], int d, int color, int fmt);
+int line_tile_width(const int n[3], int d, int nrhs, int fmt);
+long line_factor_elems(const int n[3], int d, int color, int fmt, int tile);
+long line_rb_elems(const int n[3], int d, int color, int tile);
 template <typename T>
-void launch_line_factor(const LevelView<T>& L, int d, int color, T* fac, int fmt, int* ovf,
-                        cudaStream_t st);
-// block shapes of a stored-factor sweep: the fp16 substitution's variant
-// (subst_variant_threads lines per block, a cp.async ring of
-// subst_variant_ring rows; 0 = 64 x 6) and the right-hand-side kernel's
-// threads per block (256 or 128).  No shape changes any thread's arithmetic.
+void launch_line_factor(const LevelView<T>& L, int d, int color, T* fac, int fmt, int tile,
+                        int* ovf, cudaStream_t st);
+// block shapes of a stored-factor sweep: the complex64 substitution's variant
+// (subst_variant_threads lines per block, a ring of subst_variant_ring groups
+// of five rows an end; 0 = 64 x 6) where its tiles have 32 lines, and the
+// right-hand-side kernel's threads per block (256 or 128).  No shape changes
+// any thread's arithmetic.
 constexpr int kSubstVariants = 5;
 struct SweepShape {
   int subst = 0;
@@ -58,22 +63,24 @@ struct SweepShape {
 };
 int subst_variant_threads(int v);
 int subst_variant_ring(int v);
+int line_fac_launches(const int n[3], int d, int tile, int fmt, SweepShape sh);
+void init_stored_line_kernels();
 template <typename T>
 void launch_line_sweep_fac(const LevelView<T>& L, int d, int color, const T* fac, const int* grp,
-                           C_t<T>* rb, int fmt, cudaStream_t st, SweepShape sh = SweepShape());
+                           C_t<T>* rb, int fmt, int tile, cudaStream_t st,
+                           SweepShape sh = SweepShape());
 
-// one colour of line relaxation along d in one launch (k_line_fused): each
-// thread assembles, factors and solves one line; z waits in L.r (the
-// level's residual buffer, dead while the level smooths) at each row's slot
-// and the line's multipliers in lbuf, line_l_bytes per RHS: lf = kLExact
+// one colour of line relaxation along d in one launch (k_line_fused,
+// k_line_fused_ends): assembles, factors and solves the lines; z waits in L.r
+// (the level's residual buffer, dead while the level smooths) at each row's
+// slot and the line's multipliers in lbuf, line_l_bytes per RHS: lf = kLExact
 // keeps them in T precision, kLHalf (T = float) in fp16 (both substitutions
-// use the rounded values; *ovf set when one leaves the fp16 range).  nt:
-// lines per block (32, 64 or 128; no value changes any thread's arithmetic)
+// use the rounded values; *ovf set when one leaves the fp16 range)
 constexpr int kLExact = 0, kLHalf = 1;
 long line_l_bytes(const int n[3], int d, int color, int lf, int tsize);
 template <typename T>
-void launch_line_fused(const LevelView<T>& L, int d, int color, void* lbuf, int lf, int nt,
-                       int* ovf, cudaStream_t st);
+void launch_line_fused(const LevelView<T>& L, int d, int color, void* lbuf, int lf, int* ovf,
+                       cudaStream_t st);
 
 // complex64 residual with its halos staged by tensor copies (emmi_stencil.cu):
 // tiles of TY rows x KZ planes, plane windows in a ring of shared-memory

@@ -354,14 +354,15 @@ static void line_colour(emmi_solver* s, int h, int l, int d, int col, const Leve
                         int r0) {
   if (s->opt.line_sweep || l >= s->opt.fused_level) {
     const int lf = std::is_same<T, float>::value ? s->lfmt : kLExact;
-    launch_line_fused<T>(W, d, col, s->scratch, lf, s->fused_nt[l][d], s->d_lovf, s->st);
+    launch_line_fused<T>(W, d, col, s->scratch, lf, s->d_lovf, s->st);
     return;
   }
   if (s->fac_on) {
     const long off = s->fac_off[l == 0 ? 0 : h][l][d][col];
     if (off >= 0) {
       launch_line_sweep_fac<T>(W, d, col, static_cast<const T*>(s->d_fac) + off, s->d_grp + r0,
-                               (C_t<T>*)s->scratch, s->fac_fmt, s->st, s->shape[l][d]);
+                               (C_t<T>*)s->scratch, s->fac_fmt,
+                               s->fac_tile[l == 0 ? 0 : h][l][d], s->st, s->shape[l][d]);
       return;
     }
   }
@@ -373,7 +374,8 @@ static void line_colour(emmi_solver* s, int h, int l, int d, int col, const Leve
 static int line_launches(const emmi_solver* s, int h, int l, int d) {
   if (s->opt.line_sweep || l >= s->opt.fused_level) return 1;  // k_line_fused
   if (s->fac_on && s->fac_off[l == 0 ? 0 : h][l][d][0] >= 0)
-    return (s->fac_fmt == kFacF16 && d != 0) ? 2 : 3;  // update in the substitution
+    return line_fac_launches(s->hier[h][l].n, d, s->fac_tile[l == 0 ? 0 : h][l][d], s->fac_fmt,
+                             s->shape[l][d]);
   return 3;
 }
 
@@ -560,7 +562,7 @@ static int build_line_factors(emmi_solver* s) {
         for (int d = 0; d < 3; d++)
           for (int c = 0; c < 4; c++) s->fac_off[h][l][d][c] = -1;
     // level 0 is the same in every hierarchy: its blocks live under h = 0
-    long total = 0;
+    long total = 0, rb = 0;
     for (int h = 0; h < 3; h++)
       for (int l = 0; l + 1 < s->lmax; l++)
         for (int d = 0; d < 3; d++) {
@@ -568,15 +570,25 @@ static int build_line_factors(emmi_solver* s) {
           if (l >= s->opt.fused_level) continue;  // swept by the one-launch kernel
           const int hb = l == 0 ? 0 : h;
           if (s->fac_off[hb][l][d][0] >= 0) continue;
+          const int tile = std::is_same<T, float>::value
+                               ? line_tile_width(s->hier[h][l].n, d, s->chunk, fmt) : 0;
+          s->fac_tile[hb][l][d] = tile;
           for (int c = 0; c < 4; c++) {
             s->fac_off[hb][l][d][c] = total;
-            total += (long)ng * line_factor_elems(s->hier[h][l].n, d, c, fmt);
+            total += (long)ng * line_factor_elems(s->hier[h][l].n, d, c, fmt, tile);
+            rb = std::max(rb, line_rb_elems(s->hier[h][l].n, d, c, tile));
           }
         }
     if (total == 0) return EMMI_OK;
     const size_t freeb = device_avail();
     const size_t bytes = (size_t)total * sizeof(T);
     if (bytes > freeb / 2) return EMMI_OK;  // factor in every sweep instead
+    // row buffers padded to whole tiles (short levels of a few lines)
+    if ((size_t)rb * sizeof(C_t<T>) * s->chunk > s->scratch_bytes) {
+      s->release(s->scratch);
+      s->scratch_bytes = (size_t)rb * sizeof(C_t<T>) * s->chunk;
+      if ((rc = s->alloc(&s->scratch, s->scratch_bytes)) != EMMI_OK) return rc;
+    }
     if ((rc = s->alloc((void**)&s->d_fac, bytes)) != EMMI_OK) return rc;
     if (!s->d_grp) {
       if ((rc = s->alloc((void**)&s->d_grp, nrhs * sizeof(int))) != EMMI_OK) return rc;
@@ -608,7 +620,7 @@ static int build_line_factors(emmi_solver* s) {
           V.nrhs = ng;
           for (int c = 0; c < 4; c++)
             launch_line_factor<T>(V, d, c, static_cast<T*>(s->d_fac) + s->fac_off[hb][l][d][c], fmt,
-                                  d_ovf, s->st);
+                                  s->fac_tile[hb][l][d], d_ovf, s->st);
         }
     CK(cudaGetLastError());
     int ovf = 0;
@@ -773,7 +785,8 @@ static int autotune_sweeps(emmi_solver* s) {
     SweepShape c = best;
     c.rhs_threads = 128;
     consider(c);
-    for (int v = 1; v < kSubstVariants; v++) {
+    // narrow tiles have one shape
+    for (int v = 1; v < kSubstVariants && s->fac_tile[0][0][d] == 32; v++) {
       c = best;
       c.subst = v;
       consider(c);
@@ -1201,8 +1214,11 @@ static int create_impl(emmi_solver** out, const emmi_problem* P, const emmi_opti
     TRY(s->alloc((void**)&s->d_lovf, sizeof(int)));
     CKS(cudaMemsetAsync(s->d_lovf, 0, sizeof(int), s->st));
     s->lfmt = (mixed && s->opt.line_factors == 2) ? kLHalf : kLExact;
-    for (int l = 0; l < kMaxLev; l++)
-      for (int d = 0; d < 3; d++) s->fused_nt[l][d] = 64;
+    // below level 0 blocks of 32 lines and five groups: the fastest of the
+    // shapes on 25 levels of 128 x 64 x 64 (1.53 against 1.56 ms a z sweep with
+    // 64 x 6) and 32 x 64 x 64 (0.45 against 0.50)
+    for (int l = 1; l < kMaxLev; l++)
+      for (int d = 0; d < 3; d++) s->shape[l][d].subst = 1;
     mark("field buffers");
     if (s->opt.line_factors && !s->opt.line_sweep)
       TRY(mixed ? build_line_factors<float>(s) : build_line_factors<double>(s));

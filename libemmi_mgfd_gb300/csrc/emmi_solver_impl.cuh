@@ -102,16 +102,16 @@ struct emmi_solver {
   void* d_fac = nullptr;
   size_t fac_bytes = 0;
   long fac_off[3][emmi::kMaxLev][3][4];
+  int fac_tile[3][emmi::kMaxLev][3];  // lines per tile of the complex64 blocks
 
   // one-launch line sweep (opt.line_sweep): multiplier format (kLHalf only
-  // for MIXED with line_factors = 2), the device flag an fp16 multiplier out
-  // of range sets, and lines per block per (level, direction)
+  // for MIXED with line_factors = 2) and the device flag an fp16 multiplier
+  // out of range sets
   int lfmt = 0;
   // every operator's input invmur is exactly 1: the complex64 operator takes
   // its coefficients from the spacings (LevelView::imu_vol)
   bool imu_vol = false;
   int* d_lovf = nullptr;
-  int fused_nt[emmi::kMaxLev][3];
 
   // stored FP64 edge coefficients of the level-0 true operators (MIXED):
   // the refinement residual reads them instead of recomputing (null: off)
