@@ -135,6 +135,174 @@ __global__ void __launch_bounds__(256) k_line_rhs(LevelView<T> L, int pa, int pb
   }
 }
 
+// ---------------------------------------------------------------- row residuals by node
+// The complex64 residuals of a colour's rows with the coefficients from the
+// spacings (imu_vol): a thread takes a line's node s -- E_D of the edge below
+// it and the node's four transverse edges -- and loads each of the 30 edge
+// values, 20 conductivities and six spacings the five equations share once
+// (row by row they are 65, 20 and 25), all of them before the first use.
+// With hat sizes h = (d- + d+) / 2, the equation of an edge along C of size
+// d_C between the directions X and Y reads (edge_coef with cell weight =
+// volume)
+//   sum over (X, Y): d_C h_Y [(E - E(+X)) / d_X+ + (E - E(-X)) / d_X-]
+//                    + h_Y [E_X(+C) - E_X - E_X(+C, -X) + E_X(-X)]
+//   - i wmu sbar E.
+// y and z lines: a warp takes 32 lines at a node, a block NW nodes.  x lines:
+// a warp takes 32 nodes of a line (neighbours in memory), a block NW lines,
+// whose rows are staged in shared memory and stored line by line of a tile.
+// Bound by DRAM: level 0 of 4 right-hand sides at 128^3, a colour of y lines,
+// reads and writes 503 MB (u, f and sigma once) in 90 us, 5.6 TB/s; row by row
+// the same bytes took 131 us, waiting for loads.  A sweep of 25 right-hand
+// sides with it: x 7.57 -> 5.95, y 6.37 -> 5.39, z 5.90 -> 5.47 ms.
+template <int D, int NW>
+__global__ void __launch_bounds__(32 * NW, 16 / NW) k_line_rows(LevelView<float> L, int pa, int pb,
+                                                       LineDiv dv, LineTile tl, int nodes,
+                                                       int lines, float2* __restrict__ rb) {
+  constexpr int A = (D == 0) ? 1 : 0, B = (D == 2) ? 1 : 2;
+  const int rhs = blockIdx.y;
+  if (L.active && !L.active[rhs]) return;
+  const LineGeom g = line_geom<D>(L.n, pa, pb);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  // blocks along the nodes (y lines) or the lines (z and x) first: planes of z
+  // are swept one after the other
+  const int bn = D == 1 ? blockIdx.x % nodes : blockIdx.x / lines;
+  const int bl = D == 1 ? blockIdx.x / nodes : blockIdx.x % lines;
+  const int s = D == 0 ? 1 + bn * 32 + lane : 1 + bn * NW + w;
+  const int l = D == 0 ? bl * NW + w : bl * 32 + lane;
+  const bool live = l < (int)g.nl && s <= g.nd;
+  if (D != 0 && !live) return;
+  float2 r[5];
+#pragma unroll
+  for (int t = 0; t < 5; t++) r[t] = make_float2(0.f, 0.f);
+  if (live) {
+    const unsigned lq = fdiv((unsigned)l, dv.la);
+    const int ta = g.fa + 2 * (l - (int)lq * g.la), tb = g.fb + 2 * (int)lq;
+    const int op = op_of(L, rhs);
+    const int ss[3] = {1, L.n[0] + 1, (L.n[0] + 1) * (L.n[1] + 1)};
+    const int cs[3] = {1, L.n[0], L.n[0] * L.n[1]};
+    const int sd = ss[D], sa = ss[A], sb = ss[B], cd = cs[D], ca = cs[A], cb = cs[B];
+    const int S = (int)L.S;
+    const int o = s * sd + ta * sa + tb * sb;  // the node's slot
+    const float2* u = L.u + (long)rhs * 3 * S;
+    const float2* f = L.f + (long)rhs * 3 * S;
+    const float2 *ud = u + (D * S + o), *ua = u + (A * S + o), *ub = u + (B * S + o);
+    const float2 *fd = f + (D * S + o), *fa = f + (A * S + o), *fb = f + (B * S + o);
+    const float* cells = L.cells + (long)op * 4 * L.ncell;
+    const int nc = (int)L.ncell, co = s * cd + ta * ca + tb * cb;
+    const float *gd = cells + ((long)D * nc + co), *ga = cells + ((long)A * nc + co),
+                *gb = cells + ((long)B * nc + co);
+    const Geo<float> G{L.geo + (long)op * L.gstride, L.gmax1};
+    const float wmu = L.wmu[rhs];
+    const bool node = s < g.nd;  // the last node carries its E_D row only
+    // edges along D below (0) and above (1) the node, at the five transverse
+    // positions; transverse edges - and + of the node
+    const float2 d0 = ldro(ud - sd), d0am = ldro(ud - sd - sa), d0ap = ldro(ud - sd + sa),
+                 d0bm = ldro(ud - sd - sb), d0bp = ldro(ud - sd + sb);
+    const float2 am = ldro(ua - sa), ap = ldro(ua), bm = ldro(ub - sb), bp = ldro(ub);
+    const float2 am_dm = ldro(ua - sa - sd), ap_dm = ldro(ua - sd), bm_dm = ldro(ub - sb - sd),
+                 bp_dm = ldro(ub - sd);
+    const float sg0 = ldro(gd - cd - ca - cb), sg1 = ldro(gd - cd - ca), sg2 = ldro(gd - cd - cb),
+                sg3 = ldro(gd - cd);
+    const float2 f0 = fd[-sd];
+    const float D0 = ldro(G.ds(D) + s - 1);
+    const float A0 = ldro(G.ds(A) + ta - 1), A1 = ldro(G.ds(A) + ta);
+    const float B0 = ldro(G.ds(B) + tb - 1), B1 = ldro(G.ds(B) + tb);
+    const float2 zero = make_float2(0.f, 0.f);
+    float2 d1 = zero, d1am = zero, d1ap = zero, d1bm = zero, d1bp = zero;
+    float2 am_dp = zero, ap_dp = zero, bm_dp = zero, bp_dp = zero;
+    float2 am_bm = zero, am_bp = zero, ap_bm = zero, ap_bp = zero;
+    float2 bm_am = zero, bm_ap = zero, bp_am = zero, bp_ap = zero;
+    float2 f1 = zero, f2 = zero, f3 = zero, f4 = zero;
+    float sa0 = 0.f, sa1 = 0.f, sb0 = 0.f, sb1 = 0.f, D1 = 1.f;
+    if (node) {
+      d1 = ldro(ud);
+      d1am = ldro(ud - sa);
+      d1ap = ldro(ud + sa);
+      d1bm = ldro(ud - sb);
+      d1bp = ldro(ud + sb);
+      am_dp = ldro(ua - sa + sd);
+      ap_dp = ldro(ua + sd);
+      bm_dp = ldro(ub - sb + sd);
+      bp_dp = ldro(ub + sd);
+      am_bm = ldro(ua - sa - sb);
+      am_bp = ldro(ua - sa + sb);
+      ap_bm = ldro(ua - sb);
+      ap_bp = ldro(ua + sb);
+      bm_am = ldro(ub - sb - sa);
+      bm_ap = ldro(ub - sb + sa);
+      bp_am = ldro(ub - sa);
+      bp_ap = ldro(ub + sa);
+      f1 = fa[-sa];
+      f2 = fa[0];
+      f3 = fb[-sb];
+      f4 = fb[0];
+      // conductivities around the four transverse edges
+      sa0 = ((ldro(ga - ca - cd - cb) + ldro(ga - ca - cd)) + ldro(ga - ca - cb)) + ldro(ga - ca);
+      sa1 = ((ldro(ga - cd - cb) + ldro(ga - cd)) + ldro(ga - cb)) + ldro(ga);
+      sb0 = ((ldro(gb - cb - cd - ca) + ldro(gb - cb - cd)) + ldro(gb - cb - ca)) + ldro(gb - cb);
+      sb1 = ((ldro(gb - cd - ca) + ldro(gb - cd)) + ldro(gb - ca)) + ldro(gb);
+      D1 = ldro(G.ds(D) + s);
+    }
+    const float rD0 = qdiv(1.f, D0), rD1 = qdiv(1.f, D1), rA0 = qdiv(1.f, A0),
+                rA1 = qdiv(1.f, A1), rB0 = qdiv(1.f, B0), rB1 = qdiv(1.f, B1);
+    const float hd = 0.5f * (D0 + D1), ha = 0.5f * (A0 + A1), hb = 0.5f * (B0 + B1);
+    const float qw = 0.25f * wmu;
+    // f - A e of an edge: acc holds the curl-curl part, sig the sum of the
+    // four conductivities around it
+    auto done = [&](float2 ff, float2 acc, float2 e, float sig) {
+      const float m = qw * sig;  // the mass term is -i m e
+      return make_float2(ff.x - acc.x - m * e.y, ff.y - acc.y + m * e.x);
+    };
+    auto pair = [&](float2 acc, float2 e, float2 ep, float2 em, float k, float rp, float rm,
+                    float h, float2 x1, float2 x0, float2 x1m, float2 x0m) {
+      const float kp = k * rp, km = k * rm;
+      acc.x += (kp * (e.x - ep.x) + km * (e.x - em.x)) + h * ((x1.x - x0.x) - (x1m.x - x0m.x));
+      acc.y += (kp * (e.y - ep.y) + km * (e.y - em.y)) + h * ((x1.y - x0.y) - (x1m.y - x0m.y));
+      return acc;
+    };
+    {
+      float2 c = pair(zero, d0, d0ap, d0am, D0 * hb, rA1, rA0, hb, ap, ap_dm, am, am_dm);
+      c = pair(c, d0, d0bp, d0bm, D0 * ha, rB1, rB0, ha, bp, bp_dm, bm, bm_dm);
+      r[0] = done(f0, c, d0, ((sg0 + sg1) + sg2) + sg3);
+    }
+    if (node) {
+      float2 c = pair(zero, am, am_dp, am_dm, A0 * hb, rD1, rD0, hb, d1, d1am, d0, d0am);
+      c = pair(c, am, am_bp, am_bm, A0 * hd, rB1, rB0, hd, bp, bp_am, bm, bm_am);
+      r[1] = done(f1, c, am, sa0);
+      c = pair(zero, ap, ap_dp, ap_dm, A1 * hb, rD1, rD0, hb, d1ap, d1, d0ap, d0);
+      c = pair(c, ap, ap_bp, ap_bm, A1 * hd, rB1, rB0, hd, bp_ap, bp, bm_ap, bm);
+      r[2] = done(f2, c, ap, sa1);
+      c = pair(zero, bm, bm_dp, bm_dm, B0 * ha, rD1, rD0, ha, d1, d1bm, d0, d0bm);
+      c = pair(c, bm, bm_ap, bm_am, B0 * hd, rA1, rA0, hd, ap, ap_bm, am, am_bm);
+      r[3] = done(f3, c, bm, sb0);
+      c = pair(zero, bp, bp_dp, bp_dm, B1 * ha, rD1, rD0, ha, d1bp, d1, d0bp, d0);
+      c = pair(c, bp, bp_ap, bp_am, B1 * hd, rA1, rA0, hd, ap_bp, ap, am_bp, am);
+      r[4] = done(f4, c, bp, sb1);
+    }
+  }
+  const int shift = tl.shift, mask = (1 << shift) - 1;
+  float2* out = rb + (long)rhs * rb_elems<float>(tl, g.nl);
+  const int r0 = 5 * (s - 1);
+  if constexpr (D != 0) {
+    float2* q = out + ((long)(l >> shift) * tl.m << shift) + (l & mask);
+#pragma unroll
+    for (int t = 0; t < 5; t++)
+      if (r0 + t < tl.m) q[(long)tl.pos(r0 + t) << shift] = r[t];
+  } else {
+    constexpr int kPitch = 5 * 32 + 1;
+    __shared__ float2 st[NW * kPitch];
+#pragma unroll
+    for (int t = 0; t < 5; t++) st[w * kPitch + 5 * lane + t] = r[t];
+    __syncthreads();
+    for (int e = threadIdx.x; e < 160 * NW; e += 32 * NW) {
+      const int row = 160 * bn + e / NW, ll = bl * NW + e % NW;
+      if (row < tl.m && ll < (int)g.nl)
+        out[(((long)(ll >> shift) * tl.m + tl.pos(row)) << shift) | (ll & mask)] =
+            st[(e % NW) * kPitch + e / NW];
+    }
+  }
+}
+
 // band entries (lower, real) and diagonal of row type TT of node s: the
 // band part of assemble_row's record; MIR: the entries to the rows after it
 // (band[5 - i] to row + i; the operator is bitwise symmetric), what the row
@@ -1011,6 +1179,15 @@ static void apply_rb(const LevelView<T>& L, int pa, int pb, const LineDiv& dv, c
   k_line_apply_rb<T, D><<<g1, 256, 0, st>>>(L, pa, pb, dv, tl, rb);
 }
 
+template <int D, int NW>
+static void line_rows(const LevelView<float>& L, int pa, int pb, long nl, const LineDiv& dv,
+                      const LineTile& tl, float2* rb, cudaStream_t st) {
+  const int nodes = (L.n[D] + (D == 0 ? 31 : NW - 1)) / (D == 0 ? 32 : NW);
+  const int lines = (int)((nl + (D == 0 ? NW - 1 : 31)) / (D == 0 ? NW : 32));
+  dim3 g((unsigned)(nodes * lines), L.nrhs);
+  k_line_rows<D, NW><<<g, 32 * NW, 0, st>>>(L, pa, pb, dv, tl, nodes, lines, rb);
+}
+
 template <typename T, int D>
 static void line_sweep_fac_d(const LevelView<T>& L, int color, const T* fac, const int* grp,
                              C_t<T>* rb, int fmt, int tile, SweepShape sh, cudaStream_t st) {
@@ -1023,10 +1200,15 @@ static void line_sweep_fac_d(const LevelView<T>& L, int color, const T* fac, con
   dim3 gr((unsigned)(((D == 0 ? 5 : 1) * items + rt - 1) / rt), L.nrhs);
   const LineDiv dv = line_div<D>(L.n, pa, pb);
   const LineTile tl = line_tile(L.n[D], tile);
-  if (L.imu_vol)
-    k_line_rhs<T, D, 1><<<gr, rt, 0, st>>>(L, pa, pb, dv, tl, rb);
-  else
-    k_line_rhs<T, D, 0><<<gr, rt, 0, st>>>(L, pa, pb, dv, tl, rb);
+  bool rows = false;
+  if constexpr (std::is_same<T, float>::value) {
+    if (L.imu_vol) {
+      rt == 128 ? line_rows<D, 4>(L, pa, pb, nl, dv, tl, rb, st)
+                : line_rows<D, 8>(L, pa, pb, nl, dv, tl, rb, st);
+      rows = true;
+    }
+  }
+  if (!rows) k_line_rhs<T, D, 0><<<gr, rt, 0, st>>>(L, pa, pb, dv, tl, rb);
   if constexpr (std::is_same<T, float>::value) {
     const EndsArgs a{&L, grp, nl, tl, line_factor_elems(L.n, D, color, fmt, tile), fac, rb, pa, pb,
                      dv};
