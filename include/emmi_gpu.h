@@ -96,9 +96,11 @@ typedef struct {
                        launches are short); levels above it the three-launch
                        sweep.  A value >= the number of levels keeps the
                        three-launch sweep everywhere                      */
-  int staged;       /* MIXED: 1 = the complex64 residual stages each plane's
-                       halo in shared memory with tensor copies (default);
-                       0 = the plain residual                              */
+  int staged;       /* MIXED: 1 = the complex64 residual of level 0 stages
+                       each plane's halo in shared memory with tensor copies
+                       where the batch is small (default; large batches take
+                       the plain residual, which is faster there); 0 = the
+                       plain residual                                      */
   int skip_pre;     /* bit l set: level l leaves out its pre-smoothing (0:
                        every level smooths v1 times, as the reference)     */
   int skip_post;    /* bit l set: level l leaves out its post-smoothing (0:
@@ -150,7 +152,8 @@ int emmi_solver_line_format(const emmi_solver *s);
  * them (the reference's arithmetic). */
 int emmi_solver_geometric_weights(const emmi_solver *s);
 /* 1 when the complex64 level-0 residual of s stages its halos by tensor
- * copies (emmi_options.staged and a tile that fits shared memory). */
+ * copies (emmi_options.staged, a tile that fits shared memory and a batch
+ * of fewer tiles than the device has SMs). */
 int emmi_solver_staged(const emmi_solver *s);
 /* Test hook of the staged residual's bounded waits (no counterpart in the
  * reference): the staged residuals launched after the call give up a wait

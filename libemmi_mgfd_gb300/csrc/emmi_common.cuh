@@ -48,8 +48,9 @@ template <typename T> __device__ __forceinline__ C_t<T> crcp(C_t<T> z) {
   return mk<T>(ldexp(zx * inv, -e), ldexp(-zy * inv, -e));
 }
 
-// read-only (non-coherent) loads: the data a kernel only reads during its
-// launch; lets loads move past the kernel's own stores
+// read-only (non-coherent) loads, for data that no kernel of a cycle writes
+// (operator, geometry, factors): the compiler may move them past stores, and
+// past dep_wait
 template <typename T> __device__ __forceinline__ T ldro(const T* p) { return __ldg(p); }
 
 // Division by a divisor fixed for a launch, for dividends below 2^31, as a
@@ -70,6 +71,41 @@ inline FastDiv make_fastdiv(unsigned d) {
 }
 __device__ __forceinline__ unsigned fdiv(unsigned u, const FastDiv& f) {
   return (__umulhi(u, f.m) + u) >> f.l;
+}
+
+// ---------------------------------------------------------------- dependent launches
+// The kernels of a cycle are launched with programmatic stream serialization
+// (launch_dep): a kernel's blocks may become resident while the kernel before
+// it drains, and wait here until that one is complete and its writes are
+// visible.  Every block of such a kernel calls dep_wait before it returns or
+// touches memory that another kernel writes, so completion stays transitive
+// along the stream; dep_next then lets the kernel after it be launched.  In a
+// kernel launched the ordinary way both do nothing.
+__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void dep_next() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// Grids of up to kDepBlocks blocks: the gap between small kernels is what few
+// right-hand sides wait for (one shot at 16^3 23.6 -> 18.7 ms, at 64^3 47.8 ->
+// 39.0, 25 at 128^3 400 -> 396); a grid of many waves gains nothing from an
+// early successor, whose blocks then hold shared memory beside its own last
+// ones (25 at 128^3: 431 ms with every launch dependent).
+constexpr long kDepBlocks = 1216;
+template <typename... P, typename... A>
+inline void launch_dep(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                       A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed =
+      (long)grid.x * grid.y * grid.z <= kDepBlocks ? 1 : 0;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k, P(args)...);
 }
 
 // ---------------------------------------------------------------- views
@@ -290,18 +326,19 @@ __device__ __forceinline__ C_t<T> apply_row(const LevelView<T>& L, const C_t<T>*
                                             const T* __restrict__ cells, const Geo<T>& G, T wmu,
                                             const int P[3], long s, const long ss[3],
                                             EdgeCoef<T>& e) {
-  // u, cells and geometry are not written by any thread while a residual,
-  // an assembly or a same-colour block sweep reads them: read-only loads.
-  // Offsets within the RHS's field are 32-bit.
+  // cells and geometry are constant after set-up: read-only loads; u is the
+  // work of the kernel before this one, which may still run when this one is
+  // launched (dep_wait): ordinary loads.  Offsets within the RHS's field are
+  // 32-bit.
   edge_coef<T, C, W>(L.n, P, cells + (long)C * L.ncell, cells + 3 * L.ncell, G, wmu, e, L.imu_vol);
   const int si = (int)s, Si = (int)L.S;
   const int s3[3] = {1, (int)ss[1], (int)ss[2]};
-  const C_t<T> uc = ldro(u + (C * Si + si));
+  const C_t<T> uc = u[C * Si + si];
   T ar = e.dre * uc.x - e.dim * uc.y;
   T ai = e.dre * uc.y + e.dim * uc.x;
 #pragma unroll
   for (int k = 0; k < 12; k++) {
-    const C_t<T> v = ldro(u + (si + nbr_delta32<C>(k, s3, Si)));
+    const C_t<T> v = u[si + nbr_delta32<C>(k, s3, Si)];
     ar += e.c[k] * v.x;
     ai += e.c[k] * v.y;
   }

@@ -16,6 +16,7 @@
 // along d through (ta,tb) reads transverse neighbours at ta+-1 / tb+-1 only
 // (checked by tests/test_coloring.py), so a colour is one parallel launch.
 #include "emmi_line.cuh"
+#include "emmi_node.cuh"
 
 #include <cstdio>
 #include <mutex>
@@ -96,7 +97,7 @@ __device__ __forceinline__ bool is_unknown(const int n[3], const int P[3]) {
   return P[C] < n[C] && P[p] >= 1 && P[p] < n[p] && P[q] >= 1 && P[q] < n[q];
 }
 
-template <typename T, typename TO, int C, int W>
+template <typename T, typename TO, int C>
 __device__ __forceinline__ T residual_comp(const LevelView<T>& L, const C_t<T>* u,
                                                 const C_t<T>* f, const T* cells, const Geo<T>& G,
                                                 T wmu, const int P[3], long s, const long ss[3],
@@ -105,7 +106,7 @@ __device__ __forceinline__ T residual_comp(const LevelView<T>& L, const C_t<T>* 
   C_t<T> r = f ? f[o] : mk<T>(0, 0);     // f null: r = -A u
   if (is_unknown<C>(L.n, P)) {
     EdgeCoef<T> e;
-    const C_t<T> au = apply_row<T, C, W>(L, u, cells, G, wmu, P, s, ss, e);
+    const C_t<T> au = apply_row<T, C, 0>(L, u, cells, G, wmu, P, s, ss, e);
     r = csub<T>(r, au);
   }
   if (rout) rout[o] = mk<TO>((TO)r.x, (TO)r.y);
@@ -114,9 +115,11 @@ __device__ __forceinline__ T residual_comp(const LevelView<T>& L, const C_t<T>* 
 
 // a thread per (component, slot), the component = blockIdx.z: one edge
 // equation per thread keeps more independent loads in flight than three
-template <typename T, typename TO, int W>
+template <typename T, typename TO>
 __global__ void __launch_bounds__(256) k_residual(LevelView<T> L, C_t<TO>* __restrict__ rout,
                                                   double* __restrict__ norm2) {
+  dep_wait();
+  dep_next();
   const int rhs = blockIdx.y;
   if (L.active && !L.active[rhs]) return;
   const long s = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -133,21 +136,59 @@ __global__ void __launch_bounds__(256) k_residual(LevelView<T> L, C_t<TO>* __res
     const T wmu = L.wmu[rhs];
     C_t<TO>* ro = rout ? rout + (long)rhs * 3 * L.S : nullptr;
     switch (blockIdx.z) {
-      case 0: acc = residual_comp<T, TO, 0, W>(L, u, f, cells, G, wmu, P, s, ss, ro); break;
-      case 1: acc = residual_comp<T, TO, 1, W>(L, u, f, cells, G, wmu, P, s, ss, ro); break;
-      default: acc = residual_comp<T, TO, 2, W>(L, u, f, cells, G, wmu, P, s, ss, ro); break;
+      case 0: acc = residual_comp<T, TO, 0>(L, u, f, cells, G, wmu, P, s, ss, ro); break;
+      case 1: acc = residual_comp<T, TO, 1>(L, u, f, cells, G, wmu, P, s, ss, ro); break;
+      default: acc = residual_comp<T, TO, 2>(L, u, f, cells, G, wmu, P, s, ss, ro); break;
     }
   }
   if (norm2) block_add_t<T>(acc, norm2 + rhs);
 }
 
+// the complex64 residual with the coefficients from the spacings: a thread per
+// slot and its three edges, each value they share loaded once (node_residual).
+// Level 0 of 4 RHS at 128^3: 232 us, 3.0 TB/s, where an edge a thread took 318
+// (and the tensor-copy one 316); bound by load latency at 24 warps an SM.
+// Columns of eight planes with the shared values in registers take as long
+// (239 us: fewer loads, 16 warps).
+__global__ void __launch_bounds__(256) k_residual_nodes(LevelView<float> L,
+                                                        float2* __restrict__ rout,
+                                                        double* __restrict__ norm2) {
+  dep_wait();
+  dep_next();
+  const int rhs = blockIdx.y;
+  if (L.active && !L.active[rhs]) return;
+  const long s = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  float acc = 0.f;
+  if (s < L.S) {
+    int P[3];
+    slot_nodes(s, L, P);
+    const int op = op_of(L, rhs);
+    const Geo<float> G{L.geo + (long)op * L.gstride, L.gmax1};
+    float2 r[3], d[3];
+    bool unk[3];
+    node_residual(L, L.u + (long)rhs * 3 * L.S, L.f ? L.f + (long)rhs * 3 * L.S : nullptr,
+                  L.cells + (long)op * 4 * L.ncell, G, L.wmu[rhs], P, (int)s, r, d, unk);
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      if (rout) rout[((long)rhs * 3 + c) * L.S + s] = r[c];
+      acc += r[c].x * r[c].x + r[c].y * r[c].y;
+    }
+  }
+  if (norm2) block_add_t<float>(acc, norm2 + rhs);
+}
+
 template <typename T, typename TO>
 void launch_residual(const LevelView<T>& L, C_t<TO>* rout, double* norm2, cudaStream_t st) {
-  dim3 grid((unsigned)((L.S + 255) / 256), L.nrhs, 3);
-  if (L.imu_vol)
-    k_residual<T, TO, 1><<<grid, 256, 0, st>>>(L, rout, norm2);
-  else
-    k_residual<T, TO, 0><<<grid, 256, 0, st>>>(L, rout, norm2);
+  // with a norm the kernel follows a memset, not another kernel of the cycle
+  auto go = [&](auto k, unsigned nz) {
+    const dim3 grid((unsigned)((L.S + 255) / 256), L.nrhs, nz);
+    if (norm2) k<<<grid, 256, 0, st>>>(L, rout, norm2);
+    else launch_dep(k, grid, 256, 0, st, L, rout, norm2);
+  };
+  if constexpr (sizeof(T) == 4 && sizeof(TO) == 4) {
+    if (L.imu_vol) return go(k_residual_nodes, 1);
+  }
+  go(k_residual<T, TO>, 3);
 }
 
 // ------------------------------------------------------------ stored FP64 coefficients
@@ -349,6 +390,8 @@ template <typename T, int D>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_line_assemble(LevelView<T> L,
                                                                               int pa, int pb,
                                                                               T* __restrict__ buf) {
+  dep_wait();
+  dep_next();
   constexpr int A = (D == 0) ? 1 : 0, B = (D == 2) ? 1 : 2;
   const int rhs = blockIdx.y;
   if (L.active && !L.active[rhs]) return;
@@ -385,6 +428,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_line_assemble(L
 template <typename T, int D>
 __global__ void __launch_bounds__(256) k_line_assemble_rows(LevelView<T> L, int pa, int pb,
                                                             T* __restrict__ buf) {
+  dep_wait();
+  dep_next();
   constexpr int A = (D == 0) ? 1 : 0, B = (D == 2) ? 1 : 2;
   const int rhs = blockIdx.y;
   if (L.active && !L.active[rhs]) return;
@@ -429,6 +474,8 @@ template <typename T>
 __global__ void __launch_bounds__(kSolveThreads) k_line_solve(const int* __restrict__ active,
                                                               long nl, int m,
                                                               T* __restrict__ buf) {
+  dep_wait();
+  dep_next();
   using V = typename Vec16<T>::V;
   constexpr int NP = kPlanes<T>;
   __shared__ V ring[kRing][NP][kSolveThreads];
@@ -544,7 +591,9 @@ __global__ void __launch_bounds__(kSolveThreads) k_line_solve(const int* __restr
 
 template <typename T, int D>
 __global__ void __launch_bounds__(256) k_line_apply(LevelView<T> L, int pa, int pb,
-                                                    const T* __restrict__ buf) {
+                                                    const T* buf) {
+  dep_wait();
+  dep_next();
   const int rhs = blockIdx.y;
   if (L.active && !L.active[rhs]) return;
   const LineGeom g = line_geom<D>(L.n, pa, pb);
@@ -579,13 +628,13 @@ static void line_sweep_d(const LevelView<T>& L, int color, T* buf, cudaStream_t 
   dim3 g1((unsigned)((items + 255) / 256), L.nrhs);
   if (D == 0) {
     dim3 g5((unsigned)((5 * items + 255) / 256), L.nrhs);
-    k_line_assemble_rows<T, D><<<g5, 256, 0, st>>>(L, pa, pb, buf);
+    launch_dep(k_line_assemble_rows<T, D>, g5, 256, 0, st, L, pa, pb, buf);
   } else {
-    k_line_assemble<T, D><<<g1, 256, 0, st>>>(L, pa, pb, buf);
+    launch_dep(k_line_assemble<T, D>, g1, 256, 0, st, L, pa, pb, buf);
   }
   dim3 g2((unsigned)((nl + kSolveThreads - 1) / kSolveThreads), L.nrhs);
-  k_line_solve<T><<<g2, kSolveThreads, 0, st>>>(L.active, nl, m, buf);
-  k_line_apply<T, D><<<g1, 256, 0, st>>>(L, pa, pb, buf);
+  launch_dep(k_line_solve<T>, g2, kSolveThreads, 0, st, L.active, nl, m, buf);
+  launch_dep(k_line_apply<T, D>, g1, 256, 0, st, L, pa, pb, buf);
 }
 // the line solve keeps a cp.async ring in shared memory: ask for the
 // largest shared-memory carveout so 12 blocks fit on an SM
@@ -637,6 +686,8 @@ __device__ __forceinline__ void patch_row(const LevelView<T>& L, const C_t<T>* u
 
 template <typename T>
 __global__ void __launch_bounds__(128) k_point_sweep(LevelView<T> L, int color) {
+  dep_wait();
+  dep_next();
   const int rhs = blockIdx.y;
   if (L.active && !L.active[rhs]) return;
   int cnt[3], first[3];
@@ -706,7 +757,7 @@ void launch_point_sweep(const LevelView<T>& L, int color, cudaStream_t st) {
   }
   if (cnt == 0) return;
   dim3 grid((unsigned)((cnt + 127) / 128), L.nrhs);
-  k_point_sweep<T><<<grid, 128, 0, st>>>(L, color);
+  launch_dep(k_point_sweep<T>, grid, 128, 0, st, L, color);
 }
 
 // ------------------------------------------------------------ transfers
@@ -802,7 +853,7 @@ __device__ __forceinline__ C_t<T> restrict_comp(const LevelView<T>& F, const Lev
 #pragma unroll
       for (int b = 0; b < 4; b++) {
         if (!o2[b]) continue;
-        const C_t<T> v = ldro(rf + (ba + i2[b] * fs[t2]));
+        const C_t<T> v = rf[ba + i2[b] * fs[t2]];
         const T w = w1[a] * w2[b];
         ar += w * v.x;
         ai += w * v.y;
@@ -815,6 +866,8 @@ __device__ __forceinline__ C_t<T> restrict_comp(const LevelView<T>& F, const Lev
 template <typename T>
 __global__ void __launch_bounds__(256) k_restrict(LevelView<T> F, LevelView<T> Cc, int sc0, int sc1,
                                                   int sc2) {
+  dep_wait();
+  dep_next();
   const int rhs = blockIdx.y;
   if (Cc.active && !Cc.active[rhs]) return;
   const long s = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -840,7 +893,7 @@ __global__ void __launch_bounds__(256) k_restrict(LevelView<T> F, LevelView<T> C
 template <typename T>
 void launch_restrict(const LevelView<T>& F, const LevelView<T>& Cc, const int sc[3], cudaStream_t st) {
   dim3 grid((unsigned)((Cc.S + 255) / 256), Cc.nrhs, 3);
-  k_restrict<T><<<grid, 256, 0, st>>>(F, Cc, sc[0], sc[1], sc[2]);
+  launch_dep(k_restrict<T>, grid, 256, 0, st, F, Cc, sc[0], sc[1], sc[2]);
 }
 
 template <typename T, int C>
@@ -873,6 +926,8 @@ __device__ __forceinline__ void prolong_comp(const LevelView<T>& F, const LevelV
 template <typename T>
 __global__ void __launch_bounds__(256) k_prolong(LevelView<T> F, LevelView<T> Cc, int sc0, int sc1,
                                                  int sc2) {
+  dep_wait();
+  dep_next();
   const int rhs = blockIdx.y;
   if (F.active && !F.active[rhs]) return;
   const long s = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -893,7 +948,7 @@ __global__ void __launch_bounds__(256) k_prolong(LevelView<T> F, LevelView<T> Cc
 template <typename T>
 void launch_prolong(const LevelView<T>& F, const LevelView<T>& Cc, const int sc[3], cudaStream_t st) {
   dim3 grid((unsigned)((F.S + 255) / 256), F.nrhs, 3);
-  k_prolong<T><<<grid, 256, 0, st>>>(F, Cc, sc[0], sc[1], sc[2]);
+  launch_dep(k_prolong<T>, grid, 256, 0, st, F, Cc, sc[0], sc[1], sc[2]);
 }
 
 // ------------------------------------------------------------ coarsening
@@ -931,6 +986,8 @@ void launch_coarsen_cells(const T* fine, const int nf[3], T* coarse, const int s
 
 template <typename T>
 __global__ void k_zero(C_t<T>* p, long n) {
+  dep_wait();
+  dep_next();
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
     p[i] = mk<T>(0, 0);
 }
@@ -940,7 +997,7 @@ void launch_zero(C_t<T>* p, long n, cudaStream_t st) {
   long blocks = (n + 255) / 256;
   if (blocks > 4864) blocks = 4864;
   if (blocks < 1) blocks = 1;
-  k_zero<T><<<(unsigned)blocks, 256, 0, st>>>(p, n);
+  launch_dep(k_zero<T>, (unsigned)blocks, 256, 0, st, p, n);
 }
 
 // ------------------------------------------------------------ instantiations

@@ -67,7 +67,7 @@ __host__ __device__ __forceinline__ long rb_elems(const LineTile& t, long nl) {
     return nl * t.m;
 }
 
-template <typename T, int D, int TT, int C, int W>
+template <typename T, int D, int TT, int C>
 __device__ __forceinline__ C_t<T> row_residual(const LevelView<T>& L, const C_t<T>* u,
                                                const C_t<T>* f, const T* cells,
                                                const Geo<T>& G, T wmu, int ta, int tb, int s,
@@ -79,16 +79,18 @@ __device__ __forceinline__ C_t<T> row_residual(const LevelView<T>& L, const C_t<
   P[B] = tb - (TT == 3 ? 1 : 0);
   const int sl = P[0] + (L.n[0] + 1) * (P[1] + (L.n[1] + 1) * P[2]);  // 32-bit slot
   EdgeCoef<T> e;
-  const C_t<T> au = apply_row<T, C, W>(L, u, cells, G, wmu, P, sl, ss, e);
+  const C_t<T> au = apply_row<T, C, 0>(L, u, cells, G, wmu, P, sl, ss, e);
   return csub<T>(f[C * (int)L.S + sl], au);
 }
 
 // rb[rhs][row][line] = residual of every row of one colour; y and z lines:
 // a thread per (line, node) and its five rows; x lines: a thread per
 // (row type, line, node), row type slowest
-template <typename T, int D, int W>
+template <typename T, int D>
 __global__ void __launch_bounds__(256) k_line_rhs(LevelView<T> L, int pa, int pb, LineDiv dv,
                                                   LineTile tl, C_t<T>* __restrict__ rb) {
+  dep_wait();
+  dep_next();
   constexpr int A = (D == 0) ? 1 : 0, B = (D == 2) ? 1 : 2;
   const int rhs = blockIdx.y;
   if (L.active && !L.active[rhs]) return;
@@ -118,19 +120,19 @@ __global__ void __launch_bounds__(256) k_line_rhs(LevelView<T> L, int pa, int pb
   auto put = [&](int row, C_t<T> v) { out[rb_index<T>(tl, g.nl, l, row)] = v; };
   if (D == 0) {
     switch (rt) {
-      case 0: put(r0, row_residual<T, D, 0, D, W>(L, u, f, cells, G, wmu, ta, tb, s, ss)); break;
-      case 1: put(r0 + 1, row_residual<T, D, 1, A, W>(L, u, f, cells, G, wmu, ta, tb, s, ss)); break;
-      case 2: put(r0 + 2, row_residual<T, D, 2, A, W>(L, u, f, cells, G, wmu, ta, tb, s, ss)); break;
-      case 3: put(r0 + 3, row_residual<T, D, 3, B, W>(L, u, f, cells, G, wmu, ta, tb, s, ss)); break;
-      default: put(r0 + 4, row_residual<T, D, 4, B, W>(L, u, f, cells, G, wmu, ta, tb, s, ss)); break;
+      case 0: put(r0, row_residual<T, D, 0, D>(L, u, f, cells, G, wmu, ta, tb, s, ss)); break;
+      case 1: put(r0 + 1, row_residual<T, D, 1, A>(L, u, f, cells, G, wmu, ta, tb, s, ss)); break;
+      case 2: put(r0 + 2, row_residual<T, D, 2, A>(L, u, f, cells, G, wmu, ta, tb, s, ss)); break;
+      case 3: put(r0 + 3, row_residual<T, D, 3, B>(L, u, f, cells, G, wmu, ta, tb, s, ss)); break;
+      default: put(r0 + 4, row_residual<T, D, 4, B>(L, u, f, cells, G, wmu, ta, tb, s, ss)); break;
     }
   } else {
-    put(r0, row_residual<T, D, 0, D, W>(L, u, f, cells, G, wmu, ta, tb, s, ss));
+    put(r0, row_residual<T, D, 0, D>(L, u, f, cells, G, wmu, ta, tb, s, ss));
     if (s < g.nd) {
-      put(r0 + 1, row_residual<T, D, 1, A, W>(L, u, f, cells, G, wmu, ta, tb, s, ss));
-      put(r0 + 2, row_residual<T, D, 2, A, W>(L, u, f, cells, G, wmu, ta, tb, s, ss));
-      put(r0 + 3, row_residual<T, D, 3, B, W>(L, u, f, cells, G, wmu, ta, tb, s, ss));
-      put(r0 + 4, row_residual<T, D, 4, B, W>(L, u, f, cells, G, wmu, ta, tb, s, ss));
+      put(r0 + 1, row_residual<T, D, 1, A>(L, u, f, cells, G, wmu, ta, tb, s, ss));
+      put(r0 + 2, row_residual<T, D, 2, A>(L, u, f, cells, G, wmu, ta, tb, s, ss));
+      put(r0 + 3, row_residual<T, D, 3, B>(L, u, f, cells, G, wmu, ta, tb, s, ss));
+      put(r0 + 4, row_residual<T, D, 4, B>(L, u, f, cells, G, wmu, ta, tb, s, ss));
     }
   }
 }
@@ -158,6 +160,8 @@ template <int D, int NW>
 __global__ void __launch_bounds__(32 * NW, 16 / NW) k_line_rows(LevelView<float> L, int pa, int pb,
                                                        LineDiv dv, LineTile tl, int nodes,
                                                        int lines, float2* __restrict__ rb) {
+  dep_wait();
+  dep_next();
   constexpr int A = (D == 0) ? 1 : 0, B = (D == 2) ? 1 : 2;
   const int rhs = blockIdx.y;
   if (L.active && !L.active[rhs]) return;
@@ -196,11 +200,11 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_line_rows(LevelView<float>
     const bool node = s < g.nd;  // the last node carries its E_D row only
     // edges along D below (0) and above (1) the node, at the five transverse
     // positions; transverse edges - and + of the node
-    const float2 d0 = ldro(ud - sd), d0am = ldro(ud - sd - sa), d0ap = ldro(ud - sd + sa),
-                 d0bm = ldro(ud - sd - sb), d0bp = ldro(ud - sd + sb);
-    const float2 am = ldro(ua - sa), ap = ldro(ua), bm = ldro(ub - sb), bp = ldro(ub);
-    const float2 am_dm = ldro(ua - sa - sd), ap_dm = ldro(ua - sd), bm_dm = ldro(ub - sb - sd),
-                 bp_dm = ldro(ub - sd);
+    const float2 d0 = ud[-sd], d0am = ud[-sd - sa], d0ap = ud[-sd + sa],
+                 d0bm = ud[-sd - sb], d0bp = ud[-sd + sb];
+    const float2 am = ua[-sa], ap = ua[0], bm = ub[-sb], bp = ub[0];
+    const float2 am_dm = ua[-sa - sd], ap_dm = ua[-sd], bm_dm = ub[-sb - sd],
+                 bp_dm = ub[-sd];
     const float sg0 = ldro(gd - cd - ca - cb), sg1 = ldro(gd - cd - ca), sg2 = ldro(gd - cd - cb),
                 sg3 = ldro(gd - cd);
     const float2 f0 = fd[-sd];
@@ -215,23 +219,23 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_line_rows(LevelView<float>
     float2 f1 = zero, f2 = zero, f3 = zero, f4 = zero;
     float sa0 = 0.f, sa1 = 0.f, sb0 = 0.f, sb1 = 0.f, D1 = 1.f;
     if (node) {
-      d1 = ldro(ud);
-      d1am = ldro(ud - sa);
-      d1ap = ldro(ud + sa);
-      d1bm = ldro(ud - sb);
-      d1bp = ldro(ud + sb);
-      am_dp = ldro(ua - sa + sd);
-      ap_dp = ldro(ua + sd);
-      bm_dp = ldro(ub - sb + sd);
-      bp_dp = ldro(ub + sd);
-      am_bm = ldro(ua - sa - sb);
-      am_bp = ldro(ua - sa + sb);
-      ap_bm = ldro(ua - sb);
-      ap_bp = ldro(ua + sb);
-      bm_am = ldro(ub - sb - sa);
-      bm_ap = ldro(ub - sb + sa);
-      bp_am = ldro(ub - sa);
-      bp_ap = ldro(ub + sa);
+      d1 = ud[0];
+      d1am = ud[-sa];
+      d1ap = ud[sa];
+      d1bm = ud[-sb];
+      d1bp = ud[sb];
+      am_dp = ua[-sa + sd];
+      ap_dp = ua[sd];
+      bm_dp = ub[-sb + sd];
+      bp_dp = ub[sd];
+      am_bm = ua[-sa - sb];
+      am_bp = ua[-sa + sb];
+      ap_bm = ua[-sb];
+      ap_bp = ua[sb];
+      bm_am = ub[-sb - sa];
+      bm_ap = ub[-sb + sa];
+      bp_am = ub[-sa];
+      bp_ap = ub[sa];
       f1 = fa[-sa];
       f2 = fa[0];
       f3 = fb[-sb];
@@ -583,12 +587,18 @@ __global__ void __launch_bounds__(D == 0 ? kXThreads : TW == 32 ? 128 : 32)
   constexpr unsigned kFacB = 5 * kRow * TW, kSlot = kFacB + 40 * TW;
   extern __shared__ __align__(16) unsigned char sm[];
   const int rhs = blockIdx.y;
-  if (active && !active[rhs]) return;
+  if (active && !active[rhs]) {
+    dep_wait();
+    return;
+  }
   const int tid = threadIdx.x;
   const int lane = tid & (TW - 1), end = (tid / TW) & 1, tic = D == 0 ? 0 : tid / (2 * TW);
   const int tiles = (int)((nl + TW - 1) / TW);
   const int tile = blockIdx.x * (D == 0 ? 1 : blockDim.x / (2 * TW)) + tic;
-  if (tile >= tiles) return;
+  if (tile >= tiles) {
+    dep_wait();
+    return;
+  }
   const long l = (long)tile * TW + lane;
   const bool live = l < nl;
   const int m = tl.m, G = tl.mid / 5;
@@ -615,10 +625,13 @@ __global__ void __launch_bounds__(D == 0 ? kXThreads : TW == 32 ? 128 : 32)
     const unsigned char* s8 = static_cast<const unsigned char*>(src);
     for (int c = lane; c < bytes / 16; c += TW) cp_async16(dst + 16 * c, s8 + 16 * c);
   };
+  auto issue_fac = [&](int g) { copy(slot(g), fb + (long)(p0 + 5 * g) * kRow * TW, kFacB); };
+  auto issue_rows = [&](int g) {
+    copy(slot(g) + kFacB, rt + (long)(p0 + 5 * g) * TW, 40 * TW);
+  };
   auto issue = [&](int g) {
-    unsigned char* d = slot(g);
-    copy(d, fb + (long)(p0 + 5 * g) * kRow * TW, kFacB);
-    copy(d + kFacB, rt + (long)(p0 + 5 * g) * TW, 40 * TW);
+    issue_fac(g);
+    issue_rows(g);
   };
   // slots of u: row t of group g at off[t] + g * step
   float2* u = nullptr;
@@ -660,6 +673,18 @@ __global__ void __launch_bounds__(D == 0 ? kXThreads : TW == 32 ? 128 : 32)
     }
   };
 
+  // the factors of the first groups and of the middle rows, which no kernel of
+  // a cycle writes, before the wait for the residuals
+  const int at = end * TW + lane;
+#pragma unroll
+  for (int p = 0; p < PD; p++)
+    if (p < G) issue_fac(p);
+  {
+    const unsigned char* mf = fb + (long)tl.mid * kRow * TW;
+    for (int c = at; c < 6 * kRow * TW / 16; c += 2 * TW) cp_async16(midf + 16 * c, mf + 16 * c);
+  }
+  dep_wait();
+  dep_next();
   // forward; the middle rows' u (three an end) is asked for first
   float2 um[3];
   if constexpr (D >= 1) {
@@ -668,16 +693,13 @@ __global__ void __launch_bounds__(D == 0 ? kXThreads : TW == 32 ? 128 : 32)
       um[i] = live ? u[end ? moff[3 + i] : moff[i]] : make_float2(0.f, 0.f);
   }
   {
-    const int at = end * TW + lane;
-    const unsigned char* mf = fb + (long)tl.mid * kRow * TW;
     const unsigned char* mr = reinterpret_cast<const unsigned char*>(rt + (long)tl.mid * TW);
-    for (int c = at; c < 6 * kRow * TW / 16; c += 2 * TW) cp_async16(midf + 16 * c, mf + 16 * c);
     for (int c = at; c < 3 * TW; c += 2 * TW)
       cp_async16(reinterpret_cast<unsigned char*>(midr) + 16 * c, mr + 16 * c);
   }
 #pragma unroll
   for (int p = 0; p < PD; p++) {
-    if (p < G) issue(p);
+    if (p < G) issue_rows(p);
     cp_async_commit();
   }
   float2 w[5];
@@ -802,6 +824,7 @@ __global__ void __launch_bounds__(D == 0 ? kXThreads : TW == 32 ? 128 : 32)
   }
   };
   if (D != 0 || tid < 2 * TW) work();
+  else dep_wait();
   if constexpr (D == 0) {
     // u += x along the lines by the whole block, neighbouring nodes by
     // neighbouring threads (the serial part above occupies 2 TW of them)
@@ -989,6 +1012,8 @@ __global__ void __launch_bounds__(kSolveThreads) k_line_subst(const int* __restr
                                                               long nl, int m,
                                                               const T* __restrict__ fac,
                                                               C_t<T>* __restrict__ rb) {
+  dep_wait();
+  dep_next();
   using V = typename Vec16<T>::V;
   constexpr int NP = kPlanes<T>;
   __shared__ V ring[kRing][NP][kSolveThreads];
@@ -1083,7 +1108,9 @@ __global__ void __launch_bounds__(kSolveThreads) k_line_subst(const int* __restr
 // u += x from rb
 template <typename T, int D>
 __global__ void __launch_bounds__(256) k_line_apply_rb(LevelView<T> L, int pa, int pb, LineDiv dv,
-                                                       LineTile tl, const C_t<T>* __restrict__ rb) {
+                                                       LineTile tl, const C_t<T>* rb) {
+  dep_wait();
+  dep_next();
   const int rhs = blockIdx.y;
   if (L.active && !L.active[rhs]) return;
   const LineGeom g = line_geom<D>(L.n, pa, pb);
@@ -1136,8 +1163,7 @@ static void ends_launch(const EndsArgs& a, int tpc, cudaStream_t st) {
   const long tiles = (a.nl + TW - 1) / TW;
   if (D == 0) tpc = 1;
   dim3 g((unsigned)((tiles + tpc - 1) / tpc), a.L->nrhs);
-  k_line_ends<FMT, TW, NG, D><<<g, D == 0 ? kXThreads : 2 * TW * tpc, tpc * tb, st>>>(
-      a.L->active, a.grp, a.nl, a.tl, a.gstride, a.fac, a.rb, *a.L, a.pa, a.pb, a.dv, slots, tb);
+  launch_dep(k_line_ends<FMT, TW, NG, D>, g, D == 0 ? kXThreads : 2 * TW * tpc, tpc * tb, st, a.L->active, a.grp, a.nl, a.tl, a.gstride, a.fac, a.rb, *a.L, a.pa, a.pb, a.dv, slots, tb);
 }
 
 // the ring of a launch: NG of the shape, one NG for the fp32 format
@@ -1176,7 +1202,7 @@ template <typename T, int D>
 static void apply_rb(const LevelView<T>& L, int pa, int pb, const LineDiv& dv, const LineTile& tl,
                      const C_t<T>* rb, cudaStream_t st) {
   dim3 g1((dv.items + 255) / 256, L.nrhs);
-  k_line_apply_rb<T, D><<<g1, 256, 0, st>>>(L, pa, pb, dv, tl, rb);
+  launch_dep(k_line_apply_rb<T, D>, g1, 256, 0, st, L, pa, pb, dv, tl, rb);
 }
 
 template <int D, int NW>
@@ -1185,7 +1211,7 @@ static void line_rows(const LevelView<float>& L, int pa, int pb, long nl, const 
   const int nodes = (L.n[D] + (D == 0 ? 31 : NW - 1)) / (D == 0 ? 32 : NW);
   const int lines = (int)((nl + (D == 0 ? NW - 1 : 31)) / (D == 0 ? NW : 32));
   dim3 g((unsigned)(nodes * lines), L.nrhs);
-  k_line_rows<D, NW><<<g, 32 * NW, 0, st>>>(L, pa, pb, dv, tl, nodes, lines, rb);
+  launch_dep(k_line_rows<D, NW>, g, 32 * NW, 0, st, L, pa, pb, dv, tl, nodes, lines, rb);
 }
 
 template <typename T, int D>
@@ -1208,7 +1234,7 @@ static void line_sweep_fac_d(const LevelView<T>& L, int color, const T* fac, con
       rows = true;
     }
   }
-  if (!rows) k_line_rhs<T, D, 0><<<gr, rt, 0, st>>>(L, pa, pb, dv, tl, rb);
+  if (!rows) launch_dep(k_line_rhs<T, D>, gr, rt, 0, st, L, pa, pb, dv, tl, rb);
   if constexpr (std::is_same<T, float>::value) {
     const EndsArgs a{&L, grp, nl, tl, line_factor_elems(L.n, D, color, fmt, tile), fac, rb, pa, pb,
                      dv};
@@ -1224,7 +1250,7 @@ static void line_sweep_fac_d(const LevelView<T>& L, int color, const T* fac, con
     if (D == 0 && !res) apply_rb<T, D>(L, pa, pb, dv, tl, rb, st);
   } else {
     dim3 g2((unsigned)((nl + kSolveThreads - 1) / kSolveThreads), L.nrhs);
-    k_line_subst<T><<<g2, kSolveThreads, 0, st>>>(L.active, grp, nl, m, fac, rb);
+    launch_dep(k_line_subst<T>, g2, kSolveThreads, 0, st, L.active, grp, nl, m, fac, rb);
     apply_rb<T, D>(L, pa, pb, dv, tl, rb, st);
   }
 }
@@ -1485,6 +1511,8 @@ template <typename T, int D, int LF, int NT>
 __global__ void __launch_bounds__(NT) k_line_fused(LevelView<T> L, int pa, int pb, LineDiv dv,
                                                    void* __restrict__ lbuf, long lstride,
                                                    int* __restrict__ ovf) {
+  dep_wait();
+  dep_next();
   constexpr int A = (D == 0) ? 1 : 0, B = (D == 2) ? 1 : 2;
   using LS = LineL<T, LF>;
   const int rhs = blockIdx.y;
@@ -1625,6 +1653,8 @@ template <int D, int LF>
 __global__ void __launch_bounds__(64) k_line_fused_ends(LevelView<float> L, int pa, int pb,
                                                         LineDiv dv, int G, void* __restrict__ lbuf,
                                                         long lstride, int* __restrict__ ovf) {
+  dep_wait();
+  dep_next();
   constexpr int A = (D == 0) ? 1 : 0, B = (D == 2) ? 1 : 2;
   using LS = LineL<float, LF>;
   __shared__ float2 ex[20][32];
@@ -1782,13 +1812,12 @@ static void line_fused_d(const LevelView<T>& L, int color, void* lbuf, int lf, i
     dim3 g((unsigned)((nl + 31) / 32), L.nrhs);
     const int G = (L.n[D] - 2) / 2;
     if (lf == kLHalf)
-      k_line_fused_ends<D, kLHalf><<<g, 64, 0, st>>>(L, pa, pb, dv, G, lbuf, lstride, ovf);
+      launch_dep(k_line_fused_ends<D, kLHalf>, g, 64, 0, st, L, pa, pb, dv, G, lbuf, lstride, ovf);
     else
-      k_line_fused_ends<D, kLExact><<<g, 64, 0, st>>>(L, pa, pb, dv, G, lbuf, lstride, ovf);
+      launch_dep(k_line_fused_ends<D, kLExact>, g, 64, 0, st, L, pa, pb, dv, G, lbuf, lstride, ovf);
   } else {
     dim3 g((unsigned)((nl + kSolveThreads - 1) / kSolveThreads), L.nrhs);
-    k_line_fused<T, D, kLExact, kSolveThreads>
-        <<<g, kSolveThreads, 0, st>>>(L, pa, pb, dv, lbuf, lstride, ovf);
+    launch_dep(k_line_fused<T, D, kLExact, kSolveThreads>, g, kSolveThreads, 0, st, L, pa, pb, dv, lbuf, lstride, ovf);
   }
 }
 

@@ -83,6 +83,8 @@ template <typename TO, int W>
 __global__ void __launch_bounds__(kStThreads) k_residual_staged(
     LevelView<float> L, const __grid_constant__ CUtensorMap tu, const __grid_constant__ CUtensorMap tc,
     StencilArgs a, C_t<TO>* __restrict__ rout, double* __restrict__ norm2, int* __restrict__ err) {
+  dep_wait();
+  dep_next();
   extern __shared__ __align__(128) unsigned char sm_raw[];
   __shared__ __align__(8) uint64_t bar[kStRing];
   __shared__ volatile int failed;
@@ -404,6 +406,10 @@ bool stencil_prepare(const LevelView<float>& V, long u_elems, long cell_elems, S
   if (!TY || (TY < std::min(16, Y) && (long)TY * (X - 1) < kStThreads)) return false;
   a.TY = TY;
   a.ntj = (Y + TY - 1) / TY;
+  // a batch whose 32-plane tiles fill the SMs anyway: the plain kernel, which
+  // keeps more loads in flight than one block an SM with its barriers (25 RHS
+  // at 128^3: 1.43 against 1.71 ms)
+  if ((long)a.ntj * ((Z + 31) / 32) * V.nrhs >= 152) return false;
   // planes of a tile: 32 where that gives every SM a CTA (two halo planes in
   // 34), fewer while it does not -- a tile marches its planes one after the
   // other (3 to 4 us a plane), so a small batch left most SMs idle behind 32
