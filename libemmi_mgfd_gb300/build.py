@@ -21,7 +21,7 @@ CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 INCLUDE = os.path.join(ROOT, "include")
 
-GPU_SOURCES = ["emmi_kernels.cu", "emmi_lines.cu", "emmi_solver.cu", "emmi_survey.cu", "emmi_dropin.cu",
+GPU_SOURCES = ["emmi_kernels.cu", "emmi_lines.cu", "emmi_point.cu", "emmi_solver.cu", "emmi_survey.cu", "emmi_dropin.cu",
                "emmi_krylov.cu", "emmi_learned.cu", "emmi_noalloc.cu", "emmi_frontend.cu",
                "emmi_stencil.cu"]
 HOST_SOURCES = ["emmi_host.c", "emmi_fwi.c"]

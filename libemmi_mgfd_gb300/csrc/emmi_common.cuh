@@ -37,6 +37,21 @@ template <typename T> __device__ __forceinline__ C_t<T> cfms(C_t<T> a, C_t<T> b,
 template <typename T> __device__ __forceinline__ C_t<T> crfms(C_t<T> a, T s, C_t<T> b) {
   return mk<T>(a.x - s * b.x, a.y - s * b.y);
 }
+// rounded operations that the compiler does not contract, for kernels that
+// distribute another kernel's arithmetic over lanes and have to round as it
+// does
+__device__ __forceinline__ float rmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double rmul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float rsub(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ double rsub(double a, double b) { return __dsub_rn(a, b); }
+__device__ __forceinline__ float rfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double rfma(double a, double b, double c) { return __fma_rn(a, b, c); }
+// the product b c of cfms as the compiler contracts it: real b.x c.x on
+// -(b.y c.y), imaginary b.y c.x on b.x c.y
+template <typename T> __device__ __forceinline__ C_t<T> cprod_sub(C_t<T> b, C_t<T> c) {
+  return mk<T>(rfma(b.x, c.x, -rmul(b.y, c.y)), rfma(b.y, c.x, rmul(b.x, c.y)));
+}
+
 // 1/z by the scaled formula conj(z)/|z|^2 with a power-of-two prescale so
 // |z|^2 neither overflows nor underflows (Smith-style range guard).
 template <typename T> __device__ __forceinline__ C_t<T> crcp(C_t<T> z) {

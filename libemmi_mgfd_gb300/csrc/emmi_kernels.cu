@@ -659,107 +659,6 @@ void launch_line_sweep(const LevelView<T>& L, int d, int color, C_t<T>* scratch,
   else line_sweep_d<T, 2>(L, color, buf, st);
 }
 
-// ------------------------------------------------------------ point sweep
-// row (C, side): side 0 = E_C(N - e_C), side 1 = E_C(N); patch index 2C+side.
-template <typename T, int C, int SIDE>
-__device__ __forceinline__ void patch_row(const LevelView<T>& L, const C_t<T>* u, const C_t<T>* f,
-                                          const T* cells, const Geo<T>& G, T wmu, const int N[3],
-                                          const long ss[3], C_t<T> (&M)[21], C_t<T> (&y)[6]) {
-  constexpr int p = Cyc<C>::p, q = Cyc<C>::q;
-  constexpr int ri = 2 * C + SIDE;
-  int P[3] = {N[0], N[1], N[2]};
-  P[C] -= 1 - SIDE;
-  const long sl = slot_id(L.n, P[0], P[1], P[2]);
-  EdgeCoef<T> e;
-  const C_t<T> au = apply_row<T, C>(L, u, cells, G, wmu, P, sl, ss, e);
-  y[ri] = csub<T>(f[(long)C * L.S + sl], au);
-  M[WI(ri, ri)] = mk<T>(e.dre, e.dim);
-  // in-patch neighbours: side 0 -> k=4 (p,1), 6 (p,0), 8 (q,1), 10 (q,0);
-  //                      side 1 -> k=5, 7, 9, 11
-  constexpr int kp1 = SIDE ? 5 : 4, kp0 = SIDE ? 7 : 6, kq1 = SIDE ? 9 : 8, kq0 = SIDE ? 11 : 10;
-  constexpr int ip1 = 2 * p + 1, ip0 = 2 * p, iq1 = 2 * q + 1, iq0 = 2 * q;
-  if constexpr (ip1 < ri) M[WI(ri, ip1)] = mk<T>(e.c[kp1], 0);
-  if constexpr (ip0 < ri) M[WI(ri, ip0)] = mk<T>(e.c[kp0], 0);
-  if constexpr (iq1 < ri) M[WI(ri, iq1)] = mk<T>(e.c[kq1], 0);
-  if constexpr (iq0 < ri) M[WI(ri, iq0)] = mk<T>(e.c[kq0], 0);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(128) k_point_sweep(LevelView<T> L, int color) {
-  dep_wait();
-  dep_next();
-  const int rhs = blockIdx.y;
-  if (L.active && !L.active[rhs]) return;
-  int cnt[3], first[3];
-#pragma unroll
-  for (int e = 0; e < 3; e++) {
-    const int par = (color >> e) & 1;
-    first[e] = par ? 1 : 2;
-    cnt[e] = (L.n[e] - 1 >= first[e]) ? (L.n[e] - 1 - first[e]) / 2 + 1 : 0;
-  }
-  const long tot = (long)cnt[0] * cnt[1] * cnt[2];
-  const long id = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (id >= tot) return;
-  const int N[3] = {first[0] + 2 * (int)(id % cnt[0]), first[1] + 2 * (int)((id / cnt[0]) % cnt[1]),
-                    first[2] + 2 * (int)(id / ((long)cnt[0] * cnt[1]))};
-  const int n0 = L.n[0] + 1, n1 = L.n[1] + 1;
-  const long ss[3] = {1, (long)n0, (long)n0 * n1};
-  C_t<T>* u = L.u + (long)rhs * 3 * L.S;
-  const C_t<T>* f = L.f + (long)rhs * 3 * L.S;
-  const T* cells = L.cells + (long)op_of(L, rhs) * 4 * L.ncell;
-  const Geo<T> G{L.geo + (long)op_of(L, rhs) * L.gstride, L.gmax1};
-  const T wmu = L.wmu[rhs];
-  C_t<T> M[21], y[6];
-#pragma unroll
-  for (int i = 0; i < 21; i++) M[i] = mk<T>(0, 0);
-  patch_row<T, 0, 0>(L, u, f, cells, G, wmu, N, ss, M, y);
-  patch_row<T, 0, 1>(L, u, f, cells, G, wmu, N, ss, M, y);
-  patch_row<T, 1, 0>(L, u, f, cells, G, wmu, N, ss, M, y);
-  patch_row<T, 1, 1>(L, u, f, cells, G, wmu, N, ss, M, y);
-  patch_row<T, 2, 0>(L, u, f, cells, G, wmu, N, ss, M, y);
-  patch_row<T, 2, 1>(L, u, f, cells, G, wmu, N, ss, M, y);
-  // dense complex-symmetric LDL^T on the lower triangle
-  C_t<T> Lm[21], z[6];
-#pragma unroll
-  for (int k = 0; k < 6; k++) {
-    const C_t<T> id = crcp<T>(M[WI(k, k)]);
-#pragma unroll
-    for (int i = k + 1; i < 6; i++) {
-      const C_t<T> l = cmul<T>(M[WI(i, k)], id);
-#pragma unroll
-      for (int j = k + 1; j <= i; j++) M[WI(i, j)] = cfms<T>(M[WI(i, j)], l, M[WI(j, k)]);
-      y[i] = cfms<T>(y[i], l, y[k]);
-      Lm[WI(i, k)] = l;
-    }
-    z[k] = cmul<T>(y[k], id);
-  }
-#pragma unroll
-  for (int k = 5; k >= 0; k--) {
-#pragma unroll
-    for (int i = k + 1; i < 6; i++) z[k] = cfms<T>(z[k], Lm[WI(i, k)], z[i]);
-  }
-#pragma unroll
-  for (int ri = 0; ri < 6; ri++) {
-    const int c = ri / 2;
-    int P[3] = {N[0], N[1], N[2]};
-    P[c] -= 1 - (ri & 1);
-    const long sl = (long)c * L.S + slot_id(L.n, P[0], P[1], P[2]);
-    u[sl] = cadd<T>(u[sl], z[ri]);
-  }
-}
-
-template <typename T>
-void launch_point_sweep(const LevelView<T>& L, int color, cudaStream_t st) {
-  long cnt = 1;
-  for (int e = 0; e < 3; e++) {
-    const int par = (color >> e) & 1, first = par ? 1 : 2;
-    cnt *= (L.n[e] - 1 >= first) ? (L.n[e] - 1 - first) / 2 + 1 : 0;
-  }
-  if (cnt == 0) return;
-  dim3 grid((unsigned)((cnt + 127) / 128), L.nrhs);
-  launch_dep(k_point_sweep<T>, grid, 128, 0, st, L, color);
-}
-
 // ------------------------------------------------------------ transfers
 template <typename T>
 struct Xfer {
@@ -1004,7 +903,6 @@ void launch_zero(C_t<T>* p, long n, cudaStream_t st) {
 #define EMMI_INST(T)                                                                               \
   template void launch_norm<T>(const C_t<T>*, long, int, const int*, double*, cudaStream_t);        \
   template void launch_line_sweep<T>(const LevelView<T>&, int, int, C_t<T>*, cudaStream_t);         \
-  template void launch_point_sweep<T>(const LevelView<T>&, int, cudaStream_t);                      \
   template void launch_restrict<T>(const LevelView<T>&, const LevelView<T>&, const int*,            \
                                    cudaStream_t);                                                   \
   template void launch_prolong<T>(const LevelView<T>&, const LevelView<T>&, const int*,             \

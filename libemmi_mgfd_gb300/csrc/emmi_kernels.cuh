@@ -43,7 +43,8 @@ long line_scratch_elems(const int n[3], int d, int nrhs);
 // unused), the band rows assembled in registers, into fac + g *
 // line_factor_elems and sets *ovf when an L value does not fit fp16 (kFacF16);
 // launch_line_sweep_fac then sweeps RHS r with the factors of group grp[r], rb
-// holding line_rb_elems complex values per RHS in line_fac_launches launches
+// holding line_rb_elems complex values per RHS, in line_fac_launches launches;
+// coef (complex128, may be null): launch_coef64's coefficients of the level
 constexpr int kFacF32 = 0, kFacF16 = 1;
 int line_tile_width(const int n[3], int d, int nrhs, int fmt);
 long line_factor_elems(const int n[3], int d, int color, int fmt, int tile);
@@ -68,7 +69,7 @@ void init_stored_line_kernels();
 template <typename T>
 void launch_line_sweep_fac(const LevelView<T>& L, int d, int color, const T* fac, const int* grp,
                            C_t<T>* rb, int fmt, int tile, cudaStream_t st,
-                           SweepShape sh = SweepShape());
+                           SweepShape sh = SweepShape(), const double* coef = nullptr);
 
 // one colour of line relaxation along d in one launch (k_line_fused,
 // k_line_fused_ends): assembles, factors and solves the lines; z waits in L.r
@@ -113,6 +114,27 @@ int* stencil_err();
 
 template <typename T>
 void launch_point_sweep(const LevelView<T>& L, int color, cudaStream_t st);
+// the same sweeps from stored coefficients and patch factors (emmi_point.cu):
+// launch_point_setup fills coef (point_coef_elems values per operator of ops)
+// and pf (point_factor_elems complex values per group of groups, its L.op and
+// L.wmu); launch_point_coarse runs nrep sweeps of a level whose u and f fit a
+// block's shared memory (point_coarse_smem bytes <= kPointSmem), bit r of rev
+// reversing the colours of sweep r, zero starting from u = 0;
+// launch_point_lanes one colour
+constexpr int kPointSmem = 200 << 10;
+size_t point_coarse_smem(const int n[3], int csize);
+bool point_in_block(const int n[3], int csize);
+long point_coef_elems(const int n[3]);
+long point_factor_elems(const int n[3]);
+template <typename T>
+void launch_point_setup(const LevelView<T>& ops, T* coef, const LevelView<T>& groups, C_t<T>* pf,
+                        cudaStream_t st);
+template <typename T>
+void launch_point_coarse(const LevelView<T>& L, const T* coef, const C_t<T>* pf, const int* grp,
+                         int nrep, unsigned rev, bool zero, cudaStream_t st);
+template <typename T>
+void launch_point_lanes(const LevelView<T>& L, int color, const T* coef, const C_t<T>* pf,
+                        const int* grp, cudaStream_t st);
 
 // coarse.f = R fine.r ; coarse.u = 0
 // LevelView::xw of the transfer F -> Cc for every operator (set-up)

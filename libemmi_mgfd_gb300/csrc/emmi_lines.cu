@@ -83,12 +83,52 @@ __device__ __forceinline__ C_t<T> row_residual(const LevelView<T>& L, const C_t<
   return csub<T>(f[C * (int)L.S + sl], au);
 }
 
-// rb[rhs][row][line] = residual of every row of one colour; y and z lines:
+// the same from stored coefficients (coef64_elems per operator: planes
+// [10][3][S], see emmi_kernels.cu), applied in edge_coef / apply_row's order:
+// 30 FP64 instructions a row where recomputing the coefficients takes eight
+// divisions of 13 besides (one RHS at 16^3 32 -> 18 us a launch, four at
+// 64 x 56 x 48 60 -> 23)
+template <int D, int TT, int C>
+__device__ __forceinline__ double2 row_residual_coef(const LevelView<double>& L, const double2* u,
+                                                     const double2* f,
+                                                     const double* __restrict__ cf, double wmu,
+                                                     int ta, int tb, int s, const long ss[3]) {
+  constexpr int A = (D == 0) ? 1 : 0, B = (D == 2) ? 1 : 2;
+  int P[3];
+  P[D] = (TT == 0) ? s - 1 : s;
+  P[A] = ta - (TT == 1 ? 1 : 0);
+  P[B] = tb - (TT == 3 ? 1 : 0);
+  const int S = (int)L.S;
+  const int sl = P[0] + (L.n[0] + 1) * (P[1] + (L.n[1] + 1) * P[2]), o = C * S + sl;
+  const long n3s = 3 * L.S;
+  double k[10];
+#pragma unroll
+  for (int c = 0; c < 10; c++) k[c] = ldro(cf + c * n3s + o);
+  const double c12[12] = {k[0], k[1], k[2], k[3], k[4], -k[4], -k[5], k[5],
+                          k[6], -k[6], -k[7], k[7]};
+  const double dre = k[8], dim = -wmu * k[9];
+  const int s3[3] = {1, (int)ss[1], (int)ss[2]};
+  const double2 uc = u[o];
+  // the diagonal's product contracted as apply_row's is
+  double ar = rfma(dre, uc.x, -rmul(dim, uc.y));
+  double ai = rfma(dre, uc.y, rmul(dim, uc.x));
+#pragma unroll
+  for (int c = 0; c < 12; c++) {
+    const double2 v = u[sl + nbr_delta32<C>(c, s3, S)];
+    ar = rfma(c12[c], v.x, ar);
+    ai = rfma(c12[c], v.y, ai);
+  }
+  const double2 r = f[o];
+  return mk<double>(rsub(r.x, ar), rsub(r.y, ai));
+}
+
+// rb = residual of every row of one colour; y and z lines:
 // a thread per (line, node) and its five rows; x lines: a thread per
 // (row type, line, node), row type slowest
-template <typename T, int D>
+template <typename T, int D, bool CF>
 __global__ void __launch_bounds__(256) k_line_rhs(LevelView<T> L, int pa, int pb, LineDiv dv,
-                                                  LineTile tl, C_t<T>* __restrict__ rb) {
+                                                  LineTile tl, C_t<T>* __restrict__ rb,
+                                                  const double* __restrict__ coef) {
   dep_wait();
   dep_next();
   constexpr int A = (D == 0) ? 1 : 0, B = (D == 2) ? 1 : 2;
@@ -117,22 +157,28 @@ __global__ void __launch_bounds__(256) k_line_rhs(LevelView<T> L, int pa, int pb
   const T wmu = L.wmu[rhs];
   C_t<T>* out = rb + (long)rhs * rb_elems<T>(tl, g.nl);
   const int r0 = 5 * (s - 1);
+  const double* cf = CF ? coef + (long)op_of(L, rhs) * 30 * L.S : nullptr;
+  auto row = [&](auto tt, auto comp) {
+    constexpr int TT = decltype(tt)::value, C = decltype(comp)::value;
+    if constexpr (CF) return row_residual_coef<D, TT, C>(L, u, f, cf, wmu, ta, tb, s, ss);
+    else return row_residual<T, D, TT, C>(L, u, f, cells, G, wmu, ta, tb, s, ss);
+  };
   auto put = [&](int row, C_t<T> v) { out[rb_index<T>(tl, g.nl, l, row)] = v; };
   if (D == 0) {
     switch (rt) {
-      case 0: put(r0, row_residual<T, D, 0, D>(L, u, f, cells, G, wmu, ta, tb, s, ss)); break;
-      case 1: put(r0 + 1, row_residual<T, D, 1, A>(L, u, f, cells, G, wmu, ta, tb, s, ss)); break;
-      case 2: put(r0 + 2, row_residual<T, D, 2, A>(L, u, f, cells, G, wmu, ta, tb, s, ss)); break;
-      case 3: put(r0 + 3, row_residual<T, D, 3, B>(L, u, f, cells, G, wmu, ta, tb, s, ss)); break;
-      default: put(r0 + 4, row_residual<T, D, 4, B>(L, u, f, cells, G, wmu, ta, tb, s, ss)); break;
+      case 0: put(r0, row(std::integral_constant<int, 0>(), std::integral_constant<int, D>())); break;
+      case 1: put(r0 + 1, row(std::integral_constant<int, 1>(), std::integral_constant<int, A>())); break;
+      case 2: put(r0 + 2, row(std::integral_constant<int, 2>(), std::integral_constant<int, A>())); break;
+      case 3: put(r0 + 3, row(std::integral_constant<int, 3>(), std::integral_constant<int, B>())); break;
+      default: put(r0 + 4, row(std::integral_constant<int, 4>(), std::integral_constant<int, B>())); break;
     }
   } else {
-    put(r0, row_residual<T, D, 0, D>(L, u, f, cells, G, wmu, ta, tb, s, ss));
+    put(r0, row(std::integral_constant<int, 0>(), std::integral_constant<int, D>()));
     if (s < g.nd) {
-      put(r0 + 1, row_residual<T, D, 1, A>(L, u, f, cells, G, wmu, ta, tb, s, ss));
-      put(r0 + 2, row_residual<T, D, 2, A>(L, u, f, cells, G, wmu, ta, tb, s, ss));
-      put(r0 + 3, row_residual<T, D, 3, B>(L, u, f, cells, G, wmu, ta, tb, s, ss));
-      put(r0 + 4, row_residual<T, D, 4, B>(L, u, f, cells, G, wmu, ta, tb, s, ss));
+      put(r0 + 1, row(std::integral_constant<int, 1>(), std::integral_constant<int, A>()));
+      put(r0 + 2, row(std::integral_constant<int, 2>(), std::integral_constant<int, A>()));
+      put(r0 + 3, row(std::integral_constant<int, 3>(), std::integral_constant<int, B>()));
+      put(r0 + 4, row(std::integral_constant<int, 4>(), std::integral_constant<int, B>()));
     }
   }
 }
@@ -1105,6 +1151,112 @@ __global__ void __launch_bounds__(kSolveThreads) k_line_subst(const int* __restr
 }
 
 
+// The same substitution with 12 lanes a line, two lines a warp, for few lines:
+// an FP64 instruction takes an SM quarter about 60 clocks however many of a
+// warp's lanes are active and however independent the instructions are, so
+// what a line's chain costs is the number of instructions, not of operations.
+// Lane 2 j + part of a line holds the real or imaginary part of the rows with
+// row % 6 == j.  Forward, a pivot's value is shuffled to the lanes of the five
+// rows that follow, which take their product with the multiplier off it, while
+// the pivot's lane forms z with the same instructions: three an FP64 row in
+// place of 34.  Backward, the five products are formed in the lanes of the
+// known x and subtracted in the pivot's, newest first: seven in place of 30.
+// k_line_subst's operations in its order, the same result bit for bit.
+// Mean over a cycle's launches: one RHS at 16^3 71 -> 27 us, four at
+// 64 x 56 x 48 170 -> 87.
+__global__ void __launch_bounds__(128) k_line_subst_lanes(const int* __restrict__ active,
+                                                          const int* __restrict__ grp, long nl,
+                                                          int m, const double* __restrict__ fac,
+                                                          double2* rb) {
+  dep_wait();
+  dep_next();
+  const int rhs = blockIdx.y;
+  if (active && !active[rhs]) return;
+  const int lane = threadIdx.x & 31;
+  const long w = blockIdx.x * 4L + (threadIdx.x >> 5);
+  if (2 * w >= nl) return;  // a warp at a time
+  const int sub = lane < 12 ? 0 : lane < 24 ? 1 : 2, base = sub * 12;
+  const bool live = sub < 2 && 2 * w + sub < nl;
+  const long l = live ? 2 * w + sub : 2 * w;
+  const int j = ((lane - base) >> 1) % 6, part = (lane - base) & 1;
+  const int src = sub < 2 ? base : 0;  // idle lanes shuffle from the first line
+  const long rs = 6 * nl;
+  const double2* fb = reinterpret_cast<const double2*>(fac) + (long)grp[rhs] * m * rs + l;
+  double* rr = reinterpret_cast<double*>(rb + (long)rhs * m * nl + l) + part;
+  auto role = [&](int u) { return j >= u ? j - u : j - u + 6; };  // (j - u) mod 6
+  auto factor = [&](int row, int i) -> double2 {                  // L_i, 1/d for i = 0
+    return row < m ? ldro(fb + row * rs + (i == 0 ? 5 : i - 1) * nl) : make_double2(0.0, 0.0);
+  };
+  auto res = [&](int row) { return row < m ? rr[2 * (long)row * nl] : 0.0; };
+  double2 cur[6], nxt[6];
+  double rn, y = res(j);
+#pragma unroll
+  for (int u = 0; u < 6; u++) cur[u] = factor(u, role(u));
+  for (int p0 = 0; p0 < m; p0 += 6) {
+    // the next six rows: multipliers, and the residual this lane takes next
+    rn = res(p0 + 6 + j);
+#pragma unroll
+    for (int u = 0; u < 6; u++) nxt[u] = factor(p0 + 6 + u, role(u));
+#pragma unroll
+    for (int u = 0; u < 6; u++) {
+      const double yx = __shfl_sync(0xffffffffu, y, src + 2 * u);
+      const double yy = __shfl_sync(0xffffffffu, y, src + 2 * u + 1);
+      const bool piv = j == u;
+      const double2 v = cur[u];
+      // as cfms(., L, y) and, for z, cmul(y, 1/d) round: real L.x y.x with
+      // -(L.y y.y) rounded first, imaginary L.y y.x on L.x y.y (z: y.y d.x on
+      // y.x d.y)
+      const bool sw = part && !piv;
+      const double a = sw ? v.y : v.x, b = part && piv ? yy : yx;
+      const double c = sw ? v.x : v.y, d = part ? (piv ? yx : yy) : -yy;
+      const double t = rfma(a, b, rmul(c, d));
+      const int row = p0 + u;
+      if (piv) {
+        if (live && row < m) rr[2 * (long)row * nl] = t;  // z
+        y = rn;
+      } else {
+        y = rsub(y, t);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 6; u++) cur[u] = nxt[u];
+  }
+  __syncwarp();
+  // backward: x_k = z_k - sum_i L(k+i, k) x_{k+i}
+  double x = 0.0;
+  const int c0 = (m - 1) / 6 * 6;
+  auto back = [&](int row, int u) -> double2 {  // multipliers, z in the pivot's lane
+    if (row >= m) return make_double2(0.0, 0.0);
+    return role(u) == 0 ? make_double2(rr[2 * (long)row * nl], 0.0)
+                        : ldro(fb + row * rs + (role(u) - 1) * nl);
+  };
+#pragma unroll
+  for (int u = 0; u < 6; u++) cur[u] = back(c0 + u, u);
+  for (int p0 = c0; p0 >= 0; p0 -= 6) {
+    if (p0 >= 6) {
+#pragma unroll
+      for (int u = 0; u < 6; u++) nxt[u] = back(p0 - 6 + u, u);
+    }
+#pragma unroll
+    for (int u = 5; u >= 0; u--) {
+      const double xo = __shfl_xor_sync(0xffffffffu, x, 1);
+      const double2 v = cur[u];
+      const double t = part ? rfma(v.y, xo, rmul(v.x, x)) : rfma(v.x, x, -rmul(v.y, xo));
+      double s = v.x;  // z in the pivot's lane
+#pragma unroll
+      for (int q = 1; q < 6; q++)
+        s = rsub(s, __shfl_sync(0xffffffffu, t, src + 2 * ((u + q) % 6) + part));
+      const int row = p0 + u;
+      if (j == u && row < m) {
+        x = s;
+        if (live) rr[2 * (long)row * nl] = x;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 6; u++) cur[u] = nxt[u];
+  }
+}
+
 // u += x from rb
 template <typename T, int D>
 __global__ void __launch_bounds__(256) k_line_apply_rb(LevelView<T> L, int pa, int pb, LineDiv dv,
@@ -1205,6 +1357,8 @@ static void apply_rb(const LevelView<T>& L, int pa, int pb, const LineDiv& dv, c
   launch_dep(k_line_apply_rb<T, D>, g1, 256, 0, st, L, pa, pb, dv, tl, rb);
 }
 
+constexpr long kLaneLines = 7680;
+
 template <int D, int NW>
 static void line_rows(const LevelView<float>& L, int pa, int pb, long nl, const LineDiv& dv,
                       const LineTile& tl, float2* rb, cudaStream_t st) {
@@ -1216,7 +1370,8 @@ static void line_rows(const LevelView<float>& L, int pa, int pb, long nl, const 
 
 template <typename T, int D>
 static void line_sweep_fac_d(const LevelView<T>& L, int color, const T* fac, const int* grp,
-                             C_t<T>* rb, int fmt, int tile, SweepShape sh, cudaStream_t st) {
+                             C_t<T>* rb, int fmt, int tile, SweepShape sh, const double* coef,
+                             cudaStream_t st) {
   const int pa = color & 1, pb = (color >> 1) & 1;
   const long nl = line_count(L.n, D, color);
   if (nl == 0) return;
@@ -1234,7 +1389,15 @@ static void line_sweep_fac_d(const LevelView<T>& L, int color, const T* fac, con
       rows = true;
     }
   }
-  if (!rows) launch_dep(k_line_rhs<T, D>, gr, rt, 0, st, L, pa, pb, dv, tl, rb);
+  if (!rows) {
+    if constexpr (std::is_same<T, double>::value) {
+      if (coef) {
+        launch_dep(k_line_rhs<T, D, true>, gr, rt, 0, st, L, pa, pb, dv, tl, rb, coef);
+        rows = true;
+      }
+    }
+    if (!rows) launch_dep(k_line_rhs<T, D, false>, gr, rt, 0, st, L, pa, pb, dv, tl, rb, nullptr);
+  }
   if constexpr (std::is_same<T, float>::value) {
     const EndsArgs a{&L, grp, nl, tl, line_factor_elems(L.n, D, color, fmt, tile), fac, rb, pa, pb,
                      dv};
@@ -1249,8 +1412,16 @@ static void line_sweep_fac_d(const LevelView<T>& L, int color, const T* fac, con
     }
     if (D == 0 && !res) apply_rb<T, D>(L, pa, pb, dv, tl, rb, st);
   } else {
-    dim3 g2((unsigned)((nl + kSolveThreads - 1) / kSolveThreads), L.nrhs);
-    launch_dep(k_line_subst<T>, g2, kSolveThreads, 0, st, L.active, grp, nl, m, fac, rb);
+    // 12 lanes a line while that is shorter: two lines a warp and 10 FP64
+    // instructions a row against 32 lines and 64, on 4 x 152 SM quarters --
+    // 60 clocks x 10 x lines / 1216 a row against 60 x 64
+    if (nl * L.nrhs <= kLaneLines) {
+      launch_dep(k_line_subst_lanes, dim3((unsigned)((nl + 7) / 8), L.nrhs), dim3(128), 0, st,
+                 L.active, grp, nl, m, fac, rb);
+    } else {
+      dim3 g2((unsigned)((nl + kSolveThreads - 1) / kSolveThreads), L.nrhs);
+      launch_dep(k_line_subst<T>, g2, kSolveThreads, 0, st, L.active, grp, nl, m, fac, rb);
+    }
     apply_rb<T, D>(L, pa, pb, dv, tl, rb, st);
   }
 }
@@ -1308,10 +1479,11 @@ void launch_line_factor(const LevelView<T>& L, int d, int color, T* fac, int fmt
 
 template <typename T>
 void launch_line_sweep_fac(const LevelView<T>& L, int d, int color, const T* fac, const int* grp,
-                           C_t<T>* rb, int fmt, int tile, cudaStream_t st, SweepShape sh) {
-  if (d == 0) line_sweep_fac_d<T, 0>(L, color, fac, grp, rb, fmt, tile, sh, st);
-  else if (d == 1) line_sweep_fac_d<T, 1>(L, color, fac, grp, rb, fmt, tile, sh, st);
-  else line_sweep_fac_d<T, 2>(L, color, fac, grp, rb, fmt, tile, sh, st);
+                           C_t<T>* rb, int fmt, int tile, cudaStream_t st, SweepShape sh,
+                           const double* coef) {
+  if (d == 0) line_sweep_fac_d<T, 0>(L, color, fac, grp, rb, fmt, tile, sh, coef, st);
+  else if (d == 1) line_sweep_fac_d<T, 1>(L, color, fac, grp, rb, fmt, tile, sh, coef, st);
+  else line_sweep_fac_d<T, 2>(L, color, fac, grp, rb, fmt, tile, sh, coef, st);
 }
 template void launch_line_factor<float>(const LevelView<float>&, int, int, float*, int, int, int*,
                                         cudaStream_t);
@@ -1319,10 +1491,10 @@ template void launch_line_factor<double>(const LevelView<double>&, int, int, dou
                                          int*, cudaStream_t);
 template void launch_line_sweep_fac<float>(const LevelView<float>&, int, int, const float*,
                                            const int*, C_t<float>*, int, int, cudaStream_t,
-                                           SweepShape);
+                                           SweepShape, const double*);
 template void launch_line_sweep_fac<double>(const LevelView<double>&, int, int, const double*,
                                             const int*, C_t<double>*, int, int, cudaStream_t,
-                                            SweepShape);
+                                            SweepShape, const double*);
 
 // ---------------------------------------------------------------- fused line relaxation
 // One launch per colour and direction.  A thread owns one line and walks it

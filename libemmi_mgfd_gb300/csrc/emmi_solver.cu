@@ -362,7 +362,8 @@ static void line_colour(emmi_solver* s, int h, int l, int d, int col, const Leve
     if (off >= 0) {
       launch_line_sweep_fac<T>(W, d, col, static_cast<const T*>(s->d_fac) + off, s->d_grp + r0,
                                (C_t<T>*)s->scratch, s->fac_fmt,
-                               s->fac_tile[l == 0 ? 0 : h][l][d], s->st, s->shape[l][d]);
+                               s->fac_tile[l == 0 ? 0 : h][l][d], s->st, s->shape[l][d],
+                               s->coef64[h][l]);
       return;
     }
   }
@@ -406,11 +407,35 @@ void emmi_solver::emit_smooth(int h, int l, int iter) {
       }
     }
   } else {
+    const bool stored = l == lmax - 1 && pt_coef[h];
     for (int cc = 0; cc < 8; cc++) {
-      launch_point_sweep<T>(V, rev ? 7 - cc : cc, st);
+      const int col = rev ? 7 - cc : cc;
+      if (stored)
+        launch_point_lanes<T>(V, col, static_cast<const T*>(pt_coef[h]),
+                              static_cast<const C_t<T>*>(pt_fac[h]), d_grp, st);
+      else
+        launch_point_sweep<T>(V, col, st);
       launch_counter++;
     }
   }
+}
+
+// every sweep of a visit to the coarsest level in one launch (zero: from
+// u = 0); false where it does not fit a block or there is nothing stored
+template <typename T>
+bool emmi_solver::emit_coarsest(int h, bool zero) {
+  const int l = lmax - 1;
+  const int pre = (opt.skip_pre >> l) & 1 ? 0 : opt.v1, post = (opt.skip_post >> l) & 1 ? 0 : opt.v2;
+  if (!pt_coef[h] || !pt_block[h] || pre + post < 1 || pre + post > 32 ||
+      hier[h][l].n[0] < 2 || hier[h][l].n[1] < 2 || hier[h][l].n[2] < 2)
+    return false;
+  unsigned rev = 0;
+  for (int i = 0; i < pre; i++) rev |= (unsigned)(i & 1) << i;
+  for (int i = 0; i < post; i++) rev |= (unsigned)(i & 1) << (pre + i);
+  launch_point_coarse<T>(view<T>(h, l), static_cast<const T*>(pt_coef[h]),
+                         static_cast<const C_t<T>*>(pt_fac[h]), d_grp, pre + post, rev, zero, st);
+  launch_counter++;
+  return true;
 }
 
 // r = f - A u of level l of hierarchy h (view V): the staged kernel where
@@ -420,6 +445,12 @@ void emmi_solver::resid(int h, int l, const LevelView<T>& V, C_t<T>* rout, doubl
   if constexpr (std::is_same<T, float>::value) {
     if (plan[h][l].ok) {
       launch_residual_staged(V, plan[h][l], rout, norm2, st);
+      return;
+    }
+  }
+  if constexpr (std::is_same<T, double>::value) {
+    if (coef64[h][l]) {
+      launch_residual_coef<T>(V, coef64[h][l], rout, norm2, st);
       return;
     }
   }
@@ -472,6 +503,7 @@ void emmi_solver::emit_cycle(int h, int l, int kind, int want, int& cur) {
   if (kind == 2) {  // F
     if (l == lmax - 1) {
       if (cur == want) {
+        if (emit_coarsest<T>(h, true)) return;
         LevelView<T> V = view<T>(h, l);
         launch_zero<T>(V.u, 3 * V.S * nrhs, st);
         launch_counter++;
@@ -487,6 +519,7 @@ void emmi_solver::emit_cycle(int h, int l, int kind, int want, int& cur) {
   }
   // V (kind 1) and W (kind 3); levels whose bit is set in skip_pre /
   // skip_post leave out that smoothing
+  if (l == lmax - 1 && l > 0 && !can_descend(l) && cur == want && emit_coarsest<T>(h, false)) return;
   if (!((opt.skip_pre >> l) & 1))
     for (int i = 0; i < opt.v1; i++) smooth(l, i);
   if (can_descend(l)) {
@@ -526,13 +559,9 @@ int emmi_solver::build_graphs() {
   return EMMI_OK;
 }
 
-// Stored line factors of the complex64 cycle: group the RHS by (operator,
-// frequency), size the factor blocks of every (hierarchy, level, direction,
-// colour) the smoother relaxes, and factor each group's lines once.  Leaves
-// fac_on false (factoring in every sweep) when they would take more than
-// half of the free device memory.
+// The RHS grouped by (operator, frequency): what is factored, once a group
 template <typename T>
-static int build_line_factors(emmi_solver* s) {
+static int build_groups(emmi_solver* s) {
   const int nrhs = s->nrhs;
   std::vector<int> grp(nrhs), gop;
   std::vector<T> gw;
@@ -548,7 +577,66 @@ static int build_line_factors(emmi_solver* s) {
     }
     grp[r] = g;
   }
-  const int ng = (int)gop.size();
+  const int ng = s->ngroups = (int)gop.size();
+  int rc;
+  if ((rc = s->alloc((void**)&s->d_grp, nrhs * sizeof(int))) != EMMI_OK) return rc;
+  if ((rc = s->alloc((void**)&s->d_gop, ng * sizeof(int))) != EMMI_OK) return rc;
+  if ((rc = s->alloc((void**)&s->d_gwmu, ng * sizeof(T))) != EMMI_OK) return rc;
+  CK(cudaMemcpyAsync(s->d_grp, grp.data(), nrhs * sizeof(int), cudaMemcpyHostToDevice, s->st));
+  CK(cudaMemcpyAsync(s->d_gop, gop.data(), ng * sizeof(int), cudaMemcpyHostToDevice, s->st));
+  CK(cudaMemcpyAsync(s->d_gwmu, gw.data(), ng * sizeof(T), cudaMemcpyHostToDevice, s->st));
+  CK(cudaStreamSynchronize(s->st));  // the host arrays end here
+  return EMMI_OK;
+}
+
+// Stored coefficients and patch factors of the coarsest level of every
+// hierarchy, for the node-patch sweeps (emmi_point.cu).  Left out (the sweeps
+// then factor their patches each time) when they would take more than a
+// quarter of the free device memory.
+template <typename T>
+static int build_point_data(emmi_solver* s) {
+  const int l = s->lmax - 1;
+  const int nh = s->opt.isemicoarsen ? 3 : 1;
+  size_t bytes = 0;
+  for (int h = 0; h < nh; h++)
+    bytes += (size_t)s->nop * point_coef_elems(s->hier[h][l].n) * sizeof(T) +
+             (size_t)s->ngroups * point_factor_elems(s->hier[h][l].n) * sizeof(C_t<T>);
+  if (bytes > device_avail() / 4) return EMMI_OK;
+  for (int h = 0; h < nh; h++) {
+    const int* n = s->hier[h][l].n;
+    int rc;
+    if ((rc = s->alloc(&s->pt_coef[h],
+                       (size_t)s->nop * point_coef_elems(n) * sizeof(T))) != EMMI_OK ||
+        (rc = s->alloc(&s->pt_fac[h], (size_t)s->ngroups * point_factor_elems(n) *
+                                          sizeof(C_t<T>))) != EMMI_OK)
+      return rc;
+    LevelView<T> ops = s->view<T>(h, l), groups = ops;
+    ops.nrhs = s->nop;
+    ops.op = nullptr;
+    groups.nrhs = s->ngroups;
+    groups.op = s->d_gop;
+    groups.wmu = static_cast<const T*>(s->d_gwmu);
+    launch_point_setup<T>(ops, static_cast<T*>(s->pt_coef[h]), groups,
+                          static_cast<C_t<T>*>(s->pt_fac[h]), s->st);
+    s->pt_block[h] = point_in_block(n, (int)sizeof(C_t<T>));
+  }
+  for (int h = nh; h < 3; h++) {
+    s->pt_coef[h] = s->pt_coef[0];
+    s->pt_fac[h] = s->pt_fac[0];
+    s->pt_block[h] = s->pt_block[0];
+  }
+  CK(cudaGetLastError());
+  return EMMI_OK;
+}
+
+// Stored line factors of the complex64 cycle: size the factor blocks of every
+// (hierarchy, level, direction, colour) the smoother relaxes, and factor each
+// group's lines once.  Leaves
+// fac_on false (factoring in every sweep) when they would take more than
+// half of the free device memory.
+template <typename T>
+static int build_line_factors(emmi_solver* s) {
+  const int ng = s->ngroups;
   // complex64: fp16 L (the default, line_factors = 2) unless a value leaves
   // its range, then every factor is recomputed in fp32; complex128: records
   // in FP64
@@ -590,17 +678,7 @@ static int build_line_factors(emmi_solver* s) {
       if ((rc = s->alloc(&s->scratch, s->scratch_bytes)) != EMMI_OK) return rc;
     }
     if ((rc = s->alloc((void**)&s->d_fac, bytes)) != EMMI_OK) return rc;
-    if (!s->d_grp) {
-      if ((rc = s->alloc((void**)&s->d_grp, nrhs * sizeof(int))) != EMMI_OK) return rc;
-      if ((rc = s->alloc((void**)&s->d_gop, ng * sizeof(int))) != EMMI_OK) return rc;
-      if ((rc = s->alloc((void**)&s->d_gwmu, ng * sizeof(T))) != EMMI_OK) return rc;
-      CK(cudaMemcpyAsync(s->d_grp, grp.data(), nrhs * sizeof(int), cudaMemcpyHostToDevice,
-                         s->st));
-      CK(cudaMemcpyAsync(s->d_gop, gop.data(), ng * sizeof(int), cudaMemcpyHostToDevice, s->st));
-      CK(cudaMemcpyAsync(s->d_gwmu, gw.data(), ng * sizeof(T), cudaMemcpyHostToDevice, s->st));
-    }
     CK(cudaMemsetAsync(d_ovf, 0, sizeof(int), s->st));
-    s->ngroups = ng;
     s->fac_bytes = bytes;
     // factor every block once, every group in one launch per colour
     std::vector<long> done;
@@ -799,6 +877,36 @@ static int autotune_sweeps(emmi_solver* s) {
   }
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
+  CK(cudaGetLastError());
+  return EMMI_OK;
+}
+
+// Stored FP64 coefficients of every level of the complex128 cycle: its row and
+// level residuals would spend most of their FP64 instructions on recomputing
+// them (eight divisions an edge), bit for bit the same.  240 bytes a slot and
+// operator, kept when they fit in half of the free device memory.
+static int build_coef64_levels(emmi_solver* s) {
+  size_t bytes = 0;
+  for (int h = 0; h < 3; h++)
+    for (int l = h ? 1 : 0; l < s->lmax; l++)
+      bytes += (size_t)s->nop * coef64_elems(s->hier[h][l].n) * sizeof(double);
+  if (bytes > device_avail() / 2) return EMMI_OK;
+  for (int h = 0; h < 3; h++)
+    for (int l = 0; l < s->lmax; l++) {
+      if (h && l == 0) {
+        s->coef64[h][0] = s->coef64[0][0];
+        continue;
+      }
+      const size_t b = (size_t)s->nop * coef64_elems(s->hier[h][l].n) * sizeof(double);
+      int rc;
+      if ((rc = s->alloc((void**)&s->coef64[h][l], b)) != EMMI_OK) return rc;
+      CK(cudaMemsetAsync(s->coef64[h][l], 0, b, s->st));
+      LevelView<double> V = s->view<double>(h, l);
+      V.nrhs = s->nop;
+      V.op = nullptr;
+      V.active = nullptr;
+      launch_coef64(V, s->coef64[h][l], s->st);
+    }
   CK(cudaGetLastError());
   return EMMI_OK;
 }
@@ -1220,6 +1328,10 @@ static int create_impl(emmi_solver** out, const emmi_problem* P, const emmi_opti
     for (int l = 1; l < kMaxLev; l++)
       for (int d = 0; d < 3; d++) s->shape[l][d].subst = 1;
     mark("field buffers");
+    if (s->opt.line_factors) {
+      TRY(mixed ? build_groups<float>(s) : build_groups<double>(s));
+      if (s->lmax > 1) TRY(mixed ? build_point_data<float>(s) : build_point_data<double>(s));
+    }
     if (s->opt.line_factors && !s->opt.line_sweep)
       TRY(mixed ? build_line_factors<float>(s) : build_line_factors<double>(s));
     mark("line factors");
@@ -1243,6 +1355,7 @@ static int create_impl(emmi_solver** out, const emmi_problem* P, const emmi_opti
         for (int h = 1; h < 3; h++) s->plan[h][0] = s->plan[0][0];
     }
     if (mixed) TRY(build_coef64(s));
+    else if (s->opt.line_factors) TRY(build_coef64_levels(s));
     mark("FP64 coefficients");
   }
 

@@ -104,6 +104,13 @@ struct emmi_solver {
   long fac_off[3][emmi::kMaxLev][3][4];
   int fac_tile[3][emmi::kMaxLev][3];  // lines per tile of the complex64 blocks
 
+  // node-patch sweeps of the coarsest level (per hierarchy): coefficients per
+  // operator and patch factors per group (working precision; null: factored in
+  // every sweep), and whether a block's shared memory holds the level
+  void* pt_coef[3] = {};
+  void* pt_fac[3] = {};
+  bool pt_block[3] = {};
+
   // one-launch line sweep (opt.line_sweep): multiplier format (kLHalf only
   // for MIXED with line_factors = 2) and the device flag an fp16 multiplier
   // out of range sets
@@ -116,6 +123,10 @@ struct emmi_solver {
   // stored FP64 edge coefficients of the level-0 true operators (MIXED):
   // the refinement residual reads them instead of recomputing (null: off)
   double* d_coef64 = nullptr;
+
+  // the complex128 cycle's stored coefficients per (hierarchy, level) (FP64
+  // solvers; null: off)
+  double* coef64[3][emmi::kMaxLev] = {};
 
   // FGMRES (MIXED, opt.krylov > 0): basis kv [m+1][nrhs][3S] FP64,
   // preconditioned directions kz [m][nrhs][3S] complex64, FP64 temporaries
@@ -156,6 +167,7 @@ struct emmi_solver {
 
   template <typename T> emmi::LevelView<T> view(int h, int l) const;
   template <typename T> void emit_smooth(int h, int l, int iter);
+  template <typename T> bool emit_coarsest(int h, bool zero);
   template <typename T>
   void resid(int h, int l, const emmi::LevelView<T>& V, emmi::C_t<T>* rout, double* norm2);
   template <typename T> void emit_cycle(int h, int l, int kind, int want, int& cur);
