@@ -476,9 +476,12 @@ void emmi_solver::emit_cycle(int h, int l, int kind, int want, int& cur) {
   auto can_descend = [&](int lv) {
     return lv < lmax - 1 && hier[h][lv + 1].sc[0] * hier[h][lv + 1].sc[1] * hier[h][lv + 1].sc[2] > 1;
   };
-  auto to_coarse = [&](int lv) {
+  // from_f: u of level lv is 0, so that its residual is f itself
+  auto to_coarse = [&](int lv, bool from_f = false) {
     if (cur == want) {
-      launch_restrict<T>(view<T>(h, lv), view<T>(h, lv + 1), hier[h][lv + 1].sc, st);
+      LevelView<T> V = view<T>(h, lv);
+      if (from_f) V.r = V.f;
+      launch_restrict<T>(V, view<T>(h, lv + 1), hier[h][lv + 1].sc, st);
       launch_counter++;
     }
   };
@@ -509,8 +512,9 @@ void emmi_solver::emit_cycle(int h, int l, int kind, int want, int& cur) {
         launch_counter++;
       }
     } else if (can_descend(l)) {
-      residual(l);
-      to_coarse(l);
+      // below level 0 the way down starts from the u = 0 the restriction left
+      if (l == 0) residual(l);
+      to_coarse(l, l > 0);
       emit_cycle<T>(h, l + 1, 2, want, cur);
       to_fine(l);
     }
