@@ -64,7 +64,8 @@ struct SweepShape {
 };
 int subst_variant_threads(int v);
 int subst_variant_ring(int v);
-int line_fac_launches(const int n[3], int d, int tile, int fmt, SweepShape sh);
+int line_fac_launches(const int n[3], int d, int color, int nrhs, int tile, int fmt, int imu_vol,
+                      SweepShape sh);
 void init_stored_line_kernels();
 template <typename T>
 void launch_line_sweep_fac(const LevelView<T>& L, int d, int color, const T* fac, const int* grp,
@@ -82,6 +83,11 @@ long line_l_bytes(const int n[3], int d, int color, int lf, int tsize);
 template <typename T>
 void launch_line_fused(const LevelView<T>& L, int d, int color, void* lbuf, int lf, int* ovf,
                        cudaStream_t st);
+// all four colours (reversed with rev) in one launch, for a complex64 level
+// with line_fused_block
+bool line_fused_block(const int n[3], int d);
+void launch_line_fused_block(const LevelView<float>& L, int d, bool rev, void* lbuf, int lf,
+                             int* ovf, cudaStream_t st);
 
 // complex64 residual with its halos staged by tensor copies (emmi_stencil.cu):
 // tiles of TY rows x KZ planes, plane windows in a ring of shared-memory

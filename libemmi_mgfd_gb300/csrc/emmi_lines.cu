@@ -202,13 +202,120 @@ __global__ void __launch_bounds__(256) k_line_rhs(LevelView<T> L, int pa, int pb
 // reads and writes 503 MB (u, f and sigma once) in 90 us, 5.6 TB/s; row by row
 // the same bytes took 131 us, waiting for loads.  A sweep of 25 right-hand
 // sides with it: x 7.57 -> 5.95, y 6.37 -> 5.39, z 5.90 -> 5.47 ms.
+template <int D>
+__device__ __forceinline__ void node_rows(const LevelView<float>& L, int rhs, int ta, int tb,
+                                          int s, float2 (&r)[5]) {
+  constexpr int A = (D == 0) ? 1 : 0, B = (D == 2) ? 1 : 2;
+  const int op = op_of(L, rhs);
+  const int ss[3] = {1, L.n[0] + 1, (L.n[0] + 1) * (L.n[1] + 1)};
+  const int cs[3] = {1, L.n[0], L.n[0] * L.n[1]};
+  const int sd = ss[D], sa = ss[A], sb = ss[B], cd = cs[D], ca = cs[A], cb = cs[B];
+  const int S = (int)L.S;
+  const int o = s * sd + ta * sa + tb * sb;  // the node's slot
+  const float2* u = L.u + (long)rhs * 3 * S;
+  const float2* f = L.f + (long)rhs * 3 * S;
+  const float2 *ud = u + (D * S + o), *ua = u + (A * S + o), *ub = u + (B * S + o);
+  const float2 *fd = f + (D * S + o), *fa = f + (A * S + o), *fb = f + (B * S + o);
+  const float* cells = L.cells + (long)op * 4 * L.ncell;
+  const int nc = (int)L.ncell, co = s * cd + ta * ca + tb * cb;
+  const float *gd = cells + ((long)D * nc + co), *ga = cells + ((long)A * nc + co),
+              *gb = cells + ((long)B * nc + co);
+  const Geo<float> G{L.geo + (long)op * L.gstride, L.gmax1};
+  const float wmu = L.wmu[rhs];
+  const bool node = s < L.n[D];  // the last node carries its E_D row only
+  // edges along D below (0) and above (1) the node, at the five transverse
+  // positions; transverse edges - and + of the node
+  const float2 d0 = ud[-sd], d0am = ud[-sd - sa], d0ap = ud[-sd + sa],
+               d0bm = ud[-sd - sb], d0bp = ud[-sd + sb];
+  const float2 am = ua[-sa], ap = ua[0], bm = ub[-sb], bp = ub[0];
+  const float2 am_dm = ua[-sa - sd], ap_dm = ua[-sd], bm_dm = ub[-sb - sd],
+               bp_dm = ub[-sd];
+  const float sg0 = ldro(gd - cd - ca - cb), sg1 = ldro(gd - cd - ca), sg2 = ldro(gd - cd - cb),
+              sg3 = ldro(gd - cd);
+  const float2 f0 = fd[-sd];
+  const float D0 = ldro(G.ds(D) + s - 1);
+  const float A0 = ldro(G.ds(A) + ta - 1), A1 = ldro(G.ds(A) + ta);
+  const float B0 = ldro(G.ds(B) + tb - 1), B1 = ldro(G.ds(B) + tb);
+  const float2 zero = make_float2(0.f, 0.f);
+  float2 d1 = zero, d1am = zero, d1ap = zero, d1bm = zero, d1bp = zero;
+  float2 am_dp = zero, ap_dp = zero, bm_dp = zero, bp_dp = zero;
+  float2 am_bm = zero, am_bp = zero, ap_bm = zero, ap_bp = zero;
+  float2 bm_am = zero, bm_ap = zero, bp_am = zero, bp_ap = zero;
+  float2 f1 = zero, f2 = zero, f3 = zero, f4 = zero;
+  float sa0 = 0.f, sa1 = 0.f, sb0 = 0.f, sb1 = 0.f, D1 = 1.f;
+  if (node) {
+    d1 = ud[0];
+    d1am = ud[-sa];
+    d1ap = ud[sa];
+    d1bm = ud[-sb];
+    d1bp = ud[sb];
+    am_dp = ua[-sa + sd];
+    ap_dp = ua[sd];
+    bm_dp = ub[-sb + sd];
+    bp_dp = ub[sd];
+    am_bm = ua[-sa - sb];
+    am_bp = ua[-sa + sb];
+    ap_bm = ua[-sb];
+    ap_bp = ua[sb];
+    bm_am = ub[-sb - sa];
+    bm_ap = ub[-sb + sa];
+    bp_am = ub[-sa];
+    bp_ap = ub[sa];
+    f1 = fa[-sa];
+    f2 = fa[0];
+    f3 = fb[-sb];
+    f4 = fb[0];
+    // conductivities around the four transverse edges
+    sa0 = ((ldro(ga - ca - cd - cb) + ldro(ga - ca - cd)) + ldro(ga - ca - cb)) + ldro(ga - ca);
+    sa1 = ((ldro(ga - cd - cb) + ldro(ga - cd)) + ldro(ga - cb)) + ldro(ga);
+    sb0 = ((ldro(gb - cb - cd - ca) + ldro(gb - cb - cd)) + ldro(gb - cb - ca)) + ldro(gb - cb);
+    sb1 = ((ldro(gb - cd - ca) + ldro(gb - cd)) + ldro(gb - ca)) + ldro(gb);
+    D1 = ldro(G.ds(D) + s);
+  }
+  const float rD0 = qdiv(1.f, D0), rD1 = qdiv(1.f, D1), rA0 = qdiv(1.f, A0),
+              rA1 = qdiv(1.f, A1), rB0 = qdiv(1.f, B0), rB1 = qdiv(1.f, B1);
+  const float hd = 0.5f * (D0 + D1), ha = 0.5f * (A0 + A1), hb = 0.5f * (B0 + B1);
+  const float qw = 0.25f * wmu;
+  // f - A e of an edge: acc holds the curl-curl part, sig the sum of the
+  // four conductivities around it
+  auto done = [&](float2 ff, float2 acc, float2 e, float sig) {
+    const float m = qw * sig;  // the mass term is -i m e
+    return make_float2(ff.x - acc.x - m * e.y, ff.y - acc.y + m * e.x);
+  };
+  auto pair = [&](float2 acc, float2 e, float2 ep, float2 em, float k, float rp, float rm,
+                  float h, float2 x1, float2 x0, float2 x1m, float2 x0m) {
+    const float kp = k * rp, km = k * rm;
+    acc.x += (kp * (e.x - ep.x) + km * (e.x - em.x)) + h * ((x1.x - x0.x) - (x1m.x - x0m.x));
+    acc.y += (kp * (e.y - ep.y) + km * (e.y - em.y)) + h * ((x1.y - x0.y) - (x1m.y - x0m.y));
+    return acc;
+  };
+  {
+    float2 c = pair(zero, d0, d0ap, d0am, D0 * hb, rA1, rA0, hb, ap, ap_dm, am, am_dm);
+    c = pair(c, d0, d0bp, d0bm, D0 * ha, rB1, rB0, ha, bp, bp_dm, bm, bm_dm);
+    r[0] = done(f0, c, d0, ((sg0 + sg1) + sg2) + sg3);
+  }
+  if (node) {
+    float2 c = pair(zero, am, am_dp, am_dm, A0 * hb, rD1, rD0, hb, d1, d1am, d0, d0am);
+    c = pair(c, am, am_bp, am_bm, A0 * hd, rB1, rB0, hd, bp, bp_am, bm, bm_am);
+    r[1] = done(f1, c, am, sa0);
+    c = pair(zero, ap, ap_dp, ap_dm, A1 * hb, rD1, rD0, hb, d1ap, d1, d0ap, d0);
+    c = pair(c, ap, ap_bp, ap_bm, A1 * hd, rB1, rB0, hd, bp_ap, bp, bm_ap, bm);
+    r[2] = done(f2, c, ap, sa1);
+    c = pair(zero, bm, bm_dp, bm_dm, B0 * ha, rD1, rD0, ha, d1, d1bm, d0, d0bm);
+    c = pair(c, bm, bm_ap, bm_am, B0 * hd, rA1, rA0, hd, ap, ap_bm, am, am_bm);
+    r[3] = done(f3, c, bm, sb0);
+    c = pair(zero, bp, bp_dp, bp_dm, B1 * ha, rD1, rD0, ha, d1bp, d1, d0bp, d0);
+    c = pair(c, bp, bp_ap, bp_am, B1 * hd, rA1, rA0, hd, ap_bp, ap, am_bp, am);
+    r[4] = done(f4, c, bp, sb1);
+  }
+}
+
 template <int D, int NW>
 __global__ void __launch_bounds__(32 * NW, 16 / NW) k_line_rows(LevelView<float> L, int pa, int pb,
                                                        LineDiv dv, LineTile tl, int nodes,
                                                        int lines, float2* __restrict__ rb) {
   dep_wait();
   dep_next();
-  constexpr int A = (D == 0) ? 1 : 0, B = (D == 2) ? 1 : 2;
   const int rhs = blockIdx.y;
   if (L.active && !L.active[rhs]) return;
   const LineGeom g = line_geom<D>(L.n, pa, pb);
@@ -227,108 +334,7 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_line_rows(LevelView<float>
   if (live) {
     const unsigned lq = fdiv((unsigned)l, dv.la);
     const int ta = g.fa + 2 * (l - (int)lq * g.la), tb = g.fb + 2 * (int)lq;
-    const int op = op_of(L, rhs);
-    const int ss[3] = {1, L.n[0] + 1, (L.n[0] + 1) * (L.n[1] + 1)};
-    const int cs[3] = {1, L.n[0], L.n[0] * L.n[1]};
-    const int sd = ss[D], sa = ss[A], sb = ss[B], cd = cs[D], ca = cs[A], cb = cs[B];
-    const int S = (int)L.S;
-    const int o = s * sd + ta * sa + tb * sb;  // the node's slot
-    const float2* u = L.u + (long)rhs * 3 * S;
-    const float2* f = L.f + (long)rhs * 3 * S;
-    const float2 *ud = u + (D * S + o), *ua = u + (A * S + o), *ub = u + (B * S + o);
-    const float2 *fd = f + (D * S + o), *fa = f + (A * S + o), *fb = f + (B * S + o);
-    const float* cells = L.cells + (long)op * 4 * L.ncell;
-    const int nc = (int)L.ncell, co = s * cd + ta * ca + tb * cb;
-    const float *gd = cells + ((long)D * nc + co), *ga = cells + ((long)A * nc + co),
-                *gb = cells + ((long)B * nc + co);
-    const Geo<float> G{L.geo + (long)op * L.gstride, L.gmax1};
-    const float wmu = L.wmu[rhs];
-    const bool node = s < g.nd;  // the last node carries its E_D row only
-    // edges along D below (0) and above (1) the node, at the five transverse
-    // positions; transverse edges - and + of the node
-    const float2 d0 = ud[-sd], d0am = ud[-sd - sa], d0ap = ud[-sd + sa],
-                 d0bm = ud[-sd - sb], d0bp = ud[-sd + sb];
-    const float2 am = ua[-sa], ap = ua[0], bm = ub[-sb], bp = ub[0];
-    const float2 am_dm = ua[-sa - sd], ap_dm = ua[-sd], bm_dm = ub[-sb - sd],
-                 bp_dm = ub[-sd];
-    const float sg0 = ldro(gd - cd - ca - cb), sg1 = ldro(gd - cd - ca), sg2 = ldro(gd - cd - cb),
-                sg3 = ldro(gd - cd);
-    const float2 f0 = fd[-sd];
-    const float D0 = ldro(G.ds(D) + s - 1);
-    const float A0 = ldro(G.ds(A) + ta - 1), A1 = ldro(G.ds(A) + ta);
-    const float B0 = ldro(G.ds(B) + tb - 1), B1 = ldro(G.ds(B) + tb);
-    const float2 zero = make_float2(0.f, 0.f);
-    float2 d1 = zero, d1am = zero, d1ap = zero, d1bm = zero, d1bp = zero;
-    float2 am_dp = zero, ap_dp = zero, bm_dp = zero, bp_dp = zero;
-    float2 am_bm = zero, am_bp = zero, ap_bm = zero, ap_bp = zero;
-    float2 bm_am = zero, bm_ap = zero, bp_am = zero, bp_ap = zero;
-    float2 f1 = zero, f2 = zero, f3 = zero, f4 = zero;
-    float sa0 = 0.f, sa1 = 0.f, sb0 = 0.f, sb1 = 0.f, D1 = 1.f;
-    if (node) {
-      d1 = ud[0];
-      d1am = ud[-sa];
-      d1ap = ud[sa];
-      d1bm = ud[-sb];
-      d1bp = ud[sb];
-      am_dp = ua[-sa + sd];
-      ap_dp = ua[sd];
-      bm_dp = ub[-sb + sd];
-      bp_dp = ub[sd];
-      am_bm = ua[-sa - sb];
-      am_bp = ua[-sa + sb];
-      ap_bm = ua[-sb];
-      ap_bp = ua[sb];
-      bm_am = ub[-sb - sa];
-      bm_ap = ub[-sb + sa];
-      bp_am = ub[-sa];
-      bp_ap = ub[sa];
-      f1 = fa[-sa];
-      f2 = fa[0];
-      f3 = fb[-sb];
-      f4 = fb[0];
-      // conductivities around the four transverse edges
-      sa0 = ((ldro(ga - ca - cd - cb) + ldro(ga - ca - cd)) + ldro(ga - ca - cb)) + ldro(ga - ca);
-      sa1 = ((ldro(ga - cd - cb) + ldro(ga - cd)) + ldro(ga - cb)) + ldro(ga);
-      sb0 = ((ldro(gb - cb - cd - ca) + ldro(gb - cb - cd)) + ldro(gb - cb - ca)) + ldro(gb - cb);
-      sb1 = ((ldro(gb - cd - ca) + ldro(gb - cd)) + ldro(gb - ca)) + ldro(gb);
-      D1 = ldro(G.ds(D) + s);
-    }
-    const float rD0 = qdiv(1.f, D0), rD1 = qdiv(1.f, D1), rA0 = qdiv(1.f, A0),
-                rA1 = qdiv(1.f, A1), rB0 = qdiv(1.f, B0), rB1 = qdiv(1.f, B1);
-    const float hd = 0.5f * (D0 + D1), ha = 0.5f * (A0 + A1), hb = 0.5f * (B0 + B1);
-    const float qw = 0.25f * wmu;
-    // f - A e of an edge: acc holds the curl-curl part, sig the sum of the
-    // four conductivities around it
-    auto done = [&](float2 ff, float2 acc, float2 e, float sig) {
-      const float m = qw * sig;  // the mass term is -i m e
-      return make_float2(ff.x - acc.x - m * e.y, ff.y - acc.y + m * e.x);
-    };
-    auto pair = [&](float2 acc, float2 e, float2 ep, float2 em, float k, float rp, float rm,
-                    float h, float2 x1, float2 x0, float2 x1m, float2 x0m) {
-      const float kp = k * rp, km = k * rm;
-      acc.x += (kp * (e.x - ep.x) + km * (e.x - em.x)) + h * ((x1.x - x0.x) - (x1m.x - x0m.x));
-      acc.y += (kp * (e.y - ep.y) + km * (e.y - em.y)) + h * ((x1.y - x0.y) - (x1m.y - x0m.y));
-      return acc;
-    };
-    {
-      float2 c = pair(zero, d0, d0ap, d0am, D0 * hb, rA1, rA0, hb, ap, ap_dm, am, am_dm);
-      c = pair(c, d0, d0bp, d0bm, D0 * ha, rB1, rB0, ha, bp, bp_dm, bm, bm_dm);
-      r[0] = done(f0, c, d0, ((sg0 + sg1) + sg2) + sg3);
-    }
-    if (node) {
-      float2 c = pair(zero, am, am_dp, am_dm, A0 * hb, rD1, rD0, hb, d1, d1am, d0, d0am);
-      c = pair(c, am, am_bp, am_bm, A0 * hd, rB1, rB0, hd, bp, bp_am, bm, bm_am);
-      r[1] = done(f1, c, am, sa0);
-      c = pair(zero, ap, ap_dp, ap_dm, A1 * hb, rD1, rD0, hb, d1ap, d1, d0ap, d0);
-      c = pair(c, ap, ap_bp, ap_bm, A1 * hd, rB1, rB0, hd, bp_ap, bp, bm_ap, bm);
-      r[2] = done(f2, c, ap, sa1);
-      c = pair(zero, bm, bm_dp, bm_dm, B0 * ha, rD1, rD0, ha, d1, d1bm, d0, d0bm);
-      c = pair(c, bm, bm_ap, bm_am, B0 * hd, rA1, rA0, hd, ap, ap_bm, am, am_bm);
-      r[3] = done(f3, c, bm, sb0);
-      c = pair(zero, bp, bp_dp, bp_dm, B1 * ha, rD1, rD0, ha, d1bp, d1, d0bp, d0);
-      c = pair(c, bp, bp_ap, bp_am, B1 * hd, rA1, rA0, hd, ap_bp, ap, am_bp, am);
-      r[4] = done(f4, c, bp, sb1);
-    }
+    node_rows<D>(L, rhs, ta, tb, s, r);
   }
   const int shift = tl.shift, mask = (1 << shift) - 1;
   float2* out = rb + (long)rhs * rb_elems<float>(tl, g.nl);
@@ -622,9 +628,14 @@ __device__ __forceinline__ float2 cchain(float2 a, float2 b, float2 c) {
 // residuals among them).  Loads are cooperative and of 16 bytes, 2.25 a row
 // and lane instead of 4; a ring deeper than the latency needs only saves
 // re-reads (16 groups, one block an SM: 7.2 ms).
-constexpr int kXThreads = 256;  // of a block of x lines
-template <int FMT, int TW, int NG, int D>
-__global__ void __launch_bounds__(D == 0 ? kXThreads : TW == 32 ? 128 : 32)
+//
+// ROWS (TW = 8): the block's 256 threads form the rows' residuals themselves
+// (node_rows), straight into the slots -- lines of a colour do not read each
+// other's unknowns, so a colour is one launch -- and 16 of them substitute:
+// one shot at 16^3 17.3 -> 14.7 ms, at 64^3 37.2 -> 31.4.
+constexpr int kXThreads = 256;  // of a block of x lines, or of one that forms its rows
+template <int FMT, int TW, int NG, int D, bool ROWS = false>
+__global__ void __launch_bounds__(D == 0 || ROWS ? kXThreads : TW == 32 ? 128 : 32)
     k_line_ends(const int* __restrict__ active, const int* __restrict__ grp, long nl, LineTile tl,
                 long gstride, const float* __restrict__ fac, float2* __restrict__ rb,
                 LevelView<float> L, int pa, int pb, LineDiv dv, int slots, unsigned tile_bytes) {
@@ -638,9 +649,9 @@ __global__ void __launch_bounds__(D == 0 ? kXThreads : TW == 32 ? 128 : 32)
     return;
   }
   const int tid = threadIdx.x;
-  const int lane = tid & (TW - 1), end = (tid / TW) & 1, tic = D == 0 ? 0 : tid / (2 * TW);
+  const int lane = tid & (TW - 1), end = (tid / TW) & 1, tic = D == 0 || ROWS ? 0 : tid / (2 * TW);
   const int tiles = (int)((nl + TW - 1) / TW);
-  const int tile = blockIdx.x * (D == 0 ? 1 : blockDim.x / (2 * TW)) + tic;
+  const int tile = blockIdx.x * (D == 0 || ROWS ? 1 : blockDim.x / (2 * TW)) + tic;
   if (tile >= tiles) {
     dep_wait();
     return;
@@ -657,7 +668,6 @@ __global__ void __launch_bounds__(D == 0 ? kXThreads : TW == 32 ? 128 : 32)
                             (long)tile * m * kRow * TW;
   float2* rt = rb + ((long)rhs * tiles + tile) * m * TW;  // this tile's rows by position
   const int p0 = end ? tl.mid + 6 : 0;
-  auto work = [&]() {
   auto tile_sync = [&]() {
     if constexpr (TW == 32) asm volatile("bar.sync %0, 64;\n" ::"r"(1 + tic) : "memory");
     else __syncwarp(0xffffu);
@@ -677,7 +687,7 @@ __global__ void __launch_bounds__(D == 0 ? kXThreads : TW == 32 ? 128 : 32)
   };
   auto issue = [&](int g) {
     issue_fac(g);
-    issue_rows(g);
+    if constexpr (!ROWS) issue_rows(g);
   };
   // slots of u: row t of group g at off[t] + g * step
   float2* u = nullptr;
@@ -721,16 +731,51 @@ __global__ void __launch_bounds__(D == 0 ? kXThreads : TW == 32 ? 128 : 32)
 
   // the factors of the first groups and of the middle rows, which no kernel of
   // a cycle writes, before the wait for the residuals
+  const bool worker = tid < 2 * TW || (D != 0 && !ROWS);
   const int at = end * TW + lane;
+  if (worker) {
 #pragma unroll
-  for (int p = 0; p < PD; p++)
-    if (p < G) issue_fac(p);
-  {
+    for (int p = 0; p < PD; p++)
+      if (p < G) issue_fac(p);
     const unsigned char* mf = fb + (long)tl.mid * kRow * TW;
     for (int c = at; c < 6 * kRow * TW / 16; c += 2 * TW) cp_async16(midf + 16 * c, mf + 16 * c);
   }
   dep_wait();
   dep_next();
+  if constexpr (ROWS) {
+    // y and z lines: neighbouring threads take neighbouring lines, x lines:
+    // neighbouring nodes
+    const LineGeom g = line_geom<D>(L.n, pa, pb);
+    const int li = D == 0 ? tid >> 5 : tid & 7, s0 = 1 + (D == 0 ? tid & 31 : tid >> 3);
+    const long ll = (long)tile * TW + li;
+    if (ll < nl) {
+      const unsigned lq = fdiv((unsigned)ll, dv.la);
+      const int ta = g.fa + 2 * (int)((unsigned)ll - lq * (unsigned)g.la);
+      const int tb = g.fb + 2 * (int)lq;
+      for (int s = s0; s <= g.nd; s += 32) {
+        float2 r[5];
+        node_rows<D>(L, rhs, ta, tb, s, r);
+#pragma unroll
+        for (int t = 0; t < 5; t++) {
+          const int row = 5 * (s - 1) + t;
+          if (row >= m) continue;
+          float2* q;
+          if (row < tl.mid) {
+            q = reinterpret_cast<float2*>(tsm + (size_t)(s - 1) * kSlot + kFacB) + t * TW;
+          } else if (row < tl.mid + 6) {
+            q = midr + (row - tl.mid) * TW;
+          } else {
+            const int k = m - 1 - row, j = k / 5;
+            q = reinterpret_cast<float2*>(tsm + (size_t)(slots + j) * kSlot + kFacB) +
+                (k - 5 * j) * TW;
+          }
+          q[li] = r[t];
+        }
+      }
+    }
+    __syncthreads();
+  }
+  auto work = [&]() {
   // forward; the middle rows' u (three an end) is asked for first
   float2 um[3];
   if constexpr (D >= 1) {
@@ -738,14 +783,14 @@ __global__ void __launch_bounds__(D == 0 ? kXThreads : TW == 32 ? 128 : 32)
     for (int i = 0; i < 3; i++)
       um[i] = live ? u[end ? moff[3 + i] : moff[i]] : make_float2(0.f, 0.f);
   }
-  {
+  if constexpr (!ROWS) {
     const unsigned char* mr = reinterpret_cast<const unsigned char*>(rt + (long)tl.mid * TW);
     for (int c = at; c < 3 * TW; c += 2 * TW)
       cp_async16(reinterpret_cast<unsigned char*>(midr) + 16 * c, mr + 16 * c);
   }
 #pragma unroll
   for (int p = 0; p < PD; p++) {
-    if (p < G) issue_rows(p);
+    if (!ROWS && p < G) issue_rows(p);
     cp_async_commit();
   }
   float2 w[5];
@@ -869,8 +914,7 @@ __global__ void __launch_bounds__(D == 0 ? kXThreads : TW == 32 ? 128 : 32)
     }
   }
   };
-  if (D != 0 || tid < 2 * TW) work();
-  else dep_wait();
+  if (worker) work();
   if constexpr (D == 0) {
     // u += x along the lines by the whole block, neighbouring nodes by
     // neighbouring threads (the serial part above occupies 2 TW of them)
@@ -1303,19 +1347,19 @@ struct EndsArgs {
   LineDiv dv;
 };
 
-template <int FMT, int TW, int NG, int D>
+template <int FMT, int TW, int NG, int D, bool ROWS = false>
 static void ends_launch(const EndsArgs& a, int tpc, cudaStream_t st) {
   const int G = a.tl.mid / 5, slots = NG && NG < G ? NG : G;
   const unsigned tb = ends_smem<FMT>(TW, slots);
   static std::once_flag once;
   std::call_once(once, [] {
-    cudaFuncSetAttribute(k_line_ends<FMT, TW, NG, D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(k_line_ends<FMT, TW, NG, D, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          227 << 10);
   });
   const long tiles = (a.nl + TW - 1) / TW;
-  if (D == 0) tpc = 1;
+  if (D == 0 || ROWS) tpc = 1;
   dim3 g((unsigned)((tiles + tpc - 1) / tpc), a.L->nrhs);
-  launch_dep(k_line_ends<FMT, TW, NG, D>, g, D == 0 ? kXThreads : 2 * TW * tpc, tpc * tb, st, a.L->active, a.grp, a.nl, a.tl, a.gstride, a.fac, a.rb, *a.L, a.pa, a.pb, a.dv, slots, tb);
+  launch_dep(k_line_ends<FMT, TW, NG, D, ROWS>, g, D == 0 || ROWS ? kXThreads : 2 * TW * tpc, tpc * tb, st, a.L->active, a.grp, a.nl, a.tl, a.gstride, a.fac, a.rb, *a.L, a.pa, a.pb, a.dv, slots, tb);
 }
 
 // the ring of a launch: NG of the shape, one NG for the fp32 format
@@ -1329,11 +1373,21 @@ static bool ends_resident(const int n[3], int d, int tile, int fmt, SweepShape s
   return tile < 32 || G <= (fmt == kFacF16 ? ends_ring<kFacF16>(sh) : ends_ring<kFacF32>(sh));
 }
 
+// whether a colour's blocks form their rows themselves: a block an SM holds the
+// whole colour (six RHS at 80 x 56 x 72 43.1 ms a solve; 44.6 with up to two
+// blocks an SM, 51.4 with four: 256 threads then wait for 16)
+static bool ends_rows(long nl, int nrhs, int tile, int imu_vol) {
+  return tile == 8 && imu_vol && (nl + 7) / 8 * nrhs <= kSMs;
+}
+
 template <int FMT, int D>
-static void ends_dispatch(const EndsArgs& a, SweepShape sh, cudaStream_t st) {
+static void ends_dispatch(const EndsArgs& a, SweepShape sh, bool rows, cudaStream_t st) {
   const int tw = 1 << a.tl.shift;
   if (tw == 8) {
-    if constexpr (D >= 0) ends_launch<FMT, 8, 0, D>(a, 1, st);
+    if constexpr (D >= 0) {
+      if (rows) ends_launch<FMT, 8, 0, D, true>(a, 1, st);
+      else ends_launch<FMT, 8, 0, D>(a, 1, st);
+    }
     return;
   }
   if constexpr (FMT == kFacF32) {
@@ -1381,9 +1435,10 @@ static void line_sweep_fac_d(const LevelView<T>& L, int color, const T* fac, con
   dim3 gr((unsigned)(((D == 0 ? 5 : 1) * items + rt - 1) / rt), L.nrhs);
   const LineDiv dv = line_div<D>(L.n, pa, pb);
   const LineTile tl = line_tile(L.n[D], tile);
-  bool rows = false;
+  const bool in_one = std::is_same<T, float>::value && ends_rows(nl, L.nrhs, tile, L.imu_vol);
+  bool rows = in_one;
   if constexpr (std::is_same<T, float>::value) {
-    if (L.imu_vol) {
+    if (L.imu_vol && !in_one) {
       rt == 128 ? line_rows<D, 4>(L, pa, pb, nl, dv, tl, rb, st)
                 : line_rows<D, 8>(L, pa, pb, nl, dv, tl, rb, st);
       rows = true;
@@ -1404,11 +1459,11 @@ static void line_sweep_fac_d(const LevelView<T>& L, int color, const T* fac, con
     const bool res = ends_resident(L.n, D, tile, fmt, sh);
     constexpr int DS = D == 0 ? -1 : D;  // x lines with a ring too short for them
     if (fmt == kFacF16) {
-      if (res) ends_dispatch<kFacF16, D>(a, sh, st);
-      else ends_dispatch<kFacF16, DS>(a, sh, st);
+      if (res) ends_dispatch<kFacF16, D>(a, sh, in_one, st);
+      else ends_dispatch<kFacF16, DS>(a, sh, false, st);
     } else {
-      if (res) ends_dispatch<kFacF32, D>(a, sh, st);
-      else ends_dispatch<kFacF32, DS>(a, sh, st);
+      if (res) ends_dispatch<kFacF32, D>(a, sh, in_one, st);
+      else ends_dispatch<kFacF32, DS>(a, sh, false, st);
     }
     if (D == 0 && !res) apply_rb<T, D>(L, pa, pb, dv, tl, rb, st);
   } else {
@@ -1465,7 +1520,11 @@ long line_rb_elems(const int n[3], int d, int color, int tile) {
   return tile ? (nl + tile - 1) / tile * tile * m : nl * m;
 }
 
-int line_fac_launches(const int n[3], int d, int tile, int fmt, SweepShape sh) {
+int line_fac_launches(const int n[3], int d, int color, int nrhs, int tile, int fmt, int imu_vol,
+                      SweepShape sh) {
+  const long nl = line_count(n, d, color);
+  if (nl == 0) return 0;
+  if (tile && ends_rows(nl, nrhs, tile, imu_vol)) return 1;
   return tile && (d != 0 || ends_resident(n, d, tile, fmt, sh)) ? 2 : 3;
 }
 
@@ -1821,9 +1880,12 @@ __global__ void __launch_bounds__(NT) k_line_fused(LevelView<T> L, int pa, int p
 // stored factors are (the multipliers equal theirs): a block is a warp per end
 // of 32 lines.  The mirrored end hands its Schur complement of the middle rows
 // over in shared memory and takes its side of the middle solution back.
+// A block takes ncol colours one after the other, two bits each in `order`: one
+// a launch, or all four of a level whose colours each fit one block (then
+// gridDim.x = 1).
 template <int D, int LF>
-__global__ void __launch_bounds__(64) k_line_fused_ends(LevelView<float> L, int pa, int pb,
-                                                        LineDiv dv, int G, void* __restrict__ lbuf,
+__global__ void __launch_bounds__(64) k_line_fused_ends(LevelView<float> L, unsigned order,
+                                                        int ncol, int G, void* __restrict__ lbuf,
                                                         long lstride, int* __restrict__ ovf) {
   dep_wait();
   dep_next();
@@ -1833,163 +1895,192 @@ __global__ void __launch_bounds__(64) k_line_fused_ends(LevelView<float> L, int 
   __shared__ float2 xmid[6][32];
   const int rhs = blockIdx.y;
   if (L.active && !L.active[rhs]) return;
-  const LineGeom g = line_geom<D>(L.n, pa, pb);
-  const int lane = threadIdx.x & 31;
-  const long l0 = blockIdx.x * 32L + lane;
-  const bool live = l0 < g.nl;
-  const long l = live ? l0 : g.nl - 1;
-  const unsigned lq = fdiv((unsigned)l, dv.la);
-  const int ta = g.fa + 2 * (int)((unsigned)l - lq * (unsigned)g.la), tb = g.fb + 2 * (int)lq;
-  const int n0 = L.n[0] + 1, n1 = L.n[1] + 1;
-  const long ss[3] = {1, (long)n0, (long)n0 * n1};
-  float2* __restrict__ u = L.u + (long)rhs * 3 * L.S;
-  const float2* __restrict__ f = L.f + (long)rhs * 3 * L.S;
-  float2* __restrict__ zr = L.r + (long)rhs * 3 * L.S;
-  const float* __restrict__ cells = L.cells + (long)op_of(L, rhs) * 4 * L.ncell;
-  const Geo<float> Gm{L.geo + (long)op_of(L, rhs) * L.gstride, L.gmax1};
-  const float wmu = L.wmu[rhs];
-  LS ls(static_cast<char*>(lbuf) + (long)rhs * lstride, g.m, g.nl);
-  const int nd = g.nd;
-  bool over = false;
-  // row k of group j of an end: its slot, and its row number
-  auto slot_of = [&](bool mir, int j, int k) -> long {
-    const int s = mir ? nd - 1 - j : j + 1;
-    const int t = k == 0 ? 0 : mir ? 5 - k : k;
-    switch (t) {
-      case 0: return line_slot<D, 0>(L.n, L.S, ta, tb, mir ? s + 1 : s);
-      case 1: return line_slot<D, 1>(L.n, L.S, ta, tb, s);
-      case 2: return line_slot<D, 2>(L.n, L.S, ta, tb, s);
-      case 3: return line_slot<D, 3>(L.n, L.S, ta, tb, s);
-      default: return line_slot<D, 4>(L.n, L.S, ta, tb, s);
-    }
-  };
-  auto row_of = [&](bool mir, int j, int k) { return mir ? g.m - 1 - (5 * j + k) : 5 * j + k; };
-  float2 W[21], y[6], lr[6];
+  for (int cc = 0; cc < ncol; cc++) {
+    if (cc > 0) __syncthreads();  // u of the colours before
+    const int pa = (int)(order >> (2 * cc)) & 1, pb = (int)(order >> (2 * cc + 1)) & 1;
+    const LineGeom g = line_geom<D>(L.n, pa, pb);
+    if (g.nl == 0) continue;
+    const int lane = threadIdx.x & 31;
+    const long l0 = blockIdx.x * 32L + lane;
+    const bool live = l0 < g.nl;
+    const long l = live ? l0 : g.nl - 1;
+    const unsigned lq = (unsigned)l / (unsigned)g.la;
+    const int ta = g.fa + 2 * (int)((unsigned)l - lq * (unsigned)g.la), tb = g.fb + 2 * (int)lq;
+    const int n0 = L.n[0] + 1, n1 = L.n[1] + 1;
+    const long ss[3] = {1, (long)n0, (long)n0 * n1};
+    float2* u = L.u + (long)rhs * 3 * L.S;
+    const float2* f = L.f + (long)rhs * 3 * L.S;
+    float2* zr = L.r + (long)rhs * 3 * L.S;
+    const float* __restrict__ cells = L.cells + (long)op_of(L, rhs) * 4 * L.ncell;
+    const Geo<float> Gm{L.geo + (long)op_of(L, rhs) * L.gstride, L.gmax1};
+    const float wmu = L.wmu[rhs];
+    LS ls(static_cast<char*>(lbuf) + (long)rhs * lstride, g.m, g.nl);
+    const int nd = g.nd;
+    bool over = false;
+    // row k of group j of an end: its slot, and its row number
+    auto slot_of = [&](bool mir, int j, int k) -> long {
+      const int s = mir ? nd - 1 - j : j + 1;
+      const int t = k == 0 ? 0 : mir ? 5 - k : k;
+      switch (t) {
+        case 0: return line_slot<D, 0>(L.n, L.S, ta, tb, mir ? s + 1 : s);
+        case 1: return line_slot<D, 1>(L.n, L.S, ta, tb, s);
+        case 2: return line_slot<D, 2>(L.n, L.S, ta, tb, s);
+        case 3: return line_slot<D, 3>(L.n, L.S, ta, tb, s);
+        default: return line_slot<D, 4>(L.n, L.S, ta, tb, s);
+      }
+    };
+    auto row_of = [&](bool mir, int j, int k) { return mir ? g.m - 1 - (5 * j + k) : 5 * j + k; };
+    float2 W[21], y[6], lr[6];
 #pragma unroll
-  for (int i = 0; i < 21; i++) W[i] = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int i = 0; i < 5; i++) {
-    W[WI(i, i)] = make_float2(1.f, 0.f);  // dummy leading rows
-    y[i] = make_float2(0.f, 0.f);
-  }
-  auto forward = [&](auto mir) {
-    constexpr bool MIR = decltype(mir)::value;
-    eliminate_end<MIR>(
-        G, nd, W, y[5],
-        [&](auto tt, int s, int k, float2 (&w)[6], float2& r) {
-          constexpr int TT = decltype(tt)::value;
-          constexpr int C = (TT == 0) ? D : (TT <= 2 ? A : B);
-          fused_row<float, D, TT, C, MIR>(L, u, f, cells, Gm, wmu, ta, tb, s, 5 * (s - 1) + TT, ss,
-                                          w, r);
-        },
-        [&](int j, int k) {
-          const float2 z = fused_eliminate<float>(W, y, lr, ls);
-          if (j >= 0 && live) {
-            zr[slot_of(MIR, j, k)] = z;
-            over |= ls.put((long)row_of(MIR, j, k) * g.nl + l, lr);
-          }
-        });
-  };
-  const bool bottom = threadIdx.x >= 32;
-  if (bottom) {
-    forward(std::true_type());
-#pragma unroll
-    for (int i = 0; i < 15; i++) ex[i][lane] = W[i];
-#pragma unroll
-    for (int i = 0; i < 5; i++) ex[15 + i][lane] = y[i];
-  } else {
-    forward(std::false_type());
-  }
-  __syncthreads();
-  if (!bottom) {
-    float2 wr[6], r5;
-    fused_row<float, D, 0, D>(L, u, f, cells, Gm, wmu, ta, tb, G + 2, 5 * (G + 1), ss, wr, r5);
-#pragma unroll
-    for (int i = 0; i < 6; i++) W[WI(5, i)] = wr[i];
-    y[5] = r5;
+    for (int i = 0; i < 21; i++) W[i] = make_float2(0.f, 0.f);
 #pragma unroll
     for (int i = 0; i < 5; i++) {
-      y[5 - i] = cadd<float>(y[5 - i], ex[15 + i][lane]);
-#pragma unroll
-      for (int j = 0; j <= i; j++)
-        W[WI(5 - j, 5 - i)] = cadd<float>(W[WI(5 - j, 5 - i)], ex[WI(i, j)][lane]);
+      W[WI(i, i)] = make_float2(1.f, 0.f);  // dummy leading rows
+      y[i] = make_float2(0.f, 0.f);
     }
-    float2 ml[6][5], xm[6];
+    auto forward = [&](auto mir) {
+      constexpr bool MIR = decltype(mir)::value;
+      eliminate_end<MIR>(
+          G, nd, W, y[5],
+          [&](auto tt, int s, int k, float2 (&w)[6], float2& r) {
+            constexpr int TT = decltype(tt)::value;
+            constexpr int C = (TT == 0) ? D : (TT <= 2 ? A : B);
+            fused_row<float, D, TT, C, MIR>(L, u, f, cells, Gm, wmu, ta, tb, s, 5 * (s - 1) + TT, ss,
+                                            w, r);
+          },
+          [&](int j, int k) {
+            const float2 z = fused_eliminate<float>(W, y, lr, ls);
+            if (j >= 0 && live) {
+              zr[slot_of(MIR, j, k)] = z;
+              over |= ls.put((long)row_of(MIR, j, k) * g.nl + l, lr);
+            }
+          });
+    };
+    const bool bottom = threadIdx.x >= 32;
+    if (bottom) {
+      forward(std::true_type());
 #pragma unroll
-    for (int p = 0; p < 6; p++) {
-      xm[p] = fused_eliminate<float>(W, y, lr, ls);
-      over |= ls.bad(lr);
+      for (int i = 0; i < 15; i++) ex[i][lane] = W[i];
 #pragma unroll
-      for (int i = 0; i < 5; i++) ml[p][i] = lr[i + 1];
-#pragma unroll
-      for (int i = 0; i < 5; i++) W[WI(5, i)] = make_float2(0.f, 0.f);
-      W[WI(5, 5)] = make_float2(1.f, 0.f);
-      y[5] = make_float2(0.f, 0.f);
+      for (int i = 0; i < 5; i++) ex[15 + i][lane] = y[i];
+    } else {
+      forward(std::false_type());
     }
+    __syncthreads();
+    if (!bottom) {
+      float2 wr[6], r5;
+      fused_row<float, D, 0, D>(L, u, f, cells, Gm, wmu, ta, tb, G + 2, 5 * (G + 1), ss, wr, r5);
 #pragma unroll
-    for (int p = 5; p >= 0; p--) {
+      for (int i = 0; i < 6; i++) W[WI(5, i)] = wr[i];
+      y[5] = r5;
 #pragma unroll
-      for (int i = 5; i >= 1; i--)
-        if (p + i < 6) xm[p] = cfms<float>(xm[p], ml[p][i - 1], xm[p + i]);
-      xmid[p][lane] = xm[p];
-    }
-    if (live) {
+      for (int i = 0; i < 5; i++) {
+        y[5 - i] = cadd<float>(y[5 - i], ex[15 + i][lane]);
+#pragma unroll
+        for (int j = 0; j <= i; j++)
+          W[WI(5 - j, 5 - i)] = cadd<float>(W[WI(5 - j, 5 - i)], ex[WI(i, j)][lane]);
+      }
+      float2 ml[6][5], xm[6];
 #pragma unroll
       for (int p = 0; p < 6; p++) {
-        const long sl = p < 5 ? slot_of(false, G, p) : line_slot<D, 0>(L.n, L.S, ta, tb, G + 2);
-        u[sl] = cadd<float>(u[sl], xm[p]);
+        xm[p] = fused_eliminate<float>(W, y, lr, ls);
+        over |= ls.bad(lr);
+#pragma unroll
+        for (int i = 0; i < 5; i++) ml[p][i] = lr[i + 1];
+#pragma unroll
+        for (int i = 0; i < 5; i++) W[WI(5, i)] = make_float2(0.f, 0.f);
+        W[WI(5, 5)] = make_float2(1.f, 0.f);
+        y[5] = make_float2(0.f, 0.f);
+      }
+#pragma unroll
+      for (int p = 5; p >= 0; p--) {
+#pragma unroll
+        for (int i = 5; i >= 1; i--)
+          if (p + i < 6) xm[p] = cfms<float>(xm[p], ml[p][i - 1], xm[p + i]);
+        xmid[p][lane] = xm[p];
+      }
+      if (live) {
+#pragma unroll
+        for (int p = 0; p < 6; p++) {
+          const long sl = p < 5 ? slot_of(false, G, p) : line_slot<D, 0>(L.n, L.S, ta, tb, G + 2);
+          u[sl] = cadd<float>(u[sl], xm[p]);
+        }
+      }
+    }
+    __syncthreads();
+    if (over && live && ovf) atomicOr(ovf, 1);
+    float2 xw[5];
+#pragma unroll
+    for (int i = 0; i < 5; i++) xw[i] = xmid[bottom ? 5 - i : i][lane];
+    // backward a node at a time: its rows' multipliers, z and u are loaded
+    // together before the five substitution steps
+    for (int j = live ? G - 1 : -1; j >= 0; j--) {
+      float2 bl[5][5], bz[5], bu[5];
+      long bs[5];
+#pragma unroll
+      for (int k = 4; k >= 0; k--) {
+        bs[k] = slot_of(bottom, j, k);
+        ls.get((long)row_of(bottom, j, k) * g.nl + l, bl[k]);
+        bz[k] = zr[bs[k]];
+        bu[k] = u[bs[k]];
+      }
+#pragma unroll
+      for (int k = 4; k >= 0; k--) {
+        float2 x = bz[k];
+#pragma unroll
+        for (int i = 4; i >= 0; i--) x = cfms<float>(x, bl[k][i], xw[i]);
+#pragma unroll
+        for (int i = 4; i > 0; i--) xw[i] = xw[i - 1];
+        xw[0] = x;
+        u[bs[k]] = cadd<float>(bu[k], x);
       }
     }
   }
-  __syncthreads();
-  if (over && live && ovf) atomicOr(ovf, 1);
-  float2 xw[5];
-#pragma unroll
-  for (int i = 0; i < 5; i++) xw[i] = xmid[bottom ? 5 - i : i][lane];
-  if (!live) return;
-  // backward a node at a time: its rows' multipliers, z and u are loaded
-  // together before the five substitution steps
-  for (int j = G - 1; j >= 0; j--) {
-    float2 bl[5][5], bz[5], bu[5];
-    long bs[5];
-#pragma unroll
-    for (int k = 4; k >= 0; k--) {
-      bs[k] = slot_of(bottom, j, k);
-      ls.get((long)row_of(bottom, j, k) * g.nl + l, bl[k]);
-      bz[k] = zr[bs[k]];
-      bu[k] = u[bs[k]];
-    }
-#pragma unroll
-    for (int k = 4; k >= 0; k--) {
-      float2 x = bz[k];
-#pragma unroll
-      for (int i = 4; i >= 0; i--) x = cfms<float>(x, bl[k][i], xw[i]);
-#pragma unroll
-      for (int i = 4; i > 0; i--) xw[i] = xw[i - 1];
-      xw[0] = x;
-      u[bs[k]] = cadd<float>(bu[k], x);
-    }
+}
+
+// a level whose colours of lines along d each fit one block of the one-launch
+// sweep takes all four in one launch
+bool line_fused_block(const int n[3], int d) { return line_count(n, d, 3) <= 32; }
+
+// complex64: ncol colours of `order` (k_line_fused_ends)
+template <int D>
+static void line_fused_ends(const LevelView<float>& L, unsigned order, int ncol, void* lbuf, int lf,
+                            int* ovf, cudaStream_t st) {
+  long nl = 0, lstride = 0;
+  for (int c = 0; c < ncol; c++) {
+    const int col = (int)(order >> (2 * c)) & 3;
+    nl = std::max(nl, line_count(L.n, D, col));
+    lstride = std::max(lstride, line_l_bytes(L.n, D, col, lf, 4));
   }
+  if (nl == 0) return;
+  const dim3 g((unsigned)((nl + 31) / 32), L.nrhs);
+  const int G = (L.n[D] - 2) / 2;
+  if (lf == kLHalf)
+    launch_dep(k_line_fused_ends<D, kLHalf>, g, 64, 0, st, L, order, ncol, G, lbuf, lstride, ovf);
+  else
+    launch_dep(k_line_fused_ends<D, kLExact>, g, 64, 0, st, L, order, ncol, G, lbuf, lstride, ovf);
+}
+
+void launch_line_fused_block(const LevelView<float>& L, int d, bool rev, void* lbuf, int lf,
+                             int* ovf, cudaStream_t st) {
+  const unsigned order = rev ? 0x1b : 0xe4;  // 3 2 1 0 or 0 1 2 3
+  if (d == 0) line_fused_ends<0>(L, order, 4, lbuf, lf, ovf, st);
+  else if (d == 1) line_fused_ends<1>(L, order, 4, lbuf, lf, ovf, st);
+  else line_fused_ends<2>(L, order, 4, lbuf, lf, ovf, st);
 }
 
 template <typename T, int D>
 static void line_fused_d(const LevelView<T>& L, int color, void* lbuf, int lf, int* ovf,
                          cudaStream_t st) {
-  const int pa = color & 1, pb = (color >> 1) & 1;
-  const long nl = line_count(L.n, D, color);
-  if (nl == 0) return;
-  const long lstride = line_l_bytes(L.n, D, color, lf, (int)sizeof(T));
-  const LineDiv dv = line_div<D>(L.n, pa, pb);
   if constexpr (std::is_same<T, float>::value) {
-    dim3 g((unsigned)((nl + 31) / 32), L.nrhs);
-    const int G = (L.n[D] - 2) / 2;
-    if (lf == kLHalf)
-      launch_dep(k_line_fused_ends<D, kLHalf>, g, 64, 0, st, L, pa, pb, dv, G, lbuf, lstride, ovf);
-    else
-      launch_dep(k_line_fused_ends<D, kLExact>, g, 64, 0, st, L, pa, pb, dv, G, lbuf, lstride, ovf);
+    line_fused_ends<D>(L, (unsigned)color, 1, lbuf, lf, ovf, st);
   } else {
-    dim3 g((unsigned)((nl + kSolveThreads - 1) / kSolveThreads), L.nrhs);
-    launch_dep(k_line_fused<T, D, kLExact, kSolveThreads>, g, kSolveThreads, 0, st, L, pa, pb, dv, lbuf, lstride, ovf);
+    const int pa = color & 1, pb = (color >> 1) & 1;
+    const long nl = line_count(L.n, D, color);
+    if (nl == 0) return;
+    const dim3 g((unsigned)((nl + kSolveThreads - 1) / kSolveThreads), L.nrhs);
+    launch_dep(k_line_fused<T, D, kLExact, kSolveThreads>, g, kSolveThreads, 0, st, L, pa, pb,
+               line_div<D>(L.n, pa, pb), lbuf, line_l_bytes(L.n, D, color, lf, 8), ovf);
   }
 }
 

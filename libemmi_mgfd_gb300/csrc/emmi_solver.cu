@@ -372,11 +372,11 @@ static void line_colour(emmi_solver* s, int h, int l, int d, int col, const Leve
 
 // kernel launches of one colour of line relaxation along d on level l of
 // hierarchy h (what line_colour emits per RHS chunk)
-static int line_launches(const emmi_solver* s, int h, int l, int d) {
+static int line_launches(const emmi_solver* s, int h, int l, int d, int col, int nr) {
   if (s->opt.line_sweep || l >= s->opt.fused_level) return 1;  // k_line_fused
   if (s->fac_on && s->fac_off[l == 0 ? 0 : h][l][d][0] >= 0)
-    return line_fac_launches(s->hier[h][l].n, d, s->fac_tile[l == 0 ? 0 : h][l][d], s->fac_fmt,
-                             s->shape[l][d]);
+    return line_fac_launches(s->hier[h][l].n, d, col, nr, s->fac_tile[l == 0 ? 0 : h][l][d],
+                             s->fac_fmt, s->imu_vol ? 1 : 0, s->shape[l][d]);
   return 3;
 }
 
@@ -389,6 +389,14 @@ void emmi_solver::emit_smooth(int h, int l, int iter) {
   if (opt.isemicoarsen && l < lmax - 1) {
     for (int d = 0; d < 3; d++) {
       if (hier[h][l + 1].sc[d] != 2) continue;
+      if constexpr (std::is_same<T, float>::value) {
+        if ((opt.line_sweep || l >= opt.fused_level) && chunk >= nrhs &&
+            line_fused_block(hier[h][l].n, d)) {
+          launch_line_fused_block(V, d, rev, scratch, lfmt, d_lovf, st);
+          launch_counter++;
+          continue;
+        }
+      }
       for (int cc = 0; cc < 4; cc++) {
         const int col = rev ? 3 - cc : cc;
         for (int r0 = 0; r0 < nrhs; r0 += chunk) {
@@ -402,7 +410,7 @@ void emmi_solver::emit_smooth(int h, int l, int iter) {
           W.active += r0;
           W.op += r0;
           line_colour<T>(this, h, l, d, col, W, r0);
-          launch_counter += line_launches(this, h, l, d);
+          launch_counter += line_launches(this, h, l, d, col, nr);
         }
       }
     }
@@ -1807,7 +1815,12 @@ int emmi_solver_time_smoother(emmi_solver* s, int dir, int reps, double* ms, int
   cudaEventElapsedTime(&t, s->ev0, s->ev1);
   const double c = mixed ? 8.0 : 16.0;
   if (ms) *ms = t / reps;
-  if (launches) *launches = 4 * line_launches(s, h, 0, dir) * ((s->nrhs + s->chunk - 1) / s->chunk);
+  if (launches) {
+    *launches = 0;
+    for (int c = 0; c < 4; c++)
+      for (int r0 = 0; r0 < s->nrhs; r0 += s->chunk)
+        *launches += line_launches(s, h, 0, dir, c, std::min(s->chunk, s->nrhs - r0));
+  }
   if (bytes) *bytes = (double)s->hier[0][0].S * (9 * c + 12) * s->nrhs;
   return EMMI_OK;
 }
