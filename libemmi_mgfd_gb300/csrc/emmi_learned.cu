@@ -44,9 +44,12 @@ namespace emmi {
 
 namespace {
 
+constexpr int kSMs = 152;
 constexpr int kCh = 8;
 constexpr int kTaps = 27;
-constexpr int kTcInstr = 15;  // tcgen05.mma per output tile
+constexpr int kTcPairs = 5;   // tap pairs of a plane = tcgen05.mma of one window
+constexpr int kTcN = 48;      // columns of a window's MMA: 3 output planes x 16
+constexpr int kWtLayer = kTcPairs * 2 * kTcN;  // 16-byte rows of a layer's B operands
 constexpr int kWLayer = kTaps * kCh * kCh;  // [tap][cin][cout]
 
 // tap t = (dk+1)*9 + (dj+1)*3 + (di+1)
@@ -77,29 +80,28 @@ __device__ __forceinline__ bool unknown_any(int c, const int n[3], int i, int j,
 }
 
 // ---------------------------------------------------------------- weights
-// B operands of the tensor-core convolution, one 16 x 16 bf16 matrix per
-// instruction (N = 16 output columns, 8 of them zero; K = 16 = two taps x 8
-// input channels), K-major without swizzle: the 8 x 8 core matrix (n-group
-// ng, k-group kc) at byte 256 kc + 128 ng, row n % 8 at 16 bytes, element
-// k % 8 at 2 bytes.  Instruction q covers plane dk = q / 5 - 1 and the tap
-// pair 2 (q % 5), 2 (q % 5) + 1 of that plane's 9 taps (raster (dj, di));
-// the fifth pair holds the ninth tap alone (its second half zero).
+// B operands of the tensor-core convolution, one 48 x 16 bf16 matrix per tap
+// pair (K = 16 = two taps x 8 input channels; N = 48 = the three output planes
+// a window contributes to x 16 columns, 8 of them zero), K-major without
+// swizzle: the 8 x 8 core matrix (n-group ng, k-group kc) at byte
+// 768 kc + 128 ng, row n % 8 at 16 bytes, element k % 8 at 2 bytes.  Matrix pi
+// covers the tap pair 2 pi, 2 pi + 1 of a plane's 9 taps (raster (dj, di); the
+// fifth pair holds the ninth tap alone, its second half zero); columns 16 o ..
+// 16 o + 7 are the output plane p - 1 + o of window p, its tap plane dk = 1 - o.
 __global__ void k_ls_pack(const float* __restrict__ W, uint4* __restrict__ Wt) {
-  const int id = blockIdx.x * blockDim.x + threadIdx.x;  // [layer][q][kc][ng][n8]
-  if (id >= 2 * kTcInstr * 32) return;
-  const int n8 = id & 7, ng = (id >> 3) & 1, kc = (id >> 4) & 1, q = (id >> 5) % kTcInstr,
-            layer = id / (32 * kTcInstr);
-  const int dk = q / 5 - 1, pi = q % 5;
+  const int id = blockIdx.x * blockDim.x + threadIdx.x;  // [layer][pi][kc][ng][n8]
+  if (id >= 2 * kWtLayer) return;
+  const int n8 = id & 7, ng = (id >> 3) % 6, kc = (id / kTcN) & 1,
+            pi = (id / (2 * kTcN)) % kTcPairs, layer = id / kWtLayer;
   const int r = 2 * pi + kc;  // tap of this k-group within the plane's raster
-  const int n = 8 * ng + n8;
   const float* w = W + layer * kWLayer;
   uint32_t v[4];
   for (int e = 0; e < 4; e++) {
     float lo = 0.f, hi = 0.f;
-    if (n < kCh && r < 9) {
-      const int t = (dk + 1) * 9 + r;
-      lo = w[(t * kCh + 2 * e) * kCh + n];
-      hi = w[(t * kCh + 2 * e + 1) * kCh + n];
+    if (ng % 2 == 0 && r < 9) {
+      const int t = (2 - ng / 2) * 9 + r;  // dk + 1 = 2 - o
+      lo = w[(t * kCh + 2 * e) * kCh + n8];
+      hi = w[(t * kCh + 2 * e + 1) * kCh + n8];
     }
     v[e] = pack_bf16x2(lo, hi);
   }
@@ -109,46 +111,78 @@ __global__ void k_ls_pack(const float* __restrict__ W, uint4* __restrict__ Wt) {
 // ---------------------------------------------------------------- input
 // X[b][s][8] bf16 = D^-1 r on unknown edges, 0 elsewhere.  r is read from
 // rin ([b][3][S] complex64) when given, else formed as f - A u on L.
-__global__ void __launch_bounds__(256) k_ls_input(LevelView<float> L, const float2* __restrict__ rin,
+// The roundings of a row are written out: z is rounded to bf16, and a last bit
+// that differed between the kernel's forms would show there.  Instructions
+// bound it (some 700 a slot, 75 % of the issue slots; 8 RHS at 96^3 182 -> 178
+// us with W known).  Several right-hand sides a thread to share coefficients,
+// or an interior slot's rows to share loads, cost more in occupancy (64 to 126
+// registers for 32) than they save: 196 to 283 us.
+template <int C, int W, bool RIN>
+__device__ __forceinline__ uint32_t ls_edge(const LevelView<float>& L, const float2* rin, int b,
+                                            const int P[3], long s) {
+  if (!unknown_edge<C>(L.n, P[0], P[1], P[2])) return 0u;
+  const int op = op_of(L, b);
+  const float* cells = L.cells + (long)op * 4 * L.ncell;
+  const Geo<float> G{L.geo + (long)op * L.gstride, L.gmax1};
+  EdgeCoef<float> e;
+  edge_coef<float, C, W>(L.n, P, cells + (long)C * L.ncell, cells + 3 * L.ncell, G, L.wmu[b], e);
+  const int s3[3] = {1, L.n[0] + 1, (L.n[0] + 1) * (L.n[1] + 1)};
+  const int si = (int)s, Si = (int)L.S;
+  const long o = (long)b * 3 * L.S;
+  float2 r = make_float2(0.f, 0.f);
+  if (RIN) {
+    r = rin[o + C * Si + si];
+  } else {
+    const float2* u = L.u + o;
+    if (L.f) r = L.f[o + C * Si + si];
+    const float2 uc = u[C * Si + si];
+    float ar = fmaf(e.dre, uc.x, -(e.dim * uc.y)), ai = fmaf(e.dre, uc.y, e.dim * uc.x);
+#pragma unroll
+    for (int k = 0; k < 12; k++) {
+      const float2 v = u[si + nbr_delta32<C>(k, s3, Si)];
+      ar = fmaf(e.c[k], v.x, ar);
+      ai = fmaf(e.c[k], v.y, ai);
+    }
+    r = make_float2(r.x - ar, r.y - ai);
+  }
+  // z = r / d = r conj(d) / |d|^2
+  const float inv = 1.f / fmaf(e.dre, e.dre, e.dim * e.dim);
+  return pack_bf16x2(fmaf(r.y, e.dim, r.x * e.dre) * inv, fmaf(r.y, e.dre, -(r.x * e.dim)) * inv);
+}
+
+// W: edge_coef's cell weights
+template <int W, bool RIN>
+__global__ void __launch_bounds__(256) k_ls_input(LevelView<float> L,
+                                                  const float2* __restrict__ rin,
                                                   uint32_t* __restrict__ X) {
   const int b = blockIdx.y;
   if (L.active && !L.active[b]) return;
   const long s = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (s >= L.S) return;
-  const int n0 = L.n[0] + 1, n1 = L.n[1] + 1;
   int P[3];
   slot_nodes(s, L, P);
-  const long ss[3] = {1, (long)n0, (long)n0 * n1};
-  const float2* u = L.u + (long)b * 3 * L.S;
-  const float2* f = L.f ? L.f + (long)b * 3 * L.S : nullptr;
-  const float* cells = L.cells + (long)op_of(L, b) * 4 * L.ncell;
-  const Geo<float> G{L.geo + (long)op_of(L, b) * L.gstride, L.gmax1};
-  const float wmu = L.wmu[b];
-  uint32_t out[4] = {0u, 0u, 0u, 0u};
-  auto one = [&](auto cc) {
-    constexpr int C = decltype(cc)::value;
-    if (!unknown_edge<C>(L.n, P[0], P[1], P[2])) return;
-    EdgeCoef<float> e;
-    float2 r;
-    if (rin) {
-      edge_coef<float, C>(L.n, P, cells + (long)C * L.ncell, cells + 3 * L.ncell, G, wmu, e,
-                          L.imu_vol);
-      r = rin[((long)b * 3 + C) * L.S + s];
-    } else {
-      const float2 au = apply_row<float, C>(L, u, cells, G, wmu, P, s, ss, e);
-      const float2 fv = f ? f[(long)C * L.S + s] : make_float2(0.f, 0.f);
-      r = make_float2(fv.x - au.x, fv.y - au.y);
-    }
-    // z = r / d = r conj(d) / |d|^2
-    const float inv = 1.f / (e.dre * e.dre + e.dim * e.dim);
-    const float zr = (r.x * e.dre + r.y * e.dim) * inv;
-    const float zi = (r.y * e.dre - r.x * e.dim) * inv;
-    out[C] = pack_bf16x2(zr, zi);
-  };
-  one(std::integral_constant<int, 0>());
-  one(std::integral_constant<int, 1>());
-  one(std::integral_constant<int, 2>());
-  reinterpret_cast<uint4*>(X)[(long)b * L.S + s] = make_uint4(out[0], out[1], out[2], out[3]);
+  uint4 z;
+  z.x = ls_edge<0, W, RIN>(L, rin, b, P, s);
+  z.y = ls_edge<1, W, RIN>(L, rin, b, P, s);
+  z.z = ls_edge<2, W, RIN>(L, rin, b, P, s);
+  z.w = 0u;
+  reinterpret_cast<uint4*>(X)[(long)b * L.S + s] = z;
+}
+
+template <int W>
+void launch_ls_input_w(const LevelView<float>& L, const float2* rin, uint32_t* X, cudaStream_t st) {
+  const dim3 g((unsigned)((L.S + 255) / 256), L.nrhs);
+  if (rin)
+    k_ls_input<W, true><<<g, 256, 0, st>>>(L, rin, X);
+  else
+    k_ls_input<W, false><<<g, 256, 0, st>>>(L, nullptr, X);
+}
+
+void launch_ls_input(const LevelView<float>& L, const float2* rin, uint32_t* X, cudaStream_t st) {
+  if (L.imu_vol)
+    launch_ls_input_w<1>(L, rin, X, st);
+  else
+    launch_ls_input_w<0>(L, rin, X, st);
 }
 
 // ---------------------------------------------------------------- conv
@@ -162,9 +196,6 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes)
                : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ uint32_t mbar_test(uint32_t bar, uint32_t parity) {
   uint32_t ok;
@@ -206,14 +237,16 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
   return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
          ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
-// instruction descriptor: D f32, A and B bf16, both K-major, N = 16, M = 128
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((16u >> 3) << 17) |
-                            ((128u >> 4) << 24);
-__device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t acc) {
+// instruction descriptor: D f32, A and B bf16, both K-major, M = 128, N columns
+constexpr uint32_t idesc(uint32_t N) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((128u >> 4) << 24);
+}
+// D += A B
+__device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t n) {
   asm volatile(
       "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
-      "l"(a), "l"(b), "r"(kIdesc), "r"(acc)
+      "l"(a), "l"(b), "r"(idesc(n)), "r"(1u)
       : "memory");
 }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
@@ -234,22 +267,39 @@ __device__ __forceinline__ void tc_load8(uint32_t taddr, float (&v)[8]) {
   for (int i = 0; i < 8; i++) v[i] = __uint_as_float(r[i]);
 }
 
+__device__ __forceinline__ void tc_zero32(uint32_t taddr) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,"
+      "%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};\n" ::"r"(taddr),
+      "r"(0u)
+      : "memory");
+}
+
 // One 3x3x3 convolution, 8 -> 8 channels, bf16 slots [b][S] (16 bytes per
 // slot) with kTcGuard(X, Y) zero slots before the first and after the last
 // right-hand side.  A CTA owns one column of 128 consecutive in-plane slots
-// (p = i + X j) and walks the planes k of one chunk; the tile of plane k is
-// D[m][n] = sum_taps X[s_m + off(tap)] W_tap, 15 tcgen05.mma (M = 128 slots,
-// N = 16, K = 16) into one of two tensor-memory accumulators.  One thread of
-// the producer warp issues the copies and the MMAs; 4 epilogue warps (one
-// TMEM lane per thread) read the accumulators back and store; the two sides
-// meet only at mbarriers (window landed, accumulator ready, accumulator read
-// back), so the MMAs of the next planes run while an epilogue stores.  Each
-// plane's window (slots p0 - X - 1 ... p0 + 127 + X + 2 of that plane,
-// contiguous) comes in by one bulk copy, kTcAhead planes ahead, into a ring
-// of kTcRing windows; the window serves as the A operand of the plane's
-// three dk roles directly: tap (di, dj) is the 128-row matrix starting
-// X + 1 + X dj + di slots in (rows 16 bytes apart, 8 channels each = one
-// core-matrix row).
+// (p = i + X j) and one chunk of up to kTcPlanes planes k, each with 16
+// tensor-memory columns of its own for the chunk's length.  Each plane's
+// window (slots p0 - X - 1 ... p0 + 127 + X + 2 of that plane, contiguous)
+// comes in by one bulk copy, kTcAhead planes ahead, into a ring of kTcRing
+// windows, and is the A operand directly: tap (di, dj) is the 128-row matrix
+// starting X + 1 + X dj + di slots in (rows 16 bytes apart, 8 channels each =
+// one core-matrix row).  Window p contributes to the output planes p - 1, p
+// and p + 1 in the same instructions (N = 48: tap planes dk = 1, 0, -1 side by
+// side), five tap pairs of M = 128 slots and K = 16.  What bounds the MMAs is
+// the A operand's way out of shared memory, 4 KB an instruction: a tile used
+// to be 15 instructions of N = 16, one output plane each.  The planes start
+// from zeros that the epilogue warps store; plane k sums dk = -1, 0, 1 and
+// within each the pairs in order.  Only instructions of one accumulator and
+// shape are sure to run in order, and the columns of one window overlap the
+// next one's: a window's instructions are issued when the window before is
+// done, while those of the SM's other CTAs run.  One thread of the producer
+// warp issues
+// the copies and the MMAs; 4 epilogue warps (one TMEM lane per thread) read
+// the accumulators back and store; the two sides meet only at mbarriers
+// (window landed, plane ready), so that the MMAs of the next planes run while
+// an epilogue stores.  8 RHS at 96^3: hidden layer 138 -> 97 us, deployment
+// 191 -> 102 us (u of the next plane is on its way while the MMAs run).
 //   MODE 0: hidden layer, bf16 [b][S] (guarded layout), zero on the planes
 //           i = X-1, j = Y-1, k = Z-1
 //   MODE 1: u += channels 0..5 on unknown edges (deployment)
@@ -264,6 +314,7 @@ struct ConvArgs {
   int XY;        // slots per plane
   int ncol;      // 128-slot columns per plane
   int nchunk;    // plane chunks per column
+  int planes;    // planes per chunk, at most kTcPlanes
   int W;         // window slots: 128 + 2X + 3
   int wbytes;    // window stride in shared memory (16 W rounded up to 128)
   const int* mask;
@@ -274,15 +325,24 @@ struct ConvArgs {
 
 constexpr int kTcEpiWarps = 4;  // epilogue warps (TMEM lanes 0..127); one producer warp
 constexpr int kTcThreads = 32 * (kTcEpiWarps + 1);
-constexpr int kTcRing = 7;      // plane windows in shared memory
-constexpr int kTcAhead = kTcRing - 3;  // planes loaded ahead of the MMAs
-constexpr int kTcPlanes = 32;   // planes per chunk
-constexpr int kTcCols = 32;     // tensor memory: 2 accumulators x 16 columns
+constexpr int kTcRing = 4;      // plane windows in shared memory
+constexpr int kTcAhead = kTcRing - 1;  // planes loaded ahead of the MMAs
+// A window waits for the one before it, so that what covers the waits is the
+// SM's other CTAs: short chunks with few windows and columns leave room for
+// seven.  Planes x windows, a whole application to 8 RHS at 96^3 with its host
+// side (673 us before): 16 x 7 618 us, 8 x 7 515, 8 x 4 516, 4 x 6 525, 4 x 5 506, 4 x 4 491,
+// 4 x 3 500.
+constexpr int kTcPlanes = 4;    // planes per chunk
+constexpr int kTcCols = 16 * kTcPlanes;  // tensor memory
+// a CTA asks for so much shared memory that no ninth one waits for columns
+constexpr int kConvSmemMin = 28 * 1024;
+// widest window taken, in bytes: rows of up to 930 slots
+constexpr int kTcWindowMax = 31872;
 // dynamic shared memory a CTA may ask for (227 KB less the static part)
 constexpr int kConvSmemMax = 227 * 1024 - 1024;
 __host__ __device__ inline long kTcGuard(int X, int Y) { return (long)X * Y + X + 129; }
 inline size_t conv_smem(const ConvArgs& a) {
-  return (size_t)kTcInstr * 512 + (size_t)kTcRing * a.wbytes;
+  return (size_t)kWtLayer * 16 + (size_t)kTcRing * a.wbytes;
 }
 
 template <int MODE>
@@ -293,8 +353,7 @@ __global__ void __launch_bounds__(kTcThreads) k_ls_conv(ConvArgs a, const uint4*
                                                         int* __restrict__ err) {
   extern __shared__ __align__(128) unsigned char dsm[];
   __shared__ __align__(8) uint64_t bar_full[kTcRing];  // window landed (bulk copy)
-  __shared__ __align__(8) uint64_t bar_done[2];        // accumulator ready (tcgen05.commit)
-  __shared__ __align__(8) uint64_t bar_free[2];        // accumulator read back (4 epilogue warps)
+  __shared__ __align__(8) uint64_t bar_mma[kTcPlanes + 2];  // window's MMAs done (tcgen05.commit)
   __shared__ uint32_t tmem_base;
   __shared__ volatile int failed;
   const int b = blockIdx.y;
@@ -305,16 +364,39 @@ __global__ void __launch_bounds__(kTcThreads) k_ls_conv(ConvArgs a, const uint4*
   __syncthreads();
   if (failed) return;
   const int col = blockIdx.x % a.ncol, chunk = blockIdx.x / a.ncol;
-  const int k0 = chunk * kTcPlanes;
-  const int k1 = min(k0 + kTcPlanes, a.Z - 1);  // planes [k0, k1) are computed
+  const int k0 = chunk * a.planes;
+  const int k1 = min(k0 + a.planes, a.Z - 1);  // planes [k0, k1) are computed
   const int tid = threadIdx.x, warp = tid >> 5;
   uint4* sB = reinterpret_cast<uint4*>(dsm);
-  unsigned char* ring = dsm + kTcInstr * 512;
+  unsigned char* ring = dsm + kWtLayer * 16;
   const int p0 = 128 * col;  // first in-plane slot of the column
 
-  for (int q = tid; q < kTcInstr * 32; q += blockDim.x) sB[q] = Wt[q];
-  // generic-proxy stores, read below by the tensor core (async proxy)
-  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+  // plane p -> ring slot and the parity of its use of that slot; a window's
+  // barrier completes once; plane k is done with window k + 1
+  auto slot = [&](int p) { return (p - k0 + 1) % kTcRing; };
+  auto parity = [&](int p) { return (uint32_t)(((p - k0 + 1) / kTcRing) & 1); };
+  auto done = [&](int p) { return su32(&bar_mma[p - k0 + 1]); };
+  // the producer's copies, the weights with the first window; the first ones
+  // start before tensor memory is there
+  const uint4* inb = in + (long)b * a.S;
+  int issued = k0 - 2;
+  auto load = [&](int p) {
+    const uint32_t bar = su32(&bar_full[slot(p)]);
+    const uint32_t wb = p == k0 - 1 ? 16u * kWtLayer : 0u;
+    mbar_expect_tx(bar, (uint32_t)a.W * 16u + wb);
+    if (wb) bulk_load(su32(sB), Wt, wb, bar);
+    bulk_load(su32(ring + slot(p) * a.wbytes), inb + (long)p * a.XY + p0 - a.X - 1,
+              (uint32_t)a.W * 16u, bar);
+    issued = p;
+  };
+  if (tid == 32 * kTcEpiWarps) {
+    for (int i = 0; i < kTcRing; i++) mbar_init(su32(&bar_full[i]), 1);
+    for (int i = 0; i < kTcPlanes + 2; i++) mbar_init(su32(&bar_mma[i]), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    if (!a.stall)
+      for (int p = k0 - 1; p <= min(k0 - 1 + kTcAhead, k1); p++) load(p);
+  }
   __syncwarp();
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
@@ -323,78 +405,58 @@ __global__ void __launch_bounds__(kTcThreads) k_ls_conv(ConvArgs a, const uint4*
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
-  if (tid == 0) {
-    for (int i = 0; i < kTcRing; i++) mbar_init(su32(&bar_full[i]), 1);
-    for (int i = 0; i < 2; i++) {
-      mbar_init(su32(&bar_done[i]), 1);
-      mbar_init(su32(&bar_free[i]), 4);
-    }
-    failed = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base;
-
-  // plane p -> ring slot and the parity of its use of that slot; plane k's
-  // accumulator (16 columns) alternates with k, its u-th use has parity u & 1
-  auto slot = [&](int p) { return (p - k0 + 1) % kTcRing; };
-  auto parity = [&](int p) { return (uint32_t)(((p - k0 + 1) / kTcRing) & 1); };
-  auto acc = [&](int k) { return (k - k0) & 1; };
-  auto use = [&](int k) { return (uint32_t)(((k - k0) >> 1) & 1); };
+  if (warp < kTcEpiWarps) {
+#pragma unroll
+    for (int c = 0; c < kTcCols; c += 32) tc_zero32(tmem + c + ((uint32_t)(warp * 32) << 16));
+    asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
 
   if (warp == kTcEpiWarps) {
     // ---- producer: one thread issues the window copies and the MMAs
     if ((tid & 31) == 0 && !a.stall) {
-      const uint4* inb = in + (long)b * a.S;
-      int issued = k0 - 2, waited = k0 - 2, committed = k0 - 1;
-      auto load = [&](int p) {
-        const uint32_t bar = su32(&bar_full[slot(p)]);
-        mbar_expect_tx(bar, (uint32_t)a.W * 16u);
-        bulk_load(su32(ring + slot(p) * a.wbytes), inb + (long)p * a.XY + p0 - a.X - 1,
-                  (uint32_t)a.W * 16u, bar);
-        issued = p;
-      };
-      for (int p = k0 - 1; p <= min(k0 + kTcAhead - 1, k1); p++) load(p);
+      int waited = k0 - 2, committed = k0 - 2;
       const uint32_t ring0 = su32(ring), sB0 = su32(sB);
-      for (int k = k0; k < k1; k++) {
-        bool ok = true;
-        // accumulator acc(k) and the window slot of plane k-3 are free once
-        // the epilogue of plane k-2 has read its accumulator back
-        if (k - 2 >= k0) ok = mbar_wait(su32(&bar_free[acc(k)]), use(k) ^ 1u, a.wait);
-        if (ok && k + kTcAhead <= k1) load(k + kTcAhead);
-        for (int p = waited + 1; p <= k + 1 && ok; p++) {
-          ok = mbar_wait(su32(&bar_full[slot(p)]), parity(p), a.wait);
-          if (ok) waited = p;
-        }
+      for (int p = k0 - 1; p <= k1; p++) {
+        // window p-1's MMAs done: its slot is free, its columns may be added to
+        bool ok = p == k0 - 1 || mbar_wait(done(p - 1), 0u, a.wait);
+        if (ok && p >= k0 && p + kTcAhead <= k1) load(p + kTcAhead);
+        if (ok) ok = mbar_wait(su32(&bar_full[slot(p)]), parity(p), a.wait);
         if (!ok || failed) {
           failed = 1;
           atomicExch(err, 1);
           break;
         }
+        waited = p;
         tc_fence_after();
-        const uint32_t d = tmem + 16u * (uint32_t)acc(k);
+        // output planes p - 1 + o, o in [o0, o1), that the chunk computes
+        const int o0 = max(0, k0 - (p - 1)), o1 = min(3, k1 - (p - 1));
+        const uint32_t base = ring0 + slot(p) * a.wbytes;
+        const uint32_t d = tmem + 16u * (uint32_t)(p - 1 + o0 - k0);
 #pragma unroll
-        for (int q = 0; q < kTcInstr; q++) {
-          const int dk = q / 5 - 1, pi = q % 5;
+        for (int pi = 0; pi < kTcPairs; pi++) {
           const int r0 = 2 * pi;
           const int off0 = (r0 / 3 - 1) * a.X + (r0 % 3 - 1);
           const int off1 = pi < 4 ? ((r0 + 1) / 3 - 1) * a.X + ((r0 + 1) % 3 - 1) : off0 + 1;
-          const uint32_t base = ring0 + slot(k + dk) * a.wbytes;
           const uint64_t ad = smem_desc(base + 16u * (uint32_t)(a.X + 1 + off0),
                                         16u * (uint32_t)(off1 - off0), 128u);
-          const uint64_t bd = smem_desc(sB0 + 512u * q, 256u, 128u);
-          tc_mma(d, ad, bd, q > 0 ? 1u : 0u);
+          const uint64_t bd = smem_desc(sB0 + 32u * kTcN * pi + 256u * o0, 16u * kTcN, 128u);
+          tc_mma(d, ad, bd, 16u * (uint32_t)(o1 - o0));
         }
-        tc_commit(su32(&bar_done[acc(k)]));
-        committed = k;
+        tc_commit(done(p));
+        committed = p;
       }
       if (failed) {
         // copies and MMAs in flight finish before shared and tensor memory go
         for (int p = waited + 1; p <= issued; p++)
           mbar_wait(su32(&bar_full[slot(p)]), parity(p), a.wait);
-        if (committed >= k0) mbar_wait(su32(&bar_done[acc(committed)]), use(committed), a.wait);
+        if (committed >= k0 - 1) mbar_wait(done(committed), 0u, a.wait);
       }
     }
   } else {
@@ -402,8 +464,21 @@ __global__ void __launch_bounds__(kTcThreads) k_ls_conv(ConvArgs a, const uint4*
     const int p = p0 + tid;
     const bool live = p < a.XY;
     const int j = live ? p / a.X : 0, i = p - j * a.X;
+    // MODE 1: u of the next plane is loaded before the wait for this one's MMAs
+    float2 w[3] = {}, wn[3] = {};
+    float2* ub = out + (long)b * 3 * a.S + p;
+    auto preload = [&](int k) {
+      if (MODE != 1 || !live || k >= k1) return;
+#pragma unroll
+      for (int c = 0; c < 3; c++)
+        if (unknown_any(c, a.n, i, j, k)) wn[c] = ub[c * a.S + (long)k * a.XY];
+    };
+    preload(k0);
     for (int k = k0; k < k1; k++) {
-      const bool late = !mbar_wait(su32(&bar_done[acc(k)]), use(k), a.wait);
+#pragma unroll
+      for (int c = 0; c < 3; c++) w[c] = wn[c];
+      preload(k + 1);
+      const bool late = !mbar_wait(done(k + 1), 0u, a.wait);
       // the warp leaves together (tcgen05.ld below is warp-collective)
       if (__any_sync(0xffffffffu, late || failed)) {
         if (late) {
@@ -415,10 +490,7 @@ __global__ void __launch_bounds__(kTcThreads) k_ls_conv(ConvArgs a, const uint4*
       tc_fence_after();
       __syncwarp();
       float v[8];
-      tc_load8(tmem + 16u * (uint32_t)acc(k) + ((uint32_t)(warp * 32) << 16), v);
-      tc_fence_before();
-      __syncwarp();
-      if ((tid & 31) == 0) mbar_arrive(su32(&bar_free[acc(k)]));
+      tc_load8(tmem + 16u * (uint32_t)(k - k0) + ((uint32_t)(warp * 32) << 16), v);
       if (live) {
         const long s = (long)k * a.XY + p;
         if (MODE == 0) {
@@ -433,12 +505,7 @@ __global__ void __launch_bounds__(kTcThreads) k_ls_conv(ConvArgs a, const uint4*
             float2* ob = out + ((long)b * 3 + c) * a.S + s;
             const bool unk = unknown_any(c, a.n, i, j, k);
             if (MODE == 1) {
-              if (unk) {
-                float2 w = *ob;
-                w.x += v[2 * c];
-                w.y += v[2 * c + 1];
-                *ob = w;
-              }
+              if (unk) *ob = make_float2(w[c].x + v[2 * c], w[c].y + v[2 * c + 1]);
             } else {
               *ob = unk ? make_float2(v[2 * c], v[2 * c + 1]) : make_float2(0.f, 0.f);
             }
@@ -596,7 +663,7 @@ __global__ void k_ls_adam(float* __restrict__ W, const float* __restrict__ dW,
   W[i] -= lr * (a / c1) / (sqrtf(v / c2) + eps);
 }
 
-ConvArgs conv_args(const int n[3], const int* mask) {
+ConvArgs conv_args(const int n[3], const int* mask, int nb) {
   ConvArgs a;
   for (int e = 0; e < 3; e++) a.n[e] = n[e];
   a.X = n[0] + 1;
@@ -605,7 +672,13 @@ ConvArgs conv_args(const int n[3], const int* mask) {
   a.S = (long)a.X * a.Y * a.Z;
   a.XY = a.X * a.Y;
   a.ncol = (a.XY + 127) / 128;
-  a.nchunk = (a.Z - 1 + kTcPlanes - 1) / kTcPlanes;
+  // chunks of at most kTcPlanes planes, shorter where few columns would leave
+  // SMs idle (each chunk reads two windows more than it computes)
+  const int zc = a.Z - 1;
+  const long fill = 4L * kSMs / ((long)a.ncol * nb);
+  a.nchunk = std::max((zc + kTcPlanes - 1) / kTcPlanes, (int)std::min<long>(fill, zc / 2));
+  a.planes = (zc + a.nchunk - 1) / a.nchunk;
+  a.nchunk = (zc + a.planes - 1) / a.planes;
   a.W = 128 + 2 * a.X + 3;
   a.wbytes = (16 * a.W + 127) / 128 * 128;
   a.mask = mask;
@@ -636,7 +709,7 @@ void launch_conv(const ConvArgs& a, int nb, const uint32_t* in, const uint4* Wt,
                  float2* out, cudaStream_t st) {
   int* err = conv_err();
   dim3 g((unsigned)(a.ncol * a.nchunk), nb);
-  k_ls_conv<MODE><<<g, kTcThreads, conv_smem(a), st>>>(a, reinterpret_cast<const uint4*>(in), Wt,
+  k_ls_conv<MODE><<<g, kTcThreads, std::max<size_t>(conv_smem(a), kConvSmemMin), st>>>(a, reinterpret_cast<const uint4*>(in), Wt,
                                                 reinterpret_cast<uint4*>(hid), out, err);
 }
 
@@ -644,31 +717,29 @@ void launch_conv(const ConvArgs& a, int nb, const uint32_t* in, const uint4* Wt,
 
 // ---------------------------------------------------------------- host API
 void learned_pack(const float* dW32, uint4* dWt, cudaStream_t st) {
-  k_ls_pack<<<(2 * kTcInstr * 32 + 127) / 128, 128, 0, st>>>(dW32, dWt);
+  k_ls_pack<<<(2 * kWtLayer + 127) / 128, 128, 0, st>>>(dW32, dWt);
 }
 
 // u += N(D^-1 (f - A u)) on the RHS that mask selects (level-0 view L);
 // wait > 0 / stall: the convolutions' wait limit and test stall (ConvArgs)
 void learned_apply(const LevelView<float>& L, const uint4* Wt, uint32_t* X, uint32_t* H,
                    cudaStream_t st, long long wait = 0, int stall = 0) {
-  dim3 g1((unsigned)((L.S + 255) / 256), L.nrhs);
-  k_ls_input<<<g1, 256, 0, st>>>(L, nullptr, X);
-  ConvArgs a = conv_args(L.n, L.active);
+  launch_ls_input(L, nullptr, X, st);
+  ConvArgs a = conv_args(L.n, L.active, L.nrhs);
   if (wait > 0) a.wait = wait;
   a.stall = stall;
   launch_conv<0>(a, L.nrhs, X, Wt, H, nullptr, st);
-  launch_conv<1>(a, L.nrhs, H, Wt + kTcInstr * 32, nullptr, L.u, st);
+  launch_conv<1>(a, L.nrhs, H, Wt + kWtLayer, nullptr, L.u, st);
 }
 
 // slots of zero guard before and after a bf16 slot buffer of the level
 long learned_guard(const int n[3]) { return kTcGuard(n[0] + 1, n[1] + 1); }
 
 // the shared memory one convolution needs on a level of n cells, or -1 if
-// it is more than a CTA can have
+// its windows are too wide
 long learned_smem(const int n[3]) {
-  const ConvArgs a = conv_args(n, nullptr);
-  const size_t b = conv_smem(a);
-  return b <= (size_t)kConvSmemMax ? (long)b : -1;
+  const ConvArgs a = conv_args(n, nullptr, 1);
+  return a.wbytes <= kTcWindowMax ? (long)conv_smem(a) : -1;
 }
 
 // a convolution's give-up code since the last check (0: none); clears it
@@ -698,14 +769,14 @@ struct TrainBuffers {
 int learned_train_step(const LevelView<float>& L, const TrainBuffers& B, int step, float lr,
                        cudaStream_t st) {
   const int nb = L.nrhs;
-  ConvArgs a = conv_args(L.n, nullptr);
+  ConvArgs a = conv_args(L.n, nullptr, nb);
   dim3 gs((unsigned)((L.S + 255) / 256), nb);
   LevelView<float> V = L;
   V.active = nullptr;
   // forward: X = D^-1 r, H = W1 * X, c = W2 * H (masked)
-  k_ls_input<<<gs, 256, 0, st>>>(V, V.f, B.X);
+  launch_ls_input(V, V.f, B.X, st);
   launch_conv<0>(a, nb, B.X, B.Wt, B.H, nullptr, st);
-  launch_conv<2>(a, nb, B.H, B.Wt + kTcInstr * 32, nullptr, B.c, st);
+  launch_conv<2>(a, nb, B.H, B.Wt + kWtLayer, nullptr, B.c, st);
   // e = r - A c and |e|^2
   cudaMemsetAsync(B.loss2, 0, nb * sizeof(double), st);
   LevelView<float> R = V;
@@ -892,7 +963,7 @@ int train_impl(emmi_solver* s, int steps, float lr, float* W, float* loss, float
   LCK(A.get(&B.dW, nw * sizeof(float)));
   LCK(A.get(&B.m1, nw * sizeof(float)));
   LCK(A.get(&B.m2, nw * sizeof(float)));
-  LCK(A.get(&B.Wt, (size_t)2 * kTcInstr * 32 * sizeof(uint4)));
+  LCK(A.get(&B.Wt, (size_t)2 * kWtLayer * sizeof(uint4)));
   LCK(cudaMemcpyAsync(B.W, W, nw * sizeof(float), cudaMemcpyHostToDevice, st));
   LCK(cudaMemsetAsync(B.m1, 0, nw * sizeof(float), st));
   LCK(cudaMemsetAsync(B.m2, 0, nw * sizeof(float), st));
@@ -1063,7 +1134,7 @@ int emmi_learned_set(emmi_solver* s, const float* W) {
     const size_t xb = (size_t)(s->nrhs * S + 2 * gd) * 16;
     uint32_t *rx = nullptr, *rh = nullptr;
     if ((rc = s->alloc((void**)&s->d_lsW, 2 * kWLayer * sizeof(float))) != EMMI_OK) return rc;
-    if ((rc = s->alloc((void**)&s->d_lsWt, (size_t)2 * kTcInstr * 32 * sizeof(uint4))) != EMMI_OK)
+    if ((rc = s->alloc((void**)&s->d_lsWt, (size_t)2 * kWtLayer * sizeof(uint4))) != EMMI_OK)
       return rc;
     if ((rc = s->alloc((void**)&rx, xb)) != EMMI_OK) return rc;
     if ((rc = s->alloc((void**)&rh, xb)) != EMMI_OK) return rc;
