@@ -40,8 +40,8 @@ long line_scratch_elems(const int n[3], int d, int nrhs);
 // (emmi_lines.cu), fmt kFacF32 with 48 or kFacF16 (fp16 L, fp32 1/d) with 28
 // bytes a row; line_factor_elems values of T per group.  launch_line_factor
 // fills them for the L.nrhs groups of L (L.op / L.wmu per group, u and f
-// unused), the band rows assembled in registers, into fac + g *
-// line_factor_elems and sets *ovf when an L value does not fit fp16 (kFacF16);
+// unused) and the four colours of direction d, the band rows assembled in
+// registers, into fac + off[color] + g * line_factor_elems and sets *ovf when an L value does not fit fp16 (kFacF16);
 // launch_line_sweep_fac then sweeps RHS r with the factors of group grp[r], rb
 // holding line_rb_elems complex values per RHS, in line_fac_launches launches;
 // coef (complex128, may be null): launch_coef64's coefficients of the level
@@ -50,7 +50,7 @@ int line_tile_width(const int n[3], int d, int nrhs, int fmt);
 long line_factor_elems(const int n[3], int d, int color, int fmt, int tile);
 long line_rb_elems(const int n[3], int d, int color, int tile);
 template <typename T>
-void launch_line_factor(const LevelView<T>& L, int d, int color, T* fac, int fmt, int tile,
+void launch_line_factor(const LevelView<T>& L, int d, T* fac, const long off[4], int fmt, int tile,
                         int* ovf, cudaStream_t st);
 // block shapes of a stored-factor sweep: the complex64 substitution's variant
 // (subst_variant_threads lines per block, a ring of subst_variant_ring groups

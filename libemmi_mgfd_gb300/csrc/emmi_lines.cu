@@ -511,22 +511,30 @@ __device__ __forceinline__ void eliminate_end(int G, int nd, float2 (&W)[21], fl
   }
 }
 
-// Factors of every line of one colour for group blockIdx.y of operators and
-// frequencies: a warp per end of 32 lines, each thread assembling its rows in
+// where the factors of a direction's four colours lie, and of a group in them
+struct FacBlocks {
+  long off[4], gstride[4];
+};
+
+// Factors of every line of colour blockIdx.z for group blockIdx.y of operators
+// and frequencies.  A line's rows are a chain of some 40 dependent operations
+// each and a colour has few lines (1024 at 64^3: 32 blocks), so that the chain
+// is the launch's time: the colours, which do not depend on one another, share
+// a launch (all of 64^3's: 4.5 -> 1.5 ms).  A warp per end of 32 lines, each thread assembling its rows in
 // registers (band_row) and eliminating them.  The mirrored end hands its
 // Schur complement of the middle rows to the other through shared memory.
 // An fp16 L value outside its range (or not finite) sets *ovf.
 template <int D, int FMT>
-__global__ void __launch_bounds__(64) k_line_factor_ends(LevelView<float> L, int pa, int pb,
-                                                         LineTile tl, long gstride,
-                                                         float* __restrict__ fac,
+__global__ void __launch_bounds__(64) k_line_factor_ends(LevelView<float> L, LineTile tl,
+                                                         FacBlocks fb, float* __restrict__ fac,
                                                          int* __restrict__ ovf) {
   constexpr int A = (D == 0) ? 1 : 0, B = (D == 2) ? 1 : 2;
   __shared__ float2 schur[15][32];
-  const int grp = blockIdx.y;
-  const LineGeom g = line_geom<D>(L.n, pa, pb);
+  const int grp = blockIdx.y, color = blockIdx.z;
+  const LineGeom g = line_geom<D>(L.n, color & 1, color >> 1);
   const int lane = threadIdx.x & 31;
   const long l0 = blockIdx.x * 32L + lane;
+  if (blockIdx.x * 32L >= g.nl) return;  // a colour with fewer lines
   const bool live = l0 < g.nl;
   const long l = live ? l0 : g.nl - 1;
   const unsigned lq = (unsigned)l / (unsigned)g.la;
@@ -535,7 +543,7 @@ __global__ void __launch_bounds__(64) k_line_factor_ends(LevelView<float> L, int
   const Geo<float> Gm{L.geo + (long)op_of(L, grp) * L.gstride, L.gmax1};
   const float wmu = L.wmu[grp];
   const int nd = g.nd, G = tl.mid / 5, TW = 1 << tl.shift, ln = (int)(l & (TW - 1));
-  unsigned char* out = reinterpret_cast<unsigned char*>(fac + (long)grp * gstride) +
+  unsigned char* out = reinterpret_cast<unsigned char*>(fac + fb.off[color] + (long)grp * fb.gstride[color]) +
                        (l >> tl.shift) * g.m * kFacRow<FMT> * TW;
   bool over = false;
   float2 W[21], lq5[6];
@@ -1482,22 +1490,31 @@ static void line_sweep_fac_d(const LevelView<T>& L, int color, const T* fac, con
 }
 
 template <typename T, int D>
-static void line_factor_d(const LevelView<T>& L, int color, T* fac, int fmt, int tile, int* ovf,
-                          cudaStream_t st) {
-  const int pa = color & 1, pb = (color >> 1) & 1;
-  const long nl = line_count(L.n, D, color);
-  if (nl == 0) return;
-  const long gstride = line_factor_elems(L.n, D, color, fmt, tile);
+static void line_factor_d(const LevelView<T>& L, T* fac, const long off[4], int fmt, int tile,
+                          int* ovf, cudaStream_t st) {
+  FacBlocks fb;
+  long most = 0;
+  for (int c = 0; c < 4; c++) {
+    fb.off[c] = off[c];
+    fb.gstride[c] = line_factor_elems(L.n, D, c, fmt, tile);
+    most = std::max(most, line_count(L.n, D, c));
+  }
+  if (most == 0) return;
   if constexpr (std::is_same<T, float>::value) {
     const LineTile tl = line_tile(L.n[D], tile);
-    dim3 g((unsigned)((nl + 31) / 32), L.nrhs);
+    dim3 g((unsigned)((most + 31) / 32), L.nrhs, 4);
     if (fmt == kFacF16)
-      k_line_factor_ends<D, kFacF16><<<g, 64, 0, st>>>(L, pa, pb, tl, gstride, fac, ovf);
+      k_line_factor_ends<D, kFacF16><<<g, 64, 0, st>>>(L, tl, fb, fac, ovf);
     else
-      k_line_factor_ends<D, kFacF32><<<g, 64, 0, st>>>(L, pa, pb, tl, gstride, fac, ovf);
+      k_line_factor_ends<D, kFacF32><<<g, 64, 0, st>>>(L, tl, fb, fac, ovf);
   } else {
-    dim3 g((unsigned)((nl + kSolveThreads - 1) / kSolveThreads), L.nrhs);
-    k_line_factor_direct<T, D><<<g, kSolveThreads, 0, st>>>(L, pa, pb, gstride, fac);
+    for (int c = 0; c < 4; c++) {
+      const long nl = line_count(L.n, D, c);
+      if (nl == 0) continue;
+      dim3 g((unsigned)((nl + kSolveThreads - 1) / kSolveThreads), L.nrhs);
+      k_line_factor_direct<T, D><<<g, kSolveThreads, 0, st>>>(L, c & 1, c >> 1, fb.gstride[c],
+                                                              fac + fb.off[c]);
+    }
   }
 }
 
@@ -1529,11 +1546,11 @@ int line_fac_launches(const int n[3], int d, int color, int nrhs, int tile, int 
 }
 
 template <typename T>
-void launch_line_factor(const LevelView<T>& L, int d, int color, T* fac, int fmt, int tile,
+void launch_line_factor(const LevelView<T>& L, int d, T* fac, const long off[4], int fmt, int tile,
                         int* ovf, cudaStream_t st) {
-  if (d == 0) line_factor_d<T, 0>(L, color, fac, fmt, tile, ovf, st);
-  else if (d == 1) line_factor_d<T, 1>(L, color, fac, fmt, tile, ovf, st);
-  else line_factor_d<T, 2>(L, color, fac, fmt, tile, ovf, st);
+  if (d == 0) line_factor_d<T, 0>(L, fac, off, fmt, tile, ovf, st);
+  else if (d == 1) line_factor_d<T, 1>(L, fac, off, fmt, tile, ovf, st);
+  else line_factor_d<T, 2>(L, fac, off, fmt, tile, ovf, st);
 }
 
 template <typename T>
@@ -1544,10 +1561,10 @@ void launch_line_sweep_fac(const LevelView<T>& L, int d, int color, const T* fac
   else if (d == 1) line_sweep_fac_d<T, 1>(L, color, fac, grp, rb, fmt, tile, sh, coef, st);
   else line_sweep_fac_d<T, 2>(L, color, fac, grp, rb, fmt, tile, sh, coef, st);
 }
-template void launch_line_factor<float>(const LevelView<float>&, int, int, float*, int, int, int*,
-                                        cudaStream_t);
-template void launch_line_factor<double>(const LevelView<double>&, int, int, double*, int, int,
-                                         int*, cudaStream_t);
+template void launch_line_factor<float>(const LevelView<float>&, int, float*, const long*, int, int,
+                                        int*, cudaStream_t);
+template void launch_line_factor<double>(const LevelView<double>&, int, double*, const long*, int,
+                                         int, int*, cudaStream_t);
 template void launch_line_sweep_fac<float>(const LevelView<float>&, int, int, const float*,
                                            const int*, C_t<float>*, int, int, cudaStream_t,
                                            SweepShape, const double*);

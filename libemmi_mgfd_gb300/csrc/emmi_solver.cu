@@ -692,7 +692,7 @@ static int build_line_factors(emmi_solver* s) {
     if ((rc = s->alloc((void**)&s->d_fac, bytes)) != EMMI_OK) return rc;
     CK(cudaMemsetAsync(d_ovf, 0, sizeof(int), s->st));
     s->fac_bytes = bytes;
-    // factor every block once, every group in one launch per colour
+    // factor every block once, every group and colour in one launch
     std::vector<long> done;
     for (int h = 0; h < 3; h++)
       for (int l = 0; l + 1 < s->lmax; l++)
@@ -708,9 +708,8 @@ static int build_line_factors(emmi_solver* s) {
           V.wmu = static_cast<const T*>(s->d_gwmu);
           V.active = nullptr;
           V.nrhs = ng;
-          for (int c = 0; c < 4; c++)
-            launch_line_factor<T>(V, d, c, static_cast<T*>(s->d_fac) + s->fac_off[hb][l][d][c], fmt,
-                                  s->fac_tile[hb][l][d], d_ovf, s->st);
+          launch_line_factor<T>(V, d, static_cast<T*>(s->d_fac), s->fac_off[hb][l][d], fmt,
+                                s->fac_tile[hb][l][d], d_ovf, s->st);
         }
     CK(cudaGetLastError());
     int ovf = 0;
