@@ -106,6 +106,7 @@ __device__ __forceinline__ void dep_next() {
 // early successor, whose blocks then hold shared memory beside its own last
 // ones (25 at 128^3: 431 ms with every launch dependent).
 constexpr long kDepBlocks = 1216;
+inline bool depends(dim3 grid) { return (long)grid.x * grid.y * grid.z <= kDepBlocks; }
 template <typename... P, typename... A>
 inline void launch_dep(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                        A&&... args) {
@@ -117,7 +118,7 @@ inline void launch_dep(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cuda
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed =
-      (long)grid.x * grid.y * grid.z <= kDepBlocks ? 1 : 0;
+      depends(grid) ? 1 : 0;
   cfg.attrs = at;
   cfg.numAttrs = 1;
   cudaLaunchKernelEx(&cfg, k, P(args)...);
@@ -336,7 +337,9 @@ __device__ __forceinline__ void slot_nodes(long s, const LevelView<T>& L, int P[
 
 // (A u) of the edge equation of component C at slot s, and its coefficients
 // (W: edge_coef's cell weights)
-template <typename T, int C, int W = 2>
+// RO: read-only loads of u, which move past the kernel's own stores
+// (only in a kernel launched the ordinary way)
+template <typename T, int C, int W = 2, bool RO = false>
 __device__ __forceinline__ C_t<T> apply_row(const LevelView<T>& L, const C_t<T>* __restrict__ u,
                                             const T* __restrict__ cells, const Geo<T>& G, T wmu,
                                             const int P[3], long s, const long ss[3],
@@ -348,12 +351,16 @@ __device__ __forceinline__ C_t<T> apply_row(const LevelView<T>& L, const C_t<T>*
   edge_coef<T, C, W>(L.n, P, cells + (long)C * L.ncell, cells + 3 * L.ncell, G, wmu, e, L.imu_vol);
   const int si = (int)s, Si = (int)L.S;
   const int s3[3] = {1, (int)ss[1], (int)ss[2]};
-  const C_t<T> uc = u[C * Si + si];
+  auto ld = [&](int o) {
+    if constexpr (RO) return ldro(u + o);
+    else return u[o];
+  };
+  const C_t<T> uc = ld(C * Si + si);
   T ar = e.dre * uc.x - e.dim * uc.y;
   T ai = e.dre * uc.y + e.dim * uc.x;
 #pragma unroll
   for (int k = 0; k < 12; k++) {
-    const C_t<T> v = u[si + nbr_delta32<C>(k, s3, Si)];
+    const C_t<T> v = ld(si + nbr_delta32<C>(k, s3, Si));
     ar += e.c[k] * v.x;
     ai += e.c[k] * v.y;
   }

@@ -361,7 +361,7 @@ __device__ __forceinline__ void assemble_row(const LevelView<T>& L, const C_t<T>
   P[B] = tb - (TT == 3 ? 1 : 0);
   const int sl = P[0] + (L.n[0] + 1) * (P[1] + (L.n[1] + 1) * P[2]);  // 32-bit slot
   EdgeCoef<T> e;
-  const C_t<T> au = apply_row<T, C>(L, u, cells, G, wmu, P, sl, ss, e);
+  const C_t<T> au = apply_row<T, C, 2, true>(L, u, cells, G, wmu, P, sl, ss, e);
   const C_t<T> r = csub<T>(f[C * (int)L.S + sl], au);
   T band[5] = {0, 0, 0, 0, 0};
 #define LINE_ENTRY(K)                                                         \
@@ -390,8 +390,6 @@ template <typename T, int D>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_line_assemble(LevelView<T> L,
                                                                               int pa, int pb,
                                                                               T* __restrict__ buf) {
-  dep_wait();
-  dep_next();
   constexpr int A = (D == 0) ? 1 : 0, B = (D == 2) ? 1 : 2;
   const int rhs = blockIdx.y;
   if (L.active && !L.active[rhs]) return;
@@ -428,8 +426,6 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_line_assemble(L
 template <typename T, int D>
 __global__ void __launch_bounds__(256) k_line_assemble_rows(LevelView<T> L, int pa, int pb,
                                                             T* __restrict__ buf) {
-  dep_wait();
-  dep_next();
   constexpr int A = (D == 0) ? 1 : 0, B = (D == 2) ? 1 : 2;
   const int rhs = blockIdx.y;
   if (L.active && !L.active[rhs]) return;
@@ -474,8 +470,6 @@ template <typename T>
 __global__ void __launch_bounds__(kSolveThreads) k_line_solve(const int* __restrict__ active,
                                                               long nl, int m,
                                                               T* __restrict__ buf) {
-  dep_wait();
-  dep_next();
   using V = typename Vec16<T>::V;
   constexpr int NP = kPlanes<T>;
   __shared__ V ring[kRing][NP][kSolveThreads];
@@ -592,8 +586,6 @@ __global__ void __launch_bounds__(kSolveThreads) k_line_solve(const int* __restr
 template <typename T, int D>
 __global__ void __launch_bounds__(256) k_line_apply(LevelView<T> L, int pa, int pb,
                                                     const T* buf) {
-  dep_wait();
-  dep_next();
   const int rhs = blockIdx.y;
   if (L.active && !L.active[rhs]) return;
   const LineGeom g = line_geom<D>(L.n, pa, pb);
@@ -606,16 +598,19 @@ __global__ void __launch_bounds__(256) k_line_apply(LevelView<T> L, int pa, int 
   C_t<T>* u = L.u + (long)rhs * 3 * L.S;
   const V* base = reinterpret_cast<const V*>(buf) + (long)rhs * g.m * kPlanes<T> * g.nl + l;
   const int r0 = 5 * (s - 1);
-  auto add = [&](long sl, int row) {
-    u[sl] = cadd<T>(u[sl], rec_get_x<T>(base + (long)row * kPlanes<T> * g.nl, g.nl));
-  };
-  add(line_slot<D, 0>(L.n, L.S, ta, tb, s), r0);
-  if (s < g.nd) {
-    add(line_slot<D, 1>(L.n, L.S, ta, tb, s), r0 + 1);
-    add(line_slot<D, 2>(L.n, L.S, ta, tb, s), r0 + 2);
-    add(line_slot<D, 3>(L.n, L.S, ta, tb, s), r0 + 3);
-    add(line_slot<D, 4>(L.n, L.S, ta, tb, s), r0 + 4);
-  }
+  // every load before the first store
+  auto x = [&](int row) { return rec_get_x<T>(base + (long)row * kPlanes<T> * g.nl, g.nl); };
+  const long sl[5] = {line_slot<D, 0>(L.n, L.S, ta, tb, s), line_slot<D, 1>(L.n, L.S, ta, tb, s),
+                      line_slot<D, 2>(L.n, L.S, ta, tb, s), line_slot<D, 3>(L.n, L.S, ta, tb, s),
+                      line_slot<D, 4>(L.n, L.S, ta, tb, s)};
+  const int nr = s < g.nd ? 5 : 1;
+  C_t<T> v[5];
+#pragma unroll
+  for (int t = 0; t < 5; t++)
+    if (t < nr) v[t] = cadd<T>(u[sl[t]], x(r0 + t));
+#pragma unroll
+  for (int t = 0; t < 5; t++)
+    if (t < nr) u[sl[t]] = v[t];
 }
 
 template <typename T, int D>
@@ -626,15 +621,19 @@ static void line_sweep_d(const LevelView<T>& L, int color, T* buf, cudaStream_t 
   const long items = nl * L.n[D];
   const int m = 5 * L.n[D] - 4;
   dim3 g1((unsigned)((items + 255) / 256), L.nrhs);
+  // launched the ordinary way: blocks of the solve that start beside the
+  // assembly's last ones find its shared-memory carveout, too small for more
+  // than a few of them an SM (complex128, four shots at 128^3, three cycles:
+  // 1.06 s with dependent launches, 0.79 s so)
   if (D == 0) {
     dim3 g5((unsigned)((5 * items + 255) / 256), L.nrhs);
-    launch_dep(k_line_assemble_rows<T, D>, g5, 256, 0, st, L, pa, pb, buf);
+    k_line_assemble_rows<T, D><<<g5, 256, 0, st>>>(L, pa, pb, buf);
   } else {
-    launch_dep(k_line_assemble<T, D>, g1, 256, 0, st, L, pa, pb, buf);
+    k_line_assemble<T, D><<<g1, 256, 0, st>>>(L, pa, pb, buf);
   }
   dim3 g2((unsigned)((nl + kSolveThreads - 1) / kSolveThreads), L.nrhs);
-  launch_dep(k_line_solve<T>, g2, kSolveThreads, 0, st, L.active, nl, m, buf);
-  launch_dep(k_line_apply<T, D>, g1, 256, 0, st, L, pa, pb, buf);
+  k_line_solve<T><<<g2, kSolveThreads, 0, st>>>(L.active, nl, m, buf);
+  k_line_apply<T, D><<<g1, 256, 0, st>>>(L, pa, pb, buf);
 }
 // the line solve keeps a cp.async ring in shared memory: ask for the
 // largest shared-memory carveout so 12 blocks fit on an SM

@@ -67,7 +67,7 @@ __host__ __device__ __forceinline__ long rb_elems(const LineTile& t, long nl) {
     return nl * t.m;
 }
 
-template <typename T, int D, int TT, int C>
+template <typename T, int D, int TT, int C, bool RO>
 __device__ __forceinline__ C_t<T> row_residual(const LevelView<T>& L, const C_t<T>* u,
                                                const C_t<T>* f, const T* cells,
                                                const Geo<T>& G, T wmu, int ta, int tb, int s,
@@ -79,7 +79,7 @@ __device__ __forceinline__ C_t<T> row_residual(const LevelView<T>& L, const C_t<
   P[B] = tb - (TT == 3 ? 1 : 0);
   const int sl = P[0] + (L.n[0] + 1) * (P[1] + (L.n[1] + 1) * P[2]);  // 32-bit slot
   EdgeCoef<T> e;
-  const C_t<T> au = apply_row<T, C, 0>(L, u, cells, G, wmu, P, sl, ss, e);
+  const C_t<T> au = apply_row<T, C, 0, RO>(L, u, cells, G, wmu, P, sl, ss, e);
   return csub<T>(f[C * (int)L.S + sl], au);
 }
 
@@ -125,12 +125,14 @@ __device__ __forceinline__ double2 row_residual_coef(const LevelView<double>& L,
 // rb = residual of every row of one colour; y and z lines:
 // a thread per (line, node) and its five rows; x lines: a thread per
 // (row type, line, node), row type slowest
-template <typename T, int D, bool CF>
+template <typename T, int D, bool CF, bool RO>
 __global__ void __launch_bounds__(256) k_line_rhs(LevelView<T> L, int pa, int pb, LineDiv dv,
                                                   LineTile tl, C_t<T>* __restrict__ rb,
                                                   const double* __restrict__ coef) {
-  dep_wait();
-  dep_next();
+  if constexpr (!RO) {
+    dep_wait();
+    dep_next();
+  }
   constexpr int A = (D == 0) ? 1 : 0, B = (D == 2) ? 1 : 2;
   const int rhs = blockIdx.y;
   if (L.active && !L.active[rhs]) return;
@@ -161,7 +163,7 @@ __global__ void __launch_bounds__(256) k_line_rhs(LevelView<T> L, int pa, int pb
   auto row = [&](auto tt, auto comp) {
     constexpr int TT = decltype(tt)::value, C = decltype(comp)::value;
     if constexpr (CF) return row_residual_coef<D, TT, C>(L, u, f, cf, wmu, ta, tb, s, ss);
-    else return row_residual<T, D, TT, C>(L, u, f, cells, G, wmu, ta, tb, s, ss);
+    else return row_residual<T, D, TT, C, RO>(L, u, f, cells, G, wmu, ta, tb, s, ss);
   };
   auto put = [&](int row, C_t<T> v) { out[rb_index<T>(tl, g.nl, l, row)] = v; };
   if (D == 0) {
@@ -1326,14 +1328,18 @@ __global__ void __launch_bounds__(256) k_line_apply_rb(LevelView<T> L, int pa, i
   C_t<T>* u = L.u + (long)rhs * 3 * L.S;
   const C_t<T>* x = rb + (long)rhs * rb_elems<T>(tl, g.nl);
   const int r0 = 5 * (s - 1);
-  auto add = [&](long sl, int row) { u[sl] = cadd<T>(u[sl], x[rb_index<T>(tl, g.nl, l, row)]); };
-  add(line_slot<D, 0>(L.n, L.S, ta, tb, s), r0);
-  if (s < g.nd) {
-    add(line_slot<D, 1>(L.n, L.S, ta, tb, s), r0 + 1);
-    add(line_slot<D, 2>(L.n, L.S, ta, tb, s), r0 + 2);
-    add(line_slot<D, 3>(L.n, L.S, ta, tb, s), r0 + 3);
-    add(line_slot<D, 4>(L.n, L.S, ta, tb, s), r0 + 4);
-  }
+  // every load before the first store
+  const long sl[5] = {line_slot<D, 0>(L.n, L.S, ta, tb, s), line_slot<D, 1>(L.n, L.S, ta, tb, s),
+                      line_slot<D, 2>(L.n, L.S, ta, tb, s), line_slot<D, 3>(L.n, L.S, ta, tb, s),
+                      line_slot<D, 4>(L.n, L.S, ta, tb, s)};
+  const int nr = s < g.nd ? 5 : 1;
+  C_t<T> v[5];
+#pragma unroll
+  for (int t = 0; t < 5; t++)
+    if (t < nr) v[t] = cadd<T>(u[sl[t]], x[rb_index<T>(tl, g.nl, l, r0 + t)]);
+#pragma unroll
+  for (int t = 0; t < 5; t++)
+    if (t < nr) u[sl[t]] = v[t];
 }
 // ---------------------------------------------------------------- launches
 // block shapes of the two-ended substitution with 32-line tiles: lines per
@@ -1455,11 +1461,14 @@ static void line_sweep_fac_d(const LevelView<T>& L, int color, const T* fac, con
   if (!rows) {
     if constexpr (std::is_same<T, double>::value) {
       if (coef) {
-        launch_dep(k_line_rhs<T, D, true>, gr, rt, 0, st, L, pa, pb, dv, tl, rb, coef);
+        launch_dep(k_line_rhs<T, D, true, false>, gr, rt, 0, st, L, pa, pb, dv, tl, rb, coef);
         rows = true;
       }
     }
-    if (!rows) launch_dep(k_line_rhs<T, D, false>, gr, rt, 0, st, L, pa, pb, dv, tl, rb, nullptr);
+    if (!rows && depends(gr))
+      launch_dep(k_line_rhs<T, D, false, false>, gr, rt, 0, st, L, pa, pb, dv, tl, rb, nullptr);
+    else if (!rows)
+      k_line_rhs<T, D, false, true><<<gr, rt, 0, st>>>(L, pa, pb, dv, tl, rb, nullptr);
   }
   if constexpr (std::is_same<T, float>::value) {
     const EndsArgs a{&L, grp, nl, tl, line_factor_elems(L.n, D, color, fmt, tile), fac, rb, pa, pb,
@@ -1483,7 +1492,9 @@ static void line_sweep_fac_d(const LevelView<T>& L, int color, const T* fac, con
                  L.active, grp, nl, m, fac, rb);
     } else {
       dim3 g2((unsigned)((nl + kSolveThreads - 1) / kSolveThreads), L.nrhs);
-      launch_dep(k_line_subst<T>, g2, kSolveThreads, 0, st, L.active, grp, nl, m, fac, rb);
+      // not beside the kernel before, whose carveout leaves room for few of
+      // its blocks (four shots at 128^3, three cycles: 321 -> 222 ms)
+      k_line_subst<T><<<g2, kSolveThreads, 0, st>>>(L.active, grp, nl, m, fac, rb);
     }
     apply_rb<T, D>(L, pa, pb, dv, tl, rb, st);
   }
