@@ -596,8 +596,8 @@ def main():
             # second: what the kernels achieve against the memory system
             "traffic_GBps": round(traffic / (ms * 1e-3) / 1e9, 1) if traffic else None,
             "traffic_frac": round(traffic / (ms * 1e-3) / 1e9 / peak, 4) if traffic else None,
-            "kernel": "level-0 line sweep along x, 4 colours x (k_line_rhs, k_line_subst, "
-                      "k_line_apply_rb)<float> with stored line factors, 25 RHS",
+            "kernel": "level-0 line sweep along x, 4 colours x (k_line_rows, "
+                      "k_line_ends) with stored line factors, 25 RHS",
             "ms_per_sweep": round(ms, 4), "ms_per_sweep_xyz": ms_dir, "launches_per_sweep": nl,
             "algorithmic_bytes_per_launch": by / nl, "peak_kind": peak_kind}
     solver.close()
