@@ -710,7 +710,7 @@ def main():
                        "cycle": CYCLE, "parallelism": f"replicas x{world}",
                        "l2": "inputs larger than L2 (25 x 128^3 systems, ~12 GB)",
                        "sweep_shapes": {"xyz": [list(v) for v in shapes],
-                                        "fields": "substitution lines/block, ring rows, "
+                                        "fields": "substitution lines/block, ring groups, "
                                                   "rhs threads/block (set-up autotuner)"}},
             "cycles_mean": float(np.mean(cycles)), "refinements_mean": float(np.mean(refs)),
             "max_rel_residual": float(max(rels)), "all_converged": ok,

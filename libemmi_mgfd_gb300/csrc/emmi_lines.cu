@@ -1465,6 +1465,7 @@ static void line_sweep_fac_d(const LevelView<T>& L, int color, const T* fac, con
         rows = true;
       }
     }
+    // a grid too large to be launched dependent reads u by read-only loads
     if (!rows && depends(gr))
       launch_dep(k_line_rhs<T, D, false, false>, gr, rt, 0, st, L, pa, pb, dv, tl, rb, nullptr);
     else if (!rows)
