@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "emmi_device_once.h"
+
 namespace emmi {
 
 // ---------------------------------------------------------------- complex
@@ -86,6 +88,24 @@ inline FastDiv make_fastdiv(unsigned d) {
 }
 __device__ __forceinline__ unsigned fdiv(unsigned u, const FastDiv& f) {
   return (__umulhi(u, f.m) + u) >> f.l;
+}
+
+// f() once for the calling thread's current device
+template <typename F> inline void once_on_device(DeviceOnce& once, F&& f) {
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess) dev = -1;
+  device_once(once, dev, f);
+}
+
+// address of a __device__ variable on the calling thread's current device; p
+// and dev: the caller's last answer and the device it was for
+template <typename T> inline T* symbol_on_device(T& symbol, T*& p, int& dev) {
+  int now = -1;
+  if (cudaGetDevice(&now) != cudaSuccess || now != dev || !p) {
+    cudaGetSymbolAddress((void**)&p, symbol);
+    dev = now;
+  }
+  return p;
 }
 
 // ---------------------------------------------------------------- dependent launches

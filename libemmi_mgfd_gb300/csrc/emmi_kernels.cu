@@ -19,7 +19,6 @@
 #include "emmi_node.cuh"
 
 #include <cstdio>
-#include <mutex>
 #include <type_traits>
 
 namespace emmi {
@@ -638,8 +637,8 @@ static void line_sweep_d(const LevelView<T>& L, int color, T* buf, cudaStream_t 
 // the line solve keeps a cp.async ring in shared memory: ask for the
 // largest shared-memory carveout so 12 blocks fit on an SM
 void init_line_kernels() {
-  static std::once_flag once;
-  std::call_once(once, [] {
+  static DeviceOnce once;
+  once_on_device(once, [] {
     cudaFuncSetAttribute(k_line_solve<float>, cudaFuncAttributePreferredSharedMemoryCarveout,
                          cudaSharedmemCarveoutMaxShared);
     cudaFuncSetAttribute(k_line_solve<double>, cudaFuncAttributePreferredSharedMemoryCarveout,

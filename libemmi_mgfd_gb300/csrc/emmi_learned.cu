@@ -34,7 +34,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
-#include <mutex>
 #include <type_traits>
 #include <vector>
 
@@ -692,16 +691,16 @@ ConvArgs conv_args(const int n[3], const int* mask, int nb) {
 __device__ int g_ls_err = 0;
 
 int* conv_err() {
-  static int* p = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    cudaGetSymbolAddress((void**)&p, g_ls_err);
+  static DeviceOnce once;
+  once_on_device(once, [] {
     const int lim = kConvSmemMax;
     cudaFuncSetAttribute(k_ls_conv<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
     cudaFuncSetAttribute(k_ls_conv<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
     cudaFuncSetAttribute(k_ls_conv<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   });
-  return p;
+  static thread_local int* p = nullptr;
+  static thread_local int of = -1;
+  return symbol_on_device(g_ls_err, p, of);
 }
 
 template <int MODE>

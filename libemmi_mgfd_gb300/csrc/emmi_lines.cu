@@ -23,7 +23,6 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
-#include <mutex>
 #include <type_traits>
 
 #include "emmi_line.cuh"
@@ -1365,10 +1364,10 @@ template <int FMT, int TW, int NG, int D, bool ROWS = false>
 static void ends_launch(const EndsArgs& a, int tpc, cudaStream_t st) {
   const int G = a.tl.mid / 5, slots = NG && NG < G ? NG : G;
   const unsigned tb = ends_smem<FMT>(TW, slots);
-  static std::once_flag once;
-  std::call_once(once, [] {
-    cudaFuncSetAttribute(k_line_ends<FMT, TW, NG, D, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         227 << 10);
+  static DeviceOnce once;
+  once_on_device(once, [] {
+    cudaFuncSetAttribute(k_line_ends<FMT, TW, NG, D, ROWS>,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize, 227 << 10);
   });
   const long tiles = (a.nl + TW - 1) / TW;
   if (D == 0 || ROWS) tpc = 1;

@@ -2,7 +2,6 @@
 // every level's without semi-coarsening.  8 colours of patches of the six
 // edges at a node, each patch solved with the current residual of its rows.
 #include <algorithm>
-#include <mutex>
 
 #include "emmi_line.cuh"
 
@@ -396,8 +395,8 @@ void launch_point_setup(const LevelView<T>& ops, T* coef, const LevelView<T>& gr
 template <typename T>
 void launch_point_coarse(const LevelView<T>& L, const T* coef, const C_t<T>* pf, const int* grp,
                          int nrep, unsigned rev, bool zero, cudaStream_t st) {
-  static std::once_flag once;
-  std::call_once(once, [] {
+  static DeviceOnce once;
+  once_on_device(once, [] {
     cudaFuncSetAttribute(k_point_coarse<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          kPointSmem);
   });

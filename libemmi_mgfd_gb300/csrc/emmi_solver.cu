@@ -248,11 +248,11 @@ inline unsigned blocks_for(long n, int bs = 256, long cap = 65535) {
 // device) so that destroying and creating solvers does not map and unmap
 // device memory each time.  emmi_trim_memory gives it back.
 static void keep_pool_memory() {
-  static std::once_flag once[64];
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
-  std::call_once(once[dev], [dev] {
+  static DeviceOnce once;
+  once_on_device(once, [] {
+    int dev = 0;
     cudaMemPool_t pool;
+    if (cudaGetDevice(&dev) != cudaSuccess) return;
     if (cudaDeviceGetDefaultMemPool(&pool, dev) != cudaSuccess) return;
     uint64_t thr = UINT64_MAX;
     cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
@@ -559,7 +559,15 @@ int emmi_solver::build_graphs() {
       } else {
         emit_cycle<T>(h, 0, opt.cycleopt, part, cur);
       }
-      CK(cudaStreamEndCapture(st, &g));
+      const cudaError_t refused = cudaGetLastError();
+      const cudaError_t ended = cudaStreamEndCapture(st, &g);
+      if (refused != cudaSuccess || ended != cudaSuccess) {
+        if (ended == cudaSuccess) cudaGraphDestroy(g);
+        cudaGetLastError();  // not left for the thread's next call
+        set_err("a launch of the cycle was refused: %s",
+                cudaGetErrorString(refused != cudaSuccess ? refused : ended));
+        return EMMI_ECUDA;
+      }
       size_t nn = 0;
       cudaGraphGetNodes(g, nullptr, &nn);
       (part ? nodesB : nodesA)[h] = launch_counter - before;

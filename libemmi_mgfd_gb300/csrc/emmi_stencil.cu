@@ -360,10 +360,9 @@ bool flat_map(CUtensorMap* m, const void* base, long elems, int esize, int box_r
 }  // namespace
 
 int* stencil_err() {
-  static int* p = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] { cudaGetSymbolAddress((void**)&p, g_stencil_err); });
-  return p;
+  static thread_local int* p = nullptr;
+  static thread_local int of = -1;
+  return symbol_on_device(g_stencil_err, p, of);
 }
 
 void stencil_hook(StencilPlan* P, long long wait, int stall) {
@@ -434,8 +433,8 @@ bool stencil_prepare(const LevelView<float>& V, long u_elems, long cell_elems, S
 template <typename TO, int W>
 static void staged_launch(const LevelView<float>& L, const StencilPlan& P, C_t<TO>* rout,
                           double* norm2, cudaStream_t st) {
-  static std::once_flag once;
-  std::call_once(once, [] {
+  static DeviceOnce once;
+  once_on_device(once, [] {
     cudaFuncSetAttribute(k_residual_staged<TO, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          210 * 1024);
   });
