@@ -517,25 +517,34 @@ struct FacBlocks {
   long off[4], gstride[4];
 };
 
-// Factors of every line of colour blockIdx.z for group blockIdx.y of operators
-// and frequencies.  A line's rows are a chain of some 40 dependent operations
-// each and a colour has few lines (1024 at 64^3: 32 blocks), so that the chain
-// is the launch's time: the colours, which do not depend on one another, share
-// a launch (all of 64^3's: 4.5 -> 1.5 ms).  A warp per end of 32 lines, each thread assembling its rows in
-// registers (band_row) and eliminating them.  The mirrored end hands its
+// Factors of every line of a direction's four colours, for group blockIdx.y of
+// operators and frequencies.  A thread per end of a line, each assembling its
+// rows in registers (band_row) and eliminating them; the mirrored end hands its
 // Schur complement of the middle rows to the other through shared memory.
+// What bounds it is the latency of the cells' loads and of the elimination, 16
+// warps an SM: the colours read the same cells, so that the four of a block of
+// 64 lines are neighbouring blocks (set-up's line factors of 25 operators at
+// 128^3 29.8 ms with one colour after the other, 19.6 so; 75 groups 61.5 and
+// 54.4).  A line's rows are a chain of some 40 dependent operations each and a
+// colour has few lines (1024 at 64^3), so that the chain is the launch's time:
+// all of 64^3's one colour a launch 4.5 ms, in one launch a direction 1.0.
+// SERIAL: a thread eliminates both ends of its line, the mirrored one first,
+// for launches whose lines fill the device several times over (serial_factors);
+// the same operations, so the same factors.
 // An fp16 L value outside its range (or not finite) sets *ovf.
-template <int D, int FMT>
-__global__ void __launch_bounds__(64) k_line_factor_ends(LevelView<float> L, LineTile tl,
-                                                         FacBlocks fb, float* __restrict__ fac,
-                                                         int* __restrict__ ovf) {
+constexpr int kFacLines = 64;  // lines of a block
+template <int D, int FMT, bool SERIAL>
+__global__ void __launch_bounds__(SERIAL ? kFacLines : 2 * kFacLines)
+    k_line_factor_ends(LevelView<float> L, LineTile tl, FacBlocks fb, float* __restrict__ fac,
+                       int* __restrict__ ovf) {
   constexpr int A = (D == 0) ? 1 : 0, B = (D == 2) ? 1 : 2;
-  __shared__ float2 schur[15][32];
-  const int grp = blockIdx.y, color = blockIdx.z;
+  __shared__ float2 schur[15][kFacLines];
+  const int grp = blockIdx.y, color = blockIdx.x & 3;
   const LineGeom g = line_geom<D>(L.n, color & 1, color >> 1);
-  const int lane = threadIdx.x & 31;
-  const long l0 = blockIdx.x * 32L + lane;
-  if (blockIdx.x * 32L >= g.nl) return;  // a colour with fewer lines
+  const int lane = threadIdx.x & (kFacLines - 1);
+  const bool bottom = SERIAL || threadIdx.x >= kFacLines, top = SERIAL || threadIdx.x < kFacLines;
+  const long first = (long)(blockIdx.x >> 2) * kFacLines, l0 = first + lane;
+  if (first >= g.nl) return;  // a colour with fewer lines
   const bool live = l0 < g.nl;
   const long l = live ? l0 : g.nl - 1;
   const unsigned lq = (unsigned)l / (unsigned)g.la;
@@ -548,13 +557,13 @@ __global__ void __launch_bounds__(64) k_line_factor_ends(LevelView<float> L, Lin
                        (l >> tl.shift) * g.m * kFacRow<FMT> * TW;
   bool over = false;
   float2 W[21], lq5[6];
-#pragma unroll
-  for (int i = 0; i < 21; i++) W[i] = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int i = 0; i < 5; i++) W[WI(i, i)] = make_float2(1.f, 0.f);  // dummy leading rows
   auto run = [&](auto mir) {
     constexpr bool MIR = decltype(mir)::value;
     float2 y5;
+#pragma unroll
+    for (int i = 0; i < 21; i++) W[i] = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < 5; i++) W[WI(i, i)] = make_float2(1.f, 0.f);  // dummy leading rows
     eliminate_end<MIR>(
         G, nd, W, y5,
         [&](auto tt, int s, int k, float2 (&w)[6], float2& r) {
@@ -574,15 +583,14 @@ __global__ void __launch_bounds__(64) k_line_factor_ends(LevelView<float> L, Lin
                          lq5, id, over);
         });
   };
-  if (threadIdx.x >= 32) {
+  if (bottom) {
     run(std::true_type());
 #pragma unroll
     for (int i = 0; i < 15; i++) schur[i][lane] = W[i];
-  } else {
-    run(std::false_type());
   }
-  __syncthreads();
-  if (threadIdx.x < 32) {
+  if (top) run(std::false_type());
+  if constexpr (!SERIAL) __syncthreads();
+  if (top) {
     // the middle rows: window 0..4 of this end, row 5 = E_d(G + 1) with its
     // own entries, and the mirrored end's complement of rows 5 - i
     float band[5];
@@ -1500,6 +1508,13 @@ static void line_sweep_fac_d(const LevelView<T>& L, int color, const T* fac, con
   }
 }
 
+// a line a thread where that alone is four waves of 512 threads an SM (75
+// groups at 128^3: 52.1 ms, 54.4 with a thread an end; 25: 18.8 and 19.6), an
+// end a thread below (20 at 96^3: 7.3 and 7.1 ms; one at 64^3: 1.44 and 1.02)
+static bool serial_factors(long lines, int groups) {
+  return 4 * lines * groups >= 4L * kSMs * 512;
+}
+
 template <typename T, int D>
 static void line_factor_d(const LevelView<T>& L, T* fac, const long off[4], int fmt, int tile,
                           int* ovf, cudaStream_t st) {
@@ -1513,11 +1528,13 @@ static void line_factor_d(const LevelView<T>& L, T* fac, const long off[4], int 
   if (most == 0) return;
   if constexpr (std::is_same<T, float>::value) {
     const LineTile tl = line_tile(L.n[D], tile);
-    dim3 g((unsigned)((most + 31) / 32), L.nrhs, 4);
-    if (fmt == kFacF16)
-      k_line_factor_ends<D, kFacF16><<<g, 64, 0, st>>>(L, tl, fb, fac, ovf);
-    else
-      k_line_factor_ends<D, kFacF32><<<g, 64, 0, st>>>(L, tl, fb, fac, ovf);
+    const dim3 g(4 * (unsigned)((most + kFacLines - 1) / kFacLines), L.nrhs);
+    auto go = [&](auto k, int threads) { k<<<g, threads, 0, st>>>(L, tl, fb, fac, ovf); };
+    const bool serial = serial_factors(most, L.nrhs);
+    if (fmt == kFacF16 && serial) go(k_line_factor_ends<D, kFacF16, true>, kFacLines);
+    else if (fmt == kFacF16) go(k_line_factor_ends<D, kFacF16, false>, 2 * kFacLines);
+    else if (serial) go(k_line_factor_ends<D, kFacF32, true>, kFacLines);
+    else go(k_line_factor_ends<D, kFacF32, false>, 2 * kFacLines);
   } else {
     for (int c = 0; c < 4; c++) {
       const long nl = line_count(L.n, D, c);

@@ -44,3 +44,36 @@ def test_line_ends_match_the_sweeps_that_factor(n, nrhs, lf):
         s.close()
     for r in range(nrhs):
         assert rel_err(out[0][r], out[1][r]) < 1e-5, r
+
+
+@gpu
+@pytest.mark.parametrize("lf", [1, 2])
+def test_factors_of_many_groups_match_those_of_few(lf):
+    """Line factors of 1216 groups (frequencies) of a 16^3 operator, whose
+    level-0 lines are factored a line a thread, against solvers of one group,
+    an end a thread.  The factors are the same; the sweeps differ in tiles and
+    the residual's kernel, so two cycles differ by float rounding: 1e-5 of the
+    field's norm in H."""
+    n, nrhs = (16, 16, 16), 1216
+    rng = np.random.default_rng(29)
+    x = [np.concatenate([[0.0], np.cumsum(100.0 * 1.1 ** np.abs(np.arange(v) - v // 2))])
+         .astype(np.float32) for v in n]
+    raw = np.concatenate([10.0 ** rng.uniform(-1, 0.5, (3,) + n[::-1]),
+                          np.ones((1,) + n[::-1])]).astype(np.float32)
+    om = np.linspace(3.0, 12.0, nrhs).astype(np.float32)
+    unk = np.flatnonzero(unknown_mask(n).ravel())
+    b = np.zeros((nrhs, 3 * 17 ** 3), np.complex128)
+    for r in range(nrhs):
+        b[r, rng.choice(unk, 5, replace=False)] = rng.standard_normal(5)
+
+    def run(rows):
+        s = G.Solver(n, *x, raw[None], om[rows], op=np.zeros(len(rows), np.int32),
+                     options=G.Options(precision=G.PREC_MIXED, ncycle=2, tol=0.0, autotune=0,
+                                       sigma_floor=1e-3, line_factors=lf))
+        h = s.solve(b[rows])[1]
+        assert s.line_factor_format == {1: 0, 2: 1}[lf]
+        s.close()
+        return h
+    many = run(np.arange(nrhs))
+    for r in (0, 617, nrhs - 1):
+        assert rel_err(many[r], run(np.array([r]))[0]) < 1e-5, r
