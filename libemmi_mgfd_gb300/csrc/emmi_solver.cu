@@ -609,10 +609,19 @@ static int build_groups(emmi_solver* s) {
   return EMMI_OK;
 }
 
+// Whether bytes more may be stored to save recomputing them.  The line factors
+// come first and may take half of the memory that is free before them; what is
+// stored besides fills up that half at most, so that neither the factors nor
+// the program's other allocations find less room for it.
+static bool fits_stored(const emmi_solver* s, size_t bytes) {
+  const size_t kept = (s->fac_on ? s->fac_bytes : 0) + s->stored_bytes;
+  return kept + bytes <= (device_avail() + kept) / 2;
+}
+
 // Stored coefficients and patch factors of the coarsest level of every
 // hierarchy, for the node-patch sweeps (emmi_point.cu).  Left out (the sweeps
-// then factor their patches each time) when they would take more than a
-// quarter of the free device memory.
+// then factor their patches each time) when they do not fit (fits_stored: a
+// coarsest level is large where the mesh halves only a few times).
 template <typename T>
 static int build_point_data(emmi_solver* s) {
   const int l = s->lmax - 1;
@@ -621,7 +630,8 @@ static int build_point_data(emmi_solver* s) {
   for (int h = 0; h < nh; h++)
     bytes += (size_t)s->nop * point_coef_elems(s->hier[h][l].n) * sizeof(T) +
              (size_t)s->ngroups * point_factor_elems(s->hier[h][l].n) * sizeof(C_t<T>);
-  if (bytes > device_avail() / 4) return EMMI_OK;
+  if (!fits_stored(s, bytes)) return EMMI_OK;
+  s->stored_bytes += bytes;
   for (int h = 0; h < nh; h++) {
     const int* n = s->hier[h][l].n;
     int rc;
@@ -903,13 +913,14 @@ static int autotune_sweeps(emmi_solver* s) {
 // Stored FP64 coefficients of every level of the complex128 cycle: its row and
 // level residuals would spend most of their FP64 instructions on recomputing
 // them (eight divisions an edge), bit for bit the same.  240 bytes a slot and
-// operator, kept when they fit in half of the free device memory.
+// operator, kept when they fit (fits_stored).
 static int build_coef64_levels(emmi_solver* s) {
   size_t bytes = 0;
   for (int h = 0; h < 3; h++)
     for (int l = h ? 1 : 0; l < s->lmax; l++)
       bytes += (size_t)s->nop * coef64_elems(s->hier[h][l].n) * sizeof(double);
-  if (bytes > device_avail() / 2) return EMMI_OK;
+  if (!fits_stored(s, bytes)) return EMMI_OK;
+  s->stored_bytes += bytes;
   for (int h = 0; h < 3; h++)
     for (int l = 0; l < s->lmax; l++) {
       if (h && l == 0) {
@@ -939,6 +950,7 @@ static int build_coef64(emmi_solver* s) {
   if (bytes > device_avail() / 2) return EMMI_OK;
   int rc;
   if ((rc = s->alloc((void**)&s->d_coef64, bytes)) != EMMI_OK) return rc;
+  s->stored_bytes += bytes;
   CK(cudaMemsetAsync(s->d_coef64, 0, bytes, s->st));
   LevelView<double> V = s->view<double>(0, 0);
   V.nrhs = s->nop;
@@ -1347,10 +1359,7 @@ static int create_impl(emmi_solver** out, const emmi_problem* P, const emmi_opti
     for (int l = 1; l < kMaxLev; l++)
       for (int d = 0; d < 3; d++) s->shape[l][d].subst = 1;
     mark("field buffers");
-    if (s->opt.line_factors) {
-      TRY(mixed ? build_groups<float>(s) : build_groups<double>(s));
-      if (s->lmax > 1) TRY(mixed ? build_point_data<float>(s) : build_point_data<double>(s));
-    }
+    if (s->opt.line_factors) TRY(mixed ? build_groups<float>(s) : build_groups<double>(s));
     if (s->opt.line_factors && !s->opt.line_sweep)
       TRY(mixed ? build_line_factors<float>(s) : build_line_factors<double>(s));
     mark("line factors");
@@ -1376,6 +1385,9 @@ static int create_impl(emmi_solver** out, const emmi_problem* P, const emmi_opti
     if (mixed) TRY(build_coef64(s));
     else if (s->opt.line_factors) TRY(build_coef64_levels(s));
     mark("FP64 coefficients");
+    if (s->opt.line_factors && s->lmax > 1)
+      TRY(mixed ? build_point_data<float>(s) : build_point_data<double>(s));
+    mark("coarsest level");
   }
 
   // ---- graphs

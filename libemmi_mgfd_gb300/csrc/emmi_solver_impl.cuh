@@ -104,6 +104,9 @@ struct emmi_solver {
   long fac_off[3][emmi::kMaxLev][3][4];
   int fac_tile[3][emmi::kMaxLev][3];  // lines per tile of the complex64 blocks
 
+  // what is stored besides the line factors (coefficients, patch factors)
+  size_t stored_bytes = 0;
+
   // node-patch sweeps of the coarsest level (per hierarchy): coefficients per
   // operator and patch factors per group (working precision; null: factored in
   // every sweep), and whether a block's shared memory holds the level
