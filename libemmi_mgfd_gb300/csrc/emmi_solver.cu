@@ -750,8 +750,8 @@ static int build_line_factors(emmi_solver* s) {
 // ---- autotuning of the level-0 sweep shapes ------------------------------
 // The stored-factor line sweep of each direction is timed at set-up on this
 // solver's own level-0 operators (zero fields) for a few block shapes -- the
-// right-hand-side kernel's threads per block, then the fp16 substitution's
-// lines per block and ring depth -- and the fastest is kept when it beats
+// right-hand-side kernel's threads per block, then the complex64
+// substitution's lines per block and ring depth -- and the fastest is kept when it beats
 // the incumbent by more than 2 %.  No shape changes any result.  Choices are
 // cached for the process by (grid, RHS per launch, RHS, factor format,
 // direction), so later solvers of the same shape take them without timing.
@@ -763,7 +763,11 @@ static bool g_tune_loaded = false;
 // EMMI_TUNE_FILE when that is set: read once before the first tuning,
 // rewritten whole after every new entry.  Each entry lists, in this order,
 // grid (3), chunk, nrhs, fmt, dir, subst, rhs_threads; entries that do not
-// read as nine integers are skipped.  Call with g_tune_mu held.
+// read as nine integers are skipped.  A shape is a number in a table of the
+// kernels' shapes: a file of another kTuneVersion (or none) is of other
+// kernels, so its entries are not taken and the shapes are timed anew.  Call
+// with g_tune_mu held.
+constexpr long kTuneVersion = 2;
 static void tune_file_load() {
   g_tune_loaded = true;
   const char* path = std::getenv("EMMI_TUNE_FILE");
@@ -775,6 +779,11 @@ static void tune_file_load() {
   size_t k;
   while ((k = std::fread(buf, 1, sizeof(buf), fp)) > 0) text.append(buf, k);
   std::fclose(fp);
+  const char* tag = "\"version\":";
+  const size_t ver = text.find(tag);
+  if (ver == std::string::npos ||
+      std::strtol(text.c_str() + ver + std::strlen(tag), nullptr, 10) != kTuneVersion)
+    return;
   size_t pos = text.find("\"sweep_shapes\"");
   while (pos != std::string::npos) {
     const size_t a = text.find('{', pos + 1), b = a == std::string::npos ? a : text.find('}', a);
@@ -807,7 +816,7 @@ static void tune_file_save() {
   const std::string tmp = std::string(path) + ".tmp";
   FILE* fp = std::fopen(tmp.c_str(), "w");
   if (!fp) return;
-  std::fprintf(fp, "{\"sweep_shapes\": [");
+  std::fprintf(fp, "{\"version\": %ld, \"sweep_shapes\": [", kTuneVersion);
   bool first = true;
   for (const auto& kv : g_tune) {
     const auto& q = kv.first;
