@@ -55,3 +55,29 @@ def test_complex64_stored_patches_equal_the_factoring_ones(n, nrhs, more):
     a = _solve(n, nrhs, G.PREC_MIXED, line_factors=1, **more)[1]
     b = _solve(n, nrhs, G.PREC_MIXED, line_factors=0, **more)[1]
     assert np.abs(a - b).max() <= 1e-5 * np.abs(b).max()
+
+
+# 16^3: a launch of 160 right-hand sides has 10240 lines, past the 7680 up to
+# which a line takes 12 lanes; (20, 12, 16): its level 0 alone
+@gpu
+@pytest.mark.parametrize("n", [(16, 16, 16), (20, 12, 16)])
+def test_fp64_lanes_give_the_bits_of_a_thread_a_line(n):
+    """One right-hand side alone (12 lanes a line) and 160 copies of it (a
+    thread a line), stored factors both: equal E and H."""
+    rng = np.random.default_rng(53)
+    x = [np.concatenate([[0.0], np.cumsum(100.0 * 1.1 ** np.abs(np.arange(v) - v // 2))])
+         .astype(np.float32) for v in n]
+    raw = np.concatenate([10.0 ** rng.uniform(-1, 0.5, (3,) + n[::-1]),
+                          np.ones((1,) + n[::-1])]).astype(np.float32)
+    b = np.zeros((1, 3 * (n[0] + 1) * (n[1] + 1) * (n[2] + 1)), np.complex128)
+    b[0, rng.choice(np.flatnonzero(unknown_mask(n).ravel()), 5, replace=False)] = 1.0
+    out = []
+    for k in (1, 160):
+        s = G.Solver(n, *x, raw[None], np.full(k, 6.28, np.float32), op=np.zeros(k, np.int32),
+                     options=G.Options(precision=G.PREC_FP64, ncycle=3, tol=0.0))
+        out.append(s.solve(np.repeat(b, k, 0))[:2])
+        s.close()
+    for one, many in zip(*out):
+        assert np.abs(one).max() > 0
+        for r in (0, 77, 159):
+            assert np.array_equal(one[0], many[r])

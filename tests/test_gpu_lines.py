@@ -77,3 +77,33 @@ def test_factors_of_many_groups_match_those_of_few(lf):
     many = run(np.arange(nrhs))
     for r in (0, 617, nrhs - 1):
         assert rel_err(many[r], run(np.array([r]))[0]) < 1e-5, r
+
+
+@gpu
+def test_shapes_of_wide_tiles_never_change_the_result():
+    """Every forced sweep shape on a batch whose level 0 works in tiles of 32
+    lines, with rings shorter than the x and y lines (23 groups an end) and
+    longer than the z lines (7): the defaults' iterates bit for bit."""
+    n, nrhs = (48, 48, 16), 25
+    rng = np.random.default_rng(47)
+    x = [np.concatenate([[0.0], np.cumsum(100.0 * 1.1 ** np.abs(np.arange(v) - v // 2))])
+         .astype(np.float32) for v in n]
+    raw = np.concatenate([10.0 ** rng.uniform(-1, 0.5, (3,) + n[::-1]),
+                          np.ones((1,) + n[::-1])]).astype(np.float32)
+    S = (n[0] + 1) * (n[1] + 1) * (n[2] + 1)
+    unk = np.flatnonzero(unknown_mask(n).ravel())
+    b = np.zeros((nrhs, 3 * S), np.complex128)
+    for r in range(nrhs):
+        b[r, rng.choice(unk, 5, replace=False)] = rng.standard_normal(5)
+
+    def run(autotune):
+        s = G.Solver(n, *x, raw[None], np.full(nrhs, 6.28, np.float32), op=np.zeros(nrhs, np.int32),
+                     options=G.Options(precision=G.PREC_MIXED, ncycle=3, tol=0.0,
+                                       autotune=autotune))
+        e, h, _ = s.solve(b)
+        s.close()
+        return e, h
+    e0, h0 = run(0)
+    for k in range(1, 11):
+        e, h = run(-k)
+        assert np.array_equal(e, e0) and np.array_equal(h, h0), k
