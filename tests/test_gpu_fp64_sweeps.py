@@ -58,7 +58,8 @@ def test_complex64_stored_patches_equal_the_factoring_ones(n, nrhs, more):
 
 
 # 16^3: a launch of 160 right-hand sides has 10240 lines, past the 7680 up to
-# which a line takes 12 lanes; (20, 12, 16): its level 0 alone
+# which a line takes 12 lanes; (20, 12, 16): the x lines just reach them, the y
+# and z lines pass them
 @gpu
 @pytest.mark.parametrize("n", [(16, 16, 16), (20, 12, 16)])
 def test_fp64_lanes_give_the_bits_of_a_thread_a_line(n):
