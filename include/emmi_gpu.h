@@ -72,30 +72,33 @@ typedef struct {
   int krylov;       /* MIXED: 0 = stationary FP64 refinement of complex64
                        cycles; k > 0 = FP64 FGMRES(k) (k <= 12) with one
                        complex64 cycle as its preconditioner (0)           */
-  int line_factors; /* MIXED: factor every line once per (operator,
-                       frequency) at set-up and keep the factors, when they
-                       fit in half the free device memory: 2 = L in fp16,
-                       1/d in fp32 (fp32 throughout if an L value leaves
-                       the fp16 range), 1 = fp32; 0 = factor in every
-                       sweep (2)                                           */
+  int line_factors; /* factor every line once per (operator, frequency) at
+                       set-up and keep the factors, when they fit in half
+                       the free device memory.  MIXED: 2 = L in fp16, 1/d in
+                       fp32 (fp32 throughout if an L value leaves the fp16
+                       range), 1 = fp32; FP64: 1 or 2 = in FP64.  Where the
+                       rest of that half has room, also the coarsest level's
+                       patch factors and, FP64, the coefficients of every
+                       level (240 bytes per slot and operator; with
+                       line_sweep = 1 too).  0 = factor and recompute in
+                       every sweep (2)                                     */
   int autotune;     /* MIXED with stored fp16 factors: time the level-0
                        line sweep of each direction at set-up for a few
                        block shapes and keep the fastest; cached for the
                        process per (grid, RHS, direction); no shape changes
                        any result (1); 0 = default shapes; -k (k = 1..10)
                        forces shape k in every direction (checks)          */
-  int line_sweep;   /* 1 = one launch per colour: each thread assembles,
-                       factors and solves one line, keeping the multipliers
-                       only between its two substitutions (fp16 when
-                       line_factors = 2, else working precision); no stored
-                       factors.  0 = three launches per colour (residual
-                       rows, substitution, update) with the stored factors
-                       of line_factors (default)                          */
-  int fused_level;  /* with line_sweep = 0: levels l >= fused_level use the
-                       one-launch sweep (their data sit in L2 and their
-                       launches are short); levels above it the three-launch
-                       sweep.  A value >= the number of levels keeps the
-                       three-launch sweep everywhere                      */
+  int line_sweep;   /* 1 = one launch per colour: a line is assembled,
+                       factored and solved by one thread (complex64: two,
+                       from its ends), keeping the multipliers only between
+                       its two substitutions (fp16 when line_factors = 2,
+                       else working precision); no stored line factors.
+                       0 = residual rows, substitution and update with the
+                       stored factors of line_factors, in one to three
+                       launches per colour (default)                      */
+  int fused_level;  /* with line_sweep = 0: levels l >= fused_level are swept
+                       as with line_sweep = 1 and keep no line factors; a
+                       value >= the number of levels: none                */
   int staged;       /* MIXED: 1 = the complex64 residual of level 0 stages
                        each plane's halo in shared memory with tensor copies
                        where the batch is small (default; large batches take

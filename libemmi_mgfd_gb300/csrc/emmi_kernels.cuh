@@ -41,10 +41,11 @@ long line_scratch_elems(const int n[3], int d, int nrhs);
 // bytes a row; line_factor_elems values of T per group.  launch_line_factor
 // fills them for the L.nrhs groups of L (L.op / L.wmu per group, u and f
 // unused) and the four colours of direction d, the band rows assembled in
-// registers, into fac + off[color] + g * line_factor_elems and sets *ovf when an L value does not fit fp16 (kFacF16);
-// launch_line_sweep_fac then sweeps RHS r with the factors of group grp[r], rb
-// holding line_rb_elems complex values per RHS, in line_fac_launches launches;
-// coef (complex128, may be null): launch_coef64's coefficients of the level
+// registers, into fac + off[color] + g * line_factor_elems and sets *ovf when
+// an L value does not fit fp16 (kFacF16); launch_line_sweep_fac then sweeps
+// RHS r with the factors of group grp[r], rb holding line_rb_elems complex
+// values per RHS, in line_fac_launches launches; coef (complex128, may be
+// null): launch_coef64's coefficients of the level
 constexpr int kFacF32 = 0, kFacF16 = 1;
 int line_tile_width(const int n[3], int d, int nrhs, int fmt);
 long line_factor_elems(const int n[3], int d, int color, int fmt, int tile);

@@ -708,8 +708,9 @@ void launch_conv(const ConvArgs& a, int nb, const uint32_t* in, const uint4* Wt,
                  float2* out, cudaStream_t st) {
   int* err = conv_err();
   dim3 g((unsigned)(a.ncol * a.nchunk), nb);
-  k_ls_conv<MODE><<<g, kTcThreads, std::max<size_t>(conv_smem(a), kConvSmemMin), st>>>(a, reinterpret_cast<const uint4*>(in), Wt,
-                                                reinterpret_cast<uint4*>(hid), out, err);
+  const size_t smem = std::max<size_t>(conv_smem(a), kConvSmemMin);
+  k_ls_conv<MODE><<<g, kTcThreads, smem, st>>>(a, reinterpret_cast<const uint4*>(in), Wt,
+                                               reinterpret_cast<uint4*>(hid), out, err);
 }
 
 }  // namespace

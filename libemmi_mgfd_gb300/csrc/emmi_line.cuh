@@ -66,11 +66,6 @@ __device__ __forceinline__ void rec_put(typename Vec16<T>::V* p, long ps, const 
 #pragma unroll
   for (int q = 0; q < kPlanes<T>; q++) p[q * ps] = pack16(v + q * kLanes<T>);
 }
-template <typename T>
-__device__ __forceinline__ void rec_get(const typename Vec16<T>::V* p, long ps, T (&v)[kRec]) {
-#pragma unroll
-  for (int q = 0; q < kPlanes<T>; q++) unpack16(p[q * ps], v + q * kLanes<T>);
-}
 // values [10,11] (z or x) live in the last plane for both types
 template <typename T>
 __device__ __forceinline__ C_t<T> rec_get_x(const typename Vec16<T>::V* p, long ps) {

@@ -26,6 +26,7 @@
 #include <type_traits>
 
 #include "emmi_line.cuh"
+#include "emmi_node.cuh"
 
 namespace emmi {
 
@@ -277,37 +278,24 @@ __device__ __forceinline__ void node_rows(const LevelView<float>& L, int rhs, in
               rA1 = qdiv(1.f, A1), rB0 = qdiv(1.f, B0), rB1 = qdiv(1.f, B1);
   const float hd = 0.5f * (D0 + D1), ha = 0.5f * (A0 + A1), hb = 0.5f * (B0 + B1);
   const float qw = 0.25f * wmu;
-  // f - A e of an edge: acc holds the curl-curl part, sig the sum of the
-  // four conductivities around it
-  auto done = [&](float2 ff, float2 acc, float2 e, float sig) {
-    const float m = qw * sig;  // the mass term is -i m e
-    return make_float2(ff.x - acc.x - m * e.y, ff.y - acc.y + m * e.x);
-  };
-  auto pair = [&](float2 acc, float2 e, float2 ep, float2 em, float k, float rp, float rm,
-                  float h, float2 x1, float2 x0, float2 x1m, float2 x0m) {
-    const float kp = k * rp, km = k * rm;
-    acc.x += (kp * (e.x - ep.x) + km * (e.x - em.x)) + h * ((x1.x - x0.x) - (x1m.x - x0m.x));
-    acc.y += (kp * (e.y - ep.y) + km * (e.y - em.y)) + h * ((x1.y - x0.y) - (x1m.y - x0m.y));
-    return acc;
-  };
   {
-    float2 c = pair(zero, d0, d0ap, d0am, D0 * hb, rA1, rA0, hb, ap, ap_dm, am, am_dm);
-    c = pair(c, d0, d0bp, d0bm, D0 * ha, rB1, rB0, ha, bp, bp_dm, bm, bm_dm);
-    r[0] = done(f0, c, d0, ((sg0 + sg1) + sg2) + sg3);
+    float2 c = edge_pair(zero, d0, d0ap, d0am, D0 * hb, rA1, rA0, hb, ap, ap_dm, am, am_dm);
+    c = edge_pair(c, d0, d0bp, d0bm, D0 * ha, rB1, rB0, ha, bp, bp_dm, bm, bm_dm);
+    r[0] = edge_done(f0, c, d0, qw * (((sg0 + sg1) + sg2) + sg3));
   }
   if (node) {
-    float2 c = pair(zero, am, am_dp, am_dm, A0 * hb, rD1, rD0, hb, d1, d1am, d0, d0am);
-    c = pair(c, am, am_bp, am_bm, A0 * hd, rB1, rB0, hd, bp, bp_am, bm, bm_am);
-    r[1] = done(f1, c, am, sa0);
-    c = pair(zero, ap, ap_dp, ap_dm, A1 * hb, rD1, rD0, hb, d1ap, d1, d0ap, d0);
-    c = pair(c, ap, ap_bp, ap_bm, A1 * hd, rB1, rB0, hd, bp_ap, bp, bm_ap, bm);
-    r[2] = done(f2, c, ap, sa1);
-    c = pair(zero, bm, bm_dp, bm_dm, B0 * ha, rD1, rD0, ha, d1, d1bm, d0, d0bm);
-    c = pair(c, bm, bm_ap, bm_am, B0 * hd, rA1, rA0, hd, ap, ap_bm, am, am_bm);
-    r[3] = done(f3, c, bm, sb0);
-    c = pair(zero, bp, bp_dp, bp_dm, B1 * ha, rD1, rD0, ha, d1bp, d1, d0bp, d0);
-    c = pair(c, bp, bp_ap, bp_am, B1 * hd, rA1, rA0, hd, ap_bp, ap, am_bp, am);
-    r[4] = done(f4, c, bp, sb1);
+    float2 c = edge_pair(zero, am, am_dp, am_dm, A0 * hb, rD1, rD0, hb, d1, d1am, d0, d0am);
+    c = edge_pair(c, am, am_bp, am_bm, A0 * hd, rB1, rB0, hd, bp, bp_am, bm, bm_am);
+    r[1] = edge_done(f1, c, am, qw * sa0);
+    c = edge_pair(zero, ap, ap_dp, ap_dm, A1 * hb, rD1, rD0, hb, d1ap, d1, d0ap, d0);
+    c = edge_pair(c, ap, ap_bp, ap_bm, A1 * hd, rB1, rB0, hd, bp_ap, bp, bm_ap, bm);
+    r[2] = edge_done(f2, c, ap, qw * sa1);
+    c = edge_pair(zero, bm, bm_dp, bm_dm, B0 * ha, rD1, rD0, ha, d1, d1bm, d0, d0bm);
+    c = edge_pair(c, bm, bm_ap, bm_am, B0 * hd, rA1, rA0, hd, ap, ap_bm, am, am_bm);
+    r[3] = edge_done(f3, c, bm, qw * sb0);
+    c = edge_pair(zero, bp, bp_dp, bp_dm, B1 * ha, rD1, rD0, ha, d1bp, d1, d0bp, d0);
+    c = edge_pair(c, bp, bp_ap, bp_am, B1 * hd, rA1, rA0, hd, ap_bp, ap, am_bp, am);
+    r[4] = edge_done(f4, c, bp, qw * sb1);
   }
 }
 
@@ -1380,7 +1368,9 @@ static void ends_launch(const EndsArgs& a, int tpc, cudaStream_t st) {
   const long tiles = (a.nl + TW - 1) / TW;
   if (D == 0 || ROWS) tpc = 1;
   dim3 g((unsigned)((tiles + tpc - 1) / tpc), a.L->nrhs);
-  launch_dep(k_line_ends<FMT, TW, NG, D, ROWS>, g, D == 0 || ROWS ? kXThreads : 2 * TW * tpc, tpc * tb, st, a.L->active, a.grp, a.nl, a.tl, a.gstride, a.fac, a.rb, *a.L, a.pa, a.pb, a.dv, slots, tb);
+  launch_dep(k_line_ends<FMT, TW, NG, D, ROWS>, g, D == 0 || ROWS ? kXThreads : 2 * TW * tpc,
+             tpc * tb, st, a.L->active, a.grp, a.nl, a.tl, a.gstride, a.fac, a.rb, *a.L, a.pa, a.pb,
+             a.dv, slots, tb);
 }
 
 // the ring of a launch: NG of the shape, one NG for the fp32 format
@@ -1419,7 +1409,7 @@ static void ends_dispatch(const EndsArgs& a, SweepShape sh, bool rows, cudaStrea
       case 4: ends_launch<FMT, 32, 4, D>(a, lines / 32, st); break;
       case 5: ends_launch<FMT, 32, 5, D>(a, 1, st); break;
       case 8: ends_launch<FMT, 32, 8, D>(a, 1, st); break;
-        default: ends_launch<FMT, 32, 6, D>(a, lines / 32, st); break;
+      default: ends_launch<FMT, 32, 6, D>(a, lines / 32, st); break;
     }
   }
 }
@@ -1490,7 +1480,8 @@ static void line_sweep_fac_d(const LevelView<T>& L, int color, const T* fac, con
       if (res) ends_dispatch<kFacF32, D>(a, sh, in_one, st);
       else ends_dispatch<kFacF32, DS>(a, sh, false, st);
     }
-    if (D == 0 && !res) apply_rb<T, D>(L, pa, pb, dv, tl, rb, st);
+    if constexpr (D == 0)
+      if (!res) apply_rb<T, D>(L, pa, pb, dv, tl, rb, st);
   } else {
     // 12 lanes a line while that is shorter: two lines a warp and 10 FP64
     // instructions a row against 32 lines and 64, on 4 x 152 SM quarters --
@@ -1601,8 +1592,9 @@ template void launch_line_sweep_fac<double>(const LevelView<double>&, int, int, 
                                             SweepShape, const double*);
 
 // ---------------------------------------------------------------- fused line relaxation
-// One launch per colour and direction.  A thread owns one line and walks it
-// twice:
+// One launch per colour and direction.  complex128 (k_line_fused): a thread
+// owns one line and walks it twice; complex64 (k_line_fused_ends): two threads,
+// one from either end, the multipliers as LineL keeps them.
 //   forward   node by node it assembles each row -- band entries and the
 //             residual of the current iterate, the row arithmetic of
 //             assemble_row -- and feeds it to the streaming LDL^T of
@@ -1613,9 +1605,9 @@ template void launch_line_sweep_fac<double>(const LevelView<double>&, int, int, 
 // of the colour reads or writes it, and that buffer is dead while the level
 // smooths (the cycle recomputes the residual after smoothing).  L waits in
 // the line scratch, [row][line] planes per RHS:
-//   kLExact  the T-precision values (k_line_solve's arithmetic, bit for bit
-//            the same operations in the same order);
-//   kLHalf   (T = float) rounded to fp16 and used rounded by both
+//   kLExact  the working precision's values (in complex128 k_line_solve's
+//            arithmetic, bit for bit the same operations in the same order);
+//   kLHalf   (complex64) rounded to fp16 and used rounded by both
 //            substitutions while the elimination keeps the unrounded value:
 //            each line solve is then exact for a matrix within fp16 rounding
 //            of the line's -- the arithmetic of the stored-factor format

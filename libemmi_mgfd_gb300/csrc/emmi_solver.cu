@@ -659,11 +659,10 @@ static int build_point_data(emmi_solver* s) {
   return EMMI_OK;
 }
 
-// Stored line factors of the complex64 cycle: size the factor blocks of every
-// (hierarchy, level, direction, colour) the smoother relaxes, and factor each
-// group's lines once.  Leaves
-// fac_on false (factoring in every sweep) when they would take more than
-// half of the free device memory.
+// Stored line factors: size the factor blocks of every (hierarchy, level,
+// direction, colour) the smoother relaxes, and factor each group's lines once.
+// Leaves fac_on false (factoring in every sweep) when they would take more
+// than half of the free device memory.
 template <typename T>
 static int build_line_factors(emmi_solver* s) {
   const int ng = s->ngroups;

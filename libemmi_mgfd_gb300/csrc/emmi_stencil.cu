@@ -405,16 +405,20 @@ bool stencil_prepare(const LevelView<float>& V, long u_elems, long cell_elems, S
   if (!TY || (TY < std::min(16, Y) && (long)TY * (X - 1) < kStThreads)) return false;
   a.TY = TY;
   a.ntj = (Y + TY - 1) / TY;
-  // a batch whose 32-plane tiles fill the SMs anyway: the plain kernel, which
-  // keeps more loads in flight than one block an SM with its barriers (25 RHS
-  // at 128^3: 1.43 against 1.71 ms)
+  // a batch whose tiles of 32 planes fill the SMs takes the plain kernels,
+  // which keep more loads in flight than one block an SM with its barriers:
+  // coefficients from the spacings (k_residual_nodes) 25 RHS at 128^3 1.44
+  // against 1.72 ms, 12 at 64^3 94 and 160 us; a general permeability
+  // (k_residual) 12 at 64^3 160 and 176 us, 25 330 and 338, 25 at 48^3 144 and
+  // 193.  Below, a caller's staged = 1 stands, though k_residual_nodes is the
+  // faster one there too: 3.9 against 9.0 us at 16^3, 10 and 20 at 64^3, 63 and
+  // 80 at 128^3 (one RHS each), 64 and 128 for 8 at 64^3
   if ((long)a.ntj * ((Z + 31) / 32) * V.nrhs >= 152) return false;
-  // planes of a tile: 32 where that gives every SM a CTA (two halo planes in
-  // 34), fewer while it does not -- a tile marches its planes one after the
-  // other (3 to 4 us a plane), so a small batch left most SMs idle behind 32
-  // of them: one RHS at 64^3 148 us on 15 tiles of 32 planes, about 20 us on
-  // 165 tiles of 2; at 16^3 51 and 15 us
-  for (a.KZ = 32;; a.KZ /= 2) {
+  // planes of a tile: a tile marches them one after the other (3 to 4 us a
+  // plane), so 16 of them or, where those leave SMs without a CTA, fewer (one
+  // RHS at 64^3: 138 us on 15 tiles of 32 planes, 20 on 165 tiles of 2; at 16^3
+  // 41 and 9.0)
+  for (a.KZ = 16;; a.KZ /= 2) {
     a.ntk = (Z + a.KZ - 1) / a.KZ;
     if (a.KZ == 2 || (long)a.ntj * a.ntk * V.nrhs >= 152) break;
   }
