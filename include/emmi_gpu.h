@@ -76,12 +76,12 @@ typedef struct {
                        set-up and keep the factors, when they fit in half
                        the free device memory.  MIXED: 2 = L in fp16, 1/d in
                        fp32 (fp32 throughout if an L value leaves the fp16
-                       range), 1 = fp32; FP64: 1 or 2 = in FP64.  Where the
-                       rest of that half has room, also the coarsest level's
-                       patch factors and, FP64, the coefficients of every
-                       level (240 bytes per slot and operator; with
-                       line_sweep = 1 too).  0 = factor and recompute in
-                       every sweep (2)                                     */
+                       range), 1 = fp32; FP64: 1 or 2 = in FP64.  Beside
+                       them, in the rest of that half or an eighth of the
+                       memory, the coarsest level's patch factors and, FP64,
+                       the coefficients of the levels (240 bytes per slot
+                       and operator; with line_sweep = 1 too).  0 = factor
+                       and recompute in every sweep (2)                    */
   int autotune;     /* MIXED with stored fp16 factors: time the level-0
                        line sweep of each direction at set-up for a few
                        block shapes and keep the fastest; cached for the

@@ -611,11 +611,14 @@ static int build_groups(emmi_solver* s) {
 
 // Whether bytes more may be stored to save recomputing them.  The line factors
 // come first and may take half of the memory that is free before them; what is
-// stored besides fills up that half at most, so that neither the factors nor
-// the program's other allocations find less room for it.
+// stored besides (complex128 coefficients, the coarsest level's patches) fills
+// up that half, or takes an eighth of that memory where the factors leave less
+// of the half: the coefficients of a semi-coarsening cycle, a quarter of its
+// factors, then fit whenever the factors do, and three eighths stay free.
 static bool fits_stored(const emmi_solver* s, size_t bytes) {
-  const size_t kept = (s->fac_on ? s->fac_bytes : 0) + s->stored_bytes;
-  return kept + bytes <= (device_avail() + kept) / 2;
+  const size_t fac = s->fac_on ? s->fac_bytes : 0;
+  const size_t room = device_avail() + fac + s->stored_bytes;
+  return s->stored_bytes + bytes <= std::max(room / 8, room / 2 > fac ? room / 2 - fac : 0);
 }
 
 // Stored coefficients and patch factors of the coarsest level of every
@@ -918,26 +921,24 @@ static int autotune_sweeps(emmi_solver* s) {
   return EMMI_OK;
 }
 
-// Stored FP64 coefficients of every level of the complex128 cycle: its row and
+// Stored FP64 coefficients of the levels of the complex128 cycle: its row and
 // level residuals would spend most of their FP64 instructions on recomputing
 // them (eight divisions an edge), bit for bit the same.  240 bytes a slot and
-// operator, kept when they fit (fits_stored).
+// operator, level after level while they fit (fits_stored); a level without
+// them computes them.
 static int build_coef64_levels(emmi_solver* s) {
-  size_t bytes = 0;
-  for (int h = 0; h < 3; h++)
-    for (int l = h ? 1 : 0; l < s->lmax; l++)
-      bytes += (size_t)s->nop * coef64_elems(s->hier[h][l].n) * sizeof(double);
-  if (!fits_stored(s, bytes)) return EMMI_OK;
-  s->stored_bytes += bytes;
-  for (int h = 0; h < 3; h++)
-    for (int l = 0; l < s->lmax; l++) {
-      if (h && l == 0) {
-        s->coef64[h][0] = s->coef64[0][0];
+  for (int l = 0; l < s->lmax; l++)
+    for (int h = 0; h < 3; h++) {
+      // hierarchies share level 0, and every level without semi-coarsening
+      if (h && (l == 0 || !s->opt.isemicoarsen)) {
+        s->coef64[h][l] = s->coef64[0][l];
         continue;
       }
       const size_t b = (size_t)s->nop * coef64_elems(s->hier[h][l].n) * sizeof(double);
+      if (!fits_stored(s, b)) continue;
       int rc;
       if ((rc = s->alloc((void**)&s->coef64[h][l], b)) != EMMI_OK) return rc;
+      s->stored_bytes += b;
       CK(cudaMemsetAsync(s->coef64[h][l], 0, b, s->st));
       LevelView<double> V = s->view<double>(h, l);
       V.nrhs = s->nop;
@@ -958,7 +959,6 @@ static int build_coef64(emmi_solver* s) {
   if (bytes > device_avail() / 2) return EMMI_OK;
   int rc;
   if ((rc = s->alloc((void**)&s->d_coef64, bytes)) != EMMI_OK) return rc;
-  s->stored_bytes += bytes;
   CK(cudaMemsetAsync(s->d_coef64, 0, bytes, s->st));
   LevelView<double> V = s->view<double>(0, 0);
   V.nrhs = s->nop;
@@ -1391,11 +1391,12 @@ static int create_impl(emmi_solver** out, const emmi_problem* P, const emmi_opti
         for (int h = 1; h < 3; h++) s->plan[h][0] = s->plan[0][0];
     }
     if (mixed) TRY(build_coef64(s));
-    else if (s->opt.line_factors) TRY(build_coef64_levels(s));
     mark("FP64 coefficients");
     if (s->opt.line_factors && s->lmax > 1)
       TRY(mixed ? build_point_data<float>(s) : build_point_data<double>(s));
     mark("coarsest level");
+    if (!mixed && s->opt.line_factors) TRY(build_coef64_levels(s));
+    mark("FP64 coefficients of the levels");
   }
 
   // ---- graphs

@@ -104,7 +104,8 @@ struct emmi_solver {
   long fac_off[3][emmi::kMaxLev][3][4];
   int fac_tile[3][emmi::kMaxLev][3];  // lines per tile of the complex64 blocks
 
-  // what is stored besides the line factors (coefficients, patch factors)
+  // what is stored besides the line factors (the complex128 cycle's
+  // coefficients, patch factors)
   size_t stored_bytes = 0;
 
   // node-patch sweeps of the coarsest level (per hierarchy): coefficients per

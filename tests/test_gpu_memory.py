@@ -1,6 +1,6 @@
 """What a solver stores to save recomputation, when device memory is short: the
-line factors find the room they had without the other stored data, and half of
-the memory that was free stays free."""
+line factors find the room they had without the other stored data, and three
+eighths of the memory that was free stay free."""
 import numpy as np
 import pytest
 
@@ -43,6 +43,7 @@ class _Free:
         free = torch.cuda.mem_get_info()[0]
         assert free > target, "the device is smaller than this test expects"
         self.hold = torch.empty(free - int(target), dtype=torch.uint8, device="cuda")
+        self.free = torch.cuda.mem_get_info()[0]
 
     def close(self):
         import torch
@@ -50,24 +51,35 @@ class _Free:
         torch.cuda.empty_cache()
 
 
-# 1.9 times what a complex128 solver stores: the factors fit in half of it,
-# with the coefficients (a fifth of the whole) they do not
+# 62 halves once: level 0's factors are all there are (96 bytes a row in
+# complex128, 28 in complex64), and the coarsest levels of 62 x 31 x 31 have
+# large patch data
+_N62 = (62, 62, 62)
+
+
+def _factors62(nop, row):
+    return nop * 3 * 61 * 61 * (5 * 62 - 4) * row
+
+
+# room for the factors in half of what is free, for the patch data or the
+# coefficients besides, and not for all three within five eighths (32 MB: the
+# pool's granularity)
 @gpu
-def test_stored_data_leaves_half_of_the_memory_free():
+def test_stored_data_leaves_three_eighths_of_the_memory_free():
     from libemmi_mgfd_gb300 import gpu as G
-    n, nop = (32, 32, 32), 8
+    n, nop = _N62, 8
     s = _solver(n, nop, G.PREC_FP64, 0)
     base = s.device_bytes
     s.close()
     s = _solver(n, nop, G.PREC_FP64, 1)
     stored, want = s.device_bytes - base, _solve(s, n, nop)
     s.close()
-    room = _Free(base + 1.9 * stored)
+    room = _Free(base + 2.45 * _factors62(nop, 96))
     try:
         s = _solver(n, nop, G.PREC_FP64, 1)
         kept = s.device_bytes - base
         assert s.line_factor_format == 0
-        assert kept <= 0.95 * stored, (kept, stored)
+        assert kept <= 0.625 * (room.free - base) + (32 << 20) < stored, (kept, stored)
         got = _solve(s, n, nop)
         s.close()
     finally:
@@ -76,16 +88,34 @@ def test_stored_data_leaves_half_of_the_memory_free():
         assert rel_err(got[r], want[r]) < 1e-10
 
 
-# 62 halves once: the coarsest levels of 62 x 31 x 31 have large patch data,
-# which must not push the line factors out of their half.  Level 0's factors
-# are all there are (96 bytes a row in complex128, 28 in complex64)
+# the coefficients fit beside factors that take nearly their whole half
+@gpu
+def test_coefficients_fit_wherever_the_line_factors_do():
+    from libemmi_mgfd_gb300 import gpu as G
+    n, nop = (32, 32, 32), 8
+    s = _solver(n, nop, G.PREC_FP64, 0)
+    base = s.device_bytes
+    s.close()
+    s = _solver(n, nop, G.PREC_FP64, 1)
+    stored = s.device_bytes - base
+    s.close()
+    room = _Free(base + 1.75 * stored)
+    try:
+        s = _solver(n, nop, G.PREC_FP64, 1)
+        assert s.device_bytes - base == stored
+        s.close()
+    finally:
+        room.close()
+
+
+# the patch data must not push the line factors out of their half
 @gpu
 @pytest.mark.parametrize("prec, row", [(0, 96), (1, 28)])
 def test_patch_data_does_not_displace_the_line_factors(prec, row):
     from libemmi_mgfd_gb300 import gpu as G
     assert (G.PREC_FP64, G.PREC_MIXED) == (0, 1)
-    n, nop, lf = (62, 62, 62), 4, 2 if prec else 1
-    factors = nop * 3 * 61 * 61 * (5 * 62 - 4) * row
+    n, nop, lf = _N62, 4, 2 if prec else 1
+    factors = _factors62(nop, row)
     s = _solver(n, nop, prec, 0)
     # the complex64 solver's FP64 coefficients of level 0 come after the factors
     base = s.device_bytes - (nop * 240 * 63 ** 3 if prec else 0)
